@@ -6,7 +6,8 @@
 //                      every pixel's neighbour record into six float4 planes (p.win):
 //                        W_GATE (unit normal xyz, depth)      the normal / depth gates
 //                        W_ALB  (albedo xyz, 1/max(n-1, 1))   the albedo gate; 0 marks a pixel
-//                                                             without a primary hit
+//                                                             without a primary hit, 1 + 2^-23
+//                                                             (kSingleRp) one with a single sample
 //                        W_SM   (sqrt mean rgb, rpd[4])       Welch means
 //                        W_SV   (stabilised sqrt var rgb, rpd[5])
 //                        W_RPD  (rpd[0..3])                   the RPD relaxation
@@ -126,6 +127,10 @@ __global__ void k_sqrt_var_mean(PixelPlanes p, int64_t np) {
 // the work; each quotient is rounded to float through a single-precision estimate and an exact
 // integer remainder (the double division only where that cannot decide). The values are
 // positive: sqrt_var_mean is floored at 1e-8.
+// 1 / max(n - 1, 1) of a pixel with one sample, one ulp above 1 to tell it from two samples: the
+// degrees of freedom n_i + n_j - 2 of a vanishing denominator need n (count_minus_one).
+constexpr float kSingleRp = 1.00000012f;
+
 enum WinPlane { W_GATE = 0, W_ALB, W_SM, W_SV, W_RPD, W_CM, W_COUNT };
 
 // The neighbour record of pixel i (the planes of p.win) and the window's debug planes
@@ -152,7 +157,7 @@ __device__ __forceinline__ void pack_window_record(const PixelPlanes& p, int64_t
     p.var_total[i] = var;
     p.var_eff[i] = vm;
     p.var_ratio[i] = (var > 1e-8f) ? (vm * float(n)) / var : 0.0f;
-    const float rp = 1.0f / fmaxf(float(n - 1), 1.0f);
+    const float rp = n == 1 ? kSingleRp : 1.0f / float(n - 1);
     win[W_GATE * np + i] = make_float4(p.f_normal[0][i], p.f_normal[1][i], p.f_normal[2][i], p.f_depth[i]);
     win[W_ALB * np + i] = make_float4(p.f_albedo[0][i], p.f_albedo[1][i], p.f_albedo[2][i], rp);
     win[W_SM * np + i] = make_float4(p.sqrt_mean[0][i], p.sqrt_mean[1][i], p.sqrt_mean[2][i], p.rpd[4][i]);
@@ -221,7 +226,7 @@ struct StatmcParams {
     float df_break;             // 30.5 with a table, 30 with the quantile
     float band;                 // relative guard band of the q and df decisions
     float ws_band;              // relative guard band of the weight_sum >= 1.1 test
-    float den_lim;              // 1e-8 (1 + band): the df denominator's band edge
+    float den_lo, den_lim;      // 1e-8 (1 -+ band): the df denominator's band
     float df_lim;               // df_break * band
     float q25_lim;              // 25 * band
     float qacc_lim;             // 2 ln 20 * band
@@ -396,8 +401,25 @@ struct Pix {
     float sm0, sm1, sm2;     // sqrt colour mean
     float sv0, sv1, sv2;     // stabilised sqrt variance of the mean
     float v0, v1, v2;        // sv^2 / max(n - 1, 1)
+    float nm1;               // n - 1
     float r0, r1, r2, r3, r4, r5;  // RPD components
 };
+
+// n - 1 from a record's 1 / max(n - 1, 1): the approximate reciprocal of fl(1 / k) lies within
+// k 2^-22 of the integer k, so rounding gives k for every k below 2^21 (larger ones are far above the
+// t-table switch, where their last digits do not matter).
+__device__ __forceinline__ float count_minus_one(float rp) { return rp > 1.0f ? 0.0f : rintf(div_approx(1.0f, rp)); }
+
+// df of a denominator below 1e-8: n_i + n_j - 2, an integer, so no decision on it is near; inside
+// 1e-8's band the slow pass decides.
+__device__ __forceinline__ void vanishing_df(float den, float dfn, const StatmcParams& prm, float& df, bool& near) {
+    if (den < prm.den_lo) {
+        df = dfn;
+        near = false;
+    } else {
+        near = near || den <= prm.den_lim;
+    }
+}
 
 // t critical value of a neighbour's df. MODE 0-2: an alpha with a t table (0.05, 0.01): the
 // line of the half-step table, t = v.y * df + v.x; lines 61-63 hold the normal quantile, so the
@@ -406,8 +428,8 @@ struct Pix {
 template <int MODE>
 __device__ __forceinline__ float t_crit(float df, const float2* __restrict__ line, const StatmcParams& prm) {
     if constexpr (MODE != 3) {
-        // MODE 1: every df is at most (n_i - 1) + (n_j - 1) <= 30, inside the table already
-        const float dfc = MODE == 1 ? df : fminf(df, 31.75f);
+        // MODE 1 and 4: every df is at most (n_i - 1) + (n_j - 1) <= 30, inside the table already
+        const float dfc = MODE == 1 || MODE == 4 ? df : fminf(df, 31.75f);
         // 2 dfc is exact, so one rounding down of 2 dfc + 1.5 * 2^23 leaves floor(2 dfc) in the low bits
         const float fl = __fmaf_rd(dfc, 2.0f, 12582912.0f);
         const float2 l = line[__float_as_int(fl) - 0x4B400000];
@@ -423,8 +445,14 @@ __device__ __forceinline__ float t_crit(float df, const float2* __restrict__ lin
 }
 
 // One neighbour of the window: gates, Welch q, relaxation, weight, accumulation. MODE 0: any
-// df (t table); 1: every df of the block below the switch (t table); 2: every df at or above
-// 31 (t = z); 3: any df, normal-quantile alpha.
+// df (t table); 1: every df of the block below the switch (t table) and every df denominator above
+// 1e-8's band; 2: every df at or above 31 (t = z); 3: any df, normal-quantile alpha; 4: as 1 with
+// denominators of any size.
+// A denominator below 1e-8 (both pixels nearly or wholly black, the rule in a scene's shadows)
+// takes the reference's df = n_i + n_j - 2 (main.cpp:1074) here; only one inside the band around
+// 1e-8 is left to the slow pass. With every denominator up to the band's end left to it, a
+// 1283x717x6 frame with a quarter of its samples black handed over 78,310 pixels (16.4 M
+// double-precision q): 16.1 ms a frame, 3.13 ms with this (256x256x4: 0.59 -> 0.18 ms).
 // Straight-line: the gates are folded into one predicate (each written as the negation of the
 // reference's `continue` test, so a NaN passes a gate as it does there) and only the
 // accumulation is conditional, so a warp whose lanes leave at different gates runs one path.
@@ -467,16 +495,26 @@ __device__ __forceinline__ void visit(const float4* __restrict__ T, int tn, int 
         const float den0 = __fmaf_rn(V.x * V.x, rpj, P.v0);
         const float den1 = __fmaf_rn(V.y * V.y, rpj, P.v1);
         const float den2 = __fmaf_rn(V.z * V.z, rpj, P.v2);
-        // MODE 1 blocks have every denominator above the band (their smallest term is)
-        if constexpr (MODE != 1) exact |= fminf(fminf(den0, den1), den2) <= prm.den_lim;
-        const float df0 = div_approx(vs0 * vs0, den0);
-        const float df1 = div_approx(vs1 * vs1, den1);
-        const float df2 = div_approx(vs2 * vs2, den2);
+        float df0 = div_approx(vs0 * vs0, den0);
+        float df1 = div_approx(vs1 * vs1, den1);
+        float df2 = div_approx(vs2 * vs2, den2);
+        bool near0 = false, near1 = false, near2 = false;
         if constexpr (MODE == 0 || MODE == 3) {
-            exact |= fabsf(df0 - prm.df_break) <= prm.df_lim;
-            exact |= fabsf(df1 - prm.df_break) <= prm.df_lim;
-            exact |= fabsf(df2 - prm.df_break) <= prm.df_lim;
+            near0 = fabsf(df0 - prm.df_break) <= prm.df_lim;
+            near1 = fabsf(df1 - prm.df_break) <= prm.df_lim;
+            near2 = fabsf(df2 - prm.df_break) <= prm.df_lim;
         }
+        // MODE 1 blocks have every denominator above the band (their smallest term is)
+        if constexpr (MODE != 1) {
+            if (fminf(fminf(den0, den1), den2) <= prm.den_lim) {
+                // (inf beside an invalid record's rp = 0) kept inside the t table
+                const float dfn = fminf(P.nm1 + count_minus_one(rpj), 31.75f);
+                vanishing_df(den0, dfn, prm, df0, near0);
+                vanishing_df(den1, dfn, prm, df1, near1);
+                vanishing_df(den2, dfn, prm, df2, near2);
+            }
+        }
+        exact = near0 || near1 || near2;
         const float t0 = t_crit<MODE>(df0, line, prm);
         const float t1 = t_crit<MODE>(df1, line, prm);
         const float t2 = t_crit<MODE>(df2, line, prm);
@@ -596,6 +634,7 @@ __global__ void __launch_bounds__(kSlowThreads) k_statmc_slow(PixelPlanes p, Sta
         const float smi[3] = {si.x, si.y, si.z}, svi[3] = {vi.x, vi.y, vi.z};
         const float vi0 = vi.x * vi.x * ai.w, vi1 = vi.y * vi.y * ai.w, vi2 = vi.z * vi.z * ai.w;
         const int n_i = imaxs(1, p.n[idx]);
+        const float nm1_i = float(n_i - 1);
         float acc[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
         int accepted = 0, pairs = 0;
         for (int v = lane; v < visits; v += 32) {
@@ -626,11 +665,14 @@ __global__ void __launch_bounds__(kSlowThreads) k_statmc_slow(PixelPlanes p, Sta
             const float md[3] = {si.x - S.x, si.y - S.y, si.z - S.z};
             const float den[3] = {__fmaf_rn(V.x * V.x, A.w, vi0), __fmaf_rn(V.y * V.y, A.w, vi1),
                                   __fmaf_rn(V.z * V.z, A.w, vi2)};
-            bool exact = fminf(fminf(den[0], den[1]), den[2]) <= prm.den_lim;
+            const float dfn = nm1_i + count_minus_one(A.w);
+            bool exact = false;
             float qmax = 0.0f;
             for (int c = 0; c < 3; ++c) {
-                const float df = div_approx(vs[c] * vs[c], den[c]);
-                exact |= fabsf(df - prm.df_break) <= prm.df_lim;
+                float df = div_approx(vs[c] * vs[c], den[c]);
+                bool near = fabsf(df - prm.df_break) <= prm.df_lim;
+                vanishing_df(den[c], dfn, prm, df, near);
+                exact = exact || near;
                 const float t = prm.table < 2 ? t_crit<0>(df, s_line, prm) : t_crit<3>(df, s_line, prm);
                 qmax = fmaxf(qmax, div_approx(md[c] * md[c], vs[c] * (t * t)));
             }
@@ -694,7 +736,7 @@ __global__ void __launch_bounds__(kTileX * kRows, 3)
     __shared__ __align__(8) unsigned long long bar;
     __shared__ float2 s_line[64];
     __shared__ unsigned s_rpmin, s_rpmax, s_dmin;
-    __shared__ int s_fail;
+    __shared__ int s_fail, s_huge;
     const int r = RC > 0 ? RC : prm.r;
     const int by = RC > 0 ? kRows : prm.by;
     const int tw = kTileX + 2 * r, th = by + 2 * r, tn = tw * th, side = 2 * r + 1;
@@ -712,6 +754,7 @@ __global__ void __launch_bounds__(kTileX * kRows, 3)
         s_rpmin = 0x7f800000u;  // +inf
         s_rpmax = 0u;
         s_dmin = 0x7f800000u;
+        s_huge = 0;
         s_fail = 0;
     }
     __syncthreads();
@@ -738,7 +781,9 @@ __global__ void __launch_bounds__(kTileX * kRows, 3)
 
     // the halo's range of 1/max(n-1, 1) selects the block's loop; so does the smallest term
     // fl(fl(sv^2) * rp) of a df denominator: every denominator fl(sv_j^2 * rp_j + v_i) is at
-    // least its neighbour's term, so above the band when the smallest term is
+    // least its neighbour's term, so above the band when the smallest term is. The loops that index
+    // the t table by an unclamped df (1 and 4) need its quotient finite: variances up to 1e18.
+    bool huge = false;
     float lmin = __uint_as_float(0x7f800000u), lmax = 0.0f, dmin = __uint_as_float(0x7f800000u);
     for (int e = tid; e < tn; e += nthreads) {
         const float rp = T[W_ALB * tn + e].w;
@@ -747,6 +792,7 @@ __global__ void __launch_bounds__(kTileX * kRows, 3)
             lmin = fminf(lmin, rp);
             lmax = fmaxf(lmax, rp);
             dmin = fminf(dmin, fminf(fminf((v.x * v.x) * rp, (v.y * v.y) * rp), (v.z * v.z) * rp));
+            huge = huge || !(v.x <= 1e18f && v.y <= 1e18f && v.z <= 1e18f);
         }
     }
 #pragma unroll
@@ -760,11 +806,13 @@ __global__ void __launch_bounds__(kTileX * kRows, 3)
         atomicMax(&s_rpmax, __float_as_uint(lmax));
         atomicMin(&s_dmin, __float_as_uint(dmin));
     }
+    if (huge) s_huge = 1;
     __syncthreads();
     const int mode = __uint_as_float(s_rpmax) <= prm.rp_above                                     ? 2
                      : prm.table == 2                                                              ? 3
-                     : __uint_as_float(s_rpmin) >= prm.rp_below && __uint_as_float(s_dmin) > prm.den_lim ? 1
-                                                                                                   : 0;
+                     : __uint_as_float(s_rpmin) < prm.rp_below || s_huge                           ? 0
+                     : __uint_as_float(s_dmin) > prm.den_lim                                       ? 1
+                                                                                                   : 4;
 
     const int x = x0 + threadIdx.x, y = y0 + threadIdx.y;
     if (x >= prm.w || y >= prm.h) return;
@@ -801,6 +849,7 @@ __global__ void __launch_bounds__(kTileX * kRows, 3)
         P.v0 = v.x * v.x * ali.w;
         P.v1 = v.y * v.y * ali.w;
         P.v2 = v.z * v.z * ali.w;
+        P.nm1 = count_minus_one(ali.w);
         P.r0 = rr.x;
         P.r1 = rr.y;
         P.r2 = rr.z;
@@ -815,6 +864,8 @@ __global__ void __launch_bounds__(kTileX * kRows, 3)
         window_rows<RC, 2>(T, tn, tw, r, spatial, s_line, prm, P, ei, acc, accepted, slow);
     else if (mode == 1)
         window_rows<RC, 1>(T, tn, tw, r, spatial, s_line, prm, P, ei, acc, accepted, slow);
+    else if (mode == 4)
+        window_rows<RC, 4>(T, tn, tw, r, spatial, s_line, prm, P, ei, acc, accepted, slow);
     else if (mode == 3)
         window_rows<RC, 3>(T, tn, tw, r, spatial, s_line, prm, P, ei, acc, accepted, slow);
     else
@@ -946,6 +997,7 @@ cudaError_t launch_statmc(Job& j) {
     prm.df_break = prm.table < 2 ? 30.5f : 30.0f;
     prm.band = std::ldexp(1.0f, -j.window_guard);
     prm.ws_band = std::ldexp(1.0f, -j.window_guard - 1);
+    prm.den_lo = 1e-8f * (1.0f - prm.band);
     prm.den_lim = 1e-8f * (1.0f + prm.band);
     prm.df_lim = prm.df_break * prm.band;
     prm.q25_lim = 25.0f * prm.band;
