@@ -135,7 +135,7 @@ __device__ __forceinline__ void df_add(float& hi, float& lo, float x) {
 struct SampleIn {
     float L[3], n[3], d, alb[3], pu[2], lu[2], bu[2], liu[2], eu[2];
     uint8_t f, cat;
-    uint32_t bins;  // COMPACT_IN: the lens, BRDF, light and environment bins, 4 bits each
+    uint32_t bins;  // COMPACT_IN: the BRDF, lens, light and environment bins in the key's fields
     float root[3];  // COMPACT_IN: sqrt(max(0, L)), known exactly (L is the square of a half)
 };
 
@@ -189,7 +189,7 @@ __device__ __forceinline__ void process_sample(PixelAcc& a, const SampleIn& in, 
     }
     if (!finite3(in.L[0], in.L[1], in.L[2])) {  // main.cpp:707
         lum_out = __int_as_float(0x7fc00000);  // NaN: dropped by the grid pass
-        key_out = 0;
+        key_out = kKeyNone;
         return;
     }
     // accumulate_sample (core/stats.h:25-41)
@@ -238,23 +238,25 @@ __device__ __forceinline__ void process_sample(PixelAcc& a, const SampleIn& in, 
     for (int c = 0; c < 3; ++c) a.rad[c] += in.L[c];
     ++a.nsamples;
     lum_out = lum;
-    key_out = 0;
+    key_out = kKeyNone;
     if (!prep) return;
     const uint8_t fm = in.f & plane_mask;
     // packed random-dimension bins (Dependency2D::add, core/stats.h:166-168)
-    uint32_t key = 0;
+    uint32_t key;
     if (COMPACT_IN) {
-        key = in.bins & ((fm & RPD_SAMPLE_LENS_VALID ? 0x000fu : 0u) | (fm & RPD_SAMPLE_BRDF_VALID ? 0x00f0u : 0u) |
-                         (fm & RPD_SAMPLE_LIGHT_VALID ? 0x0f00u : 0u) | (fm & RPD_SAMPLE_ENV_VALID ? 0xf000u : 0u));
+        key = (fm & RPD_SAMPLE_BRDF_VALID) ? in.bins & 0x1fu : key_absent_bit(1);
+        key |= (fm & RPD_SAMPLE_LENS_VALID) ? in.bins & (0x1fu << 5) : key_absent_bit(2);
+        key |= (fm & RPD_SAMPLE_LIGHT_VALID) ? in.bins & (0x1fu << 10) : key_absent_bit(3);
+        key |= (fm & RPD_SAMPLE_ENV_VALID) ? in.bins & (0x1fu << 15) : key_absent_bit(4);
     } else {
-        if (fm & RPD_SAMPLE_LENS_VALID) key |= uint32_t(bin2d_k(in.lu[0], in.lu[1]));
-        if (fm & RPD_SAMPLE_BRDF_VALID) key |= uint32_t(bin2d_k(in.bu[0], in.bu[1])) << 4;
-        if (fm & RPD_SAMPLE_LIGHT_VALID) key |= uint32_t(bin2d_k(in.liu[0], in.liu[1])) << 8;
-        if (fm & RPD_SAMPLE_ENV_VALID) key |= uint32_t(bin2d_k(in.eu[0], in.eu[1])) << 12;
+        key = (fm & RPD_SAMPLE_BRDF_VALID) ? uint32_t(bin2d_k(in.bu[0], in.bu[1])) : key_absent_bit(1);
+        key |= (fm & RPD_SAMPLE_LENS_VALID) ? uint32_t(bin2d_k(in.lu[0], in.lu[1])) << 5 : key_absent_bit(2);
+        key |= (fm & RPD_SAMPLE_LIGHT_VALID) ? uint32_t(bin2d_k(in.liu[0], in.liu[1])) << 10 : key_absent_bit(3);
+        key |= (fm & RPD_SAMPLE_ENV_VALID) ? uint32_t(bin2d_k(in.eu[0], in.eu[1])) << 15 : key_absent_bit(4);
     }
-    key |= uint32_t(in.cat & RPD_CATEGORY_LIGHT_INDEX_MASK) << 16;
-    key |= (in.cat & RPD_CATEGORY_RR_SURVIVED) ? (1u << 20) : 0u;
-    key |= uint32_t(fm & 0xfe) << (kKeyValidShift - 1);
+    key |= (fm & RPD_SAMPLE_LIGHT_SELECT_VALID) ? uint32_t(in.cat & RPD_CATEGORY_LIGHT_INDEX_MASK) << 20 : key_absent_bit(5);
+    key |= (fm & RPD_SAMPLE_RR_VALID) ? ((in.cat & RPD_CATEGORY_RR_SURVIVED) ? 1u << 25 : 0u) : key_absent_bit(6);
+    key |= (fm & RPD_SAMPLE_PIXEL_VALID) ? 0u : key_absent_bit(0);
     key_out = key;
     const uint8_t cls_bits = fm & 0xfe;
     const float y2 = lum * lum;
@@ -504,10 +506,10 @@ __global__ void __launch_bounds__(128, MINB) k_accumulate_pixels(PixelPlanes p, 
                     }
                     in.d = h2f(lane16(D, i)) * dscale;
                     for (int c = 0; c < 2; ++c) in.pu[c] = unorm16(lane16(PU[c], i));
-                    in.bins = bin2d_q(lane16(LU[0], i), lane16(LU[1], i)) |
-                              (bin2d_q(lane16(BU[0], i), lane16(BU[1], i)) << 4) |
-                              (bin2d_q(lane16(LI[0], i), lane16(LI[1], i)) << 8) |
-                              (bin2d_q(lane16(EU[0], i), lane16(EU[1], i)) << 12);
+                    in.bins = bin2d_q(lane16(BU[0], i), lane16(BU[1], i)) |
+                              (bin2d_q(lane16(LU[0], i), lane16(LU[1], i)) << 5) |
+                              (bin2d_q(lane16(LI[0], i), lane16(LI[1], i)) << 10) |
+                              (bin2d_q(lane16(EU[0], i), lane16(EU[1], i)) << 15);
                     in.f = uint8_t(F[i >> 2] >> (8 * (i & 3)));
                     in.cat = uint8_t(Cg[i >> 2] >> (8 * (i & 3)));
                     process_sample<true>(a, in, false, palb, prep, plane_mask, fx, fy, lumv[i], keyv[i]);
@@ -539,8 +541,8 @@ __global__ void __launch_bounds__(128, MINB) k_accumulate_pixels(PixelPlanes p, 
                     q[2][c] = (dims && has_li) ? h.light_u[c][k] : uint16_t(0);
                     q[3][c] = (dims && has_eu) ? h.env_u[c][k] : uint16_t(0);
                 }
-                in.bins = bin2d_q(q[0][0], q[0][1]) | (bin2d_q(q[1][0], q[1][1]) << 4) |
-                          (bin2d_q(q[2][0], q[2][1]) << 8) | (bin2d_q(q[3][0], q[3][1]) << 12);
+                in.bins = bin2d_q(q[1][0], q[1][1]) | (bin2d_q(q[0][0], q[0][1]) << 5) |
+                          (bin2d_q(q[2][0], q[2][1]) << 10) | (bin2d_q(q[3][0], q[3][1]) << 15);
                 in.f = s.flags[k];
                 in.cat = (dims && s.category) ? s.category[k] : 0;
                 float lum;

@@ -264,8 +264,7 @@ __global__ void __launch_bounds__(kGroups * 32) k_grid_fast(GridParams gpar, flo
     const Geometry& g = gpar.g;
     const int nx = int(node % g.nodes_x), ny = int(node / g.nodes_x);
     LaneBins<INT_W> bins{sm + grp * LaneBins<INT_W>::kSlots * 32, lane, float(g.step) * float(g.step)};
-    const uint32_t vbit = key_valid_bit(grp);
-    const uint32_t pbit = key_valid_bit(0);
+    const uint32_t absent = key_absent_bit(grp) | key_absent_bit(0);
     int dep_x = D_PIXEL, dep_s = D_PIXEL;
     switch (grp) {
     case 1: dep_x = D_BRDF; dep_s = D_SCREEN_BRDF; break;
@@ -339,7 +338,7 @@ __global__ void __launch_bounds__(kGroups * 32) k_grid_fast(GridParams gpar, flo
             const int64_t kend = offsets[local + 1];
             for (int64_t k = offsets[local] + lane; k < kend; k += 32) {
                 const uint32_t key = gp.key[k];
-                if (!(key & pbit) || !(key & vbit)) continue;
+                if (key & absent) continue;
                 const float yv = gp.lum[k];
                 const float su = fclamps((fx + sample_pu(s, 0, k) - support_left) / support, 0.0f, 1.0f);
                 const float sv = fclamps((fy + sample_pu(s, 1, k) - support_top) / support, 0.0f, 1.0f);
@@ -397,7 +396,6 @@ __global__ void __launch_bounds__(32) k_grid_screen(GridParams gpar, float2* pas
     const int bsh = __ffs(g.support) - 3;             // log2(support / 4) when uniform_ok
     const int sl = nx * g.step - g.support / 2, st = ny * g.step - g.support / 2;  // integer when uniform_ok
     const float inv_wscale = 1.0f / wscale;
-    const uint32_t pbit = key_valid_bit(0);
 
     auto weight = [&](int x, int y) -> float {
         if (gpar.pow2_step)
@@ -413,14 +411,14 @@ __global__ void __launch_bounds__(32) k_grid_screen(GridParams gpar, float2* pas
     // samples of pixel (px, py) binned one by one by the whole warp (main.cpp:349-357): every
     // lane into its own bins; also the screen totals of a mixed pixel (samples with the
     // position and the class)
-    auto bin_samples = [&](LaneBins<INT_W>& bins, int64_t pidx, float pw, int px, int py, uint32_t vbit,
+    auto bin_samples = [&](LaneBins<INT_W>& bins, int64_t pidx, float pw, int px, int py, uint32_t absent,
                            bool pmixed, Totals& ts) {
         const float fx = float(px), fy = float(py);
         const int64_t local = pidx - gpar.first;
         const int64_t kend = offsets[local + 1];
         for (int64_t k = offsets[local] + lane; k < kend; k += 32) {
             const uint32_t key = gp.key[k];
-            if (!(key & pbit) || !(key & vbit)) continue;
+            if (key & absent) continue;
             const float yv = gp.lum[k];
             const float su = fclamps((fx + sample_pu(s, 0, k) - support_left) / support, 0.0f, 1.0f);
             const float sv = fclamps((fy + sample_pu(s, 1, k) - support_top) / support, 0.0f, 1.0f);
@@ -510,7 +508,7 @@ __global__ void __launch_bounds__(32) k_grid_screen(GridParams gpar, float2* pas
             const int64_t pidx = __shfl_sync(0xffffffffu, idx, src);
             const float pw = __shfl_sync(0xffffffffu, w, src);
             const int px = __shfl_sync(0xffffffffu, cx, src), py = __shfl_sync(0xffffffffu, cy, src);
-            bin_samples(binsA, pidx, pw, px, py, pbit, false, unused);
+            bin_samples(binsA, pidx, pw, px, py, key_absent_bit(0), false, unused);
         }
     }
     __syncwarp();
@@ -527,7 +525,7 @@ __global__ void __launch_bounds__(32) k_grid_screen(GridParams gpar, float2* pas
     for (int cl = 0; cl < kClasses; ++cl) {
         const bool inP0 = (P0 & class_bit(cl)) != 0;
         const bool p0screen = inP0 && p0pix;  // P0 pixels enter the screen sums of this class
-        const uint32_t vbit = key_valid_bit(cl);
+        const uint32_t absent = key_absent_bit(cl) | key_absent_bit(0);
         Totals tx, ts;
         float2 vb = make_float2(0.0f, 0.0f);
         if (nlist > 0) {
@@ -569,7 +567,7 @@ __global__ void __launch_bounds__(32) k_grid_screen(GridParams gpar, float2* pas
                     const float pw = __shfl_sync(0xffffffffu, w, src);
                     const bool pmixed = __shfl_sync(0xffffffffu, int(mixed), src) != 0;
                     const int sx = __shfl_sync(0xffffffffu, px, src), sy = __shfl_sync(0xffffffffu, py, src);
-                    bin_samples(binsB, pidx, pw, sx, sy, vbit, pmixed, ts);
+                    bin_samples(binsB, pidx, pw, sx, sy, absent, pmixed, ts);
                 }
             }
             vb = binsB.reduce_value();
@@ -660,7 +658,6 @@ __host__ __device__ constexpr int rand_slot0(int d) { return d * 16; }
 __host__ __device__ constexpr int rand_dep(int d) {
     return d == 0 ? D_BRDF : d == 1 ? D_LENS : d == 2 ? D_LIGHT_UV : d == 3 ? D_ENV : d == 4 ? D_LIGHT_SELECT : D_RR;
 }
-__host__ __device__ constexpr int rand_shift(int d) { return d == 5 ? 20 : key_bin_shift(d + 1); }
 __host__ __device__ constexpr uint32_t rand_mask(int d) { return d == 5 ? 1u : 15u; }
 
 // The six dimensions split into DS sets (one warp of a row group each): fewer private bins per
@@ -746,8 +743,8 @@ __device__ __forceinline__ void rand_update(const WalkCtx<WB, DS>& c, uint32_t k
 #pragma unroll
     for (int d = 0; d < kRandDims; ++d) {
         if (dim_set<DS>(d) != SET || !((DIMS >> d) & 1)) continue;
-        const bool on = wok && (key & key_valid_bit(d + 1)) != 0;
-        const int bin = int((key >> rand_shift(d)) & rand_mask(d));
+        const bool on = wok && (key & key_absent_bit(d + 1)) == 0;
+        const int bin = int((key >> key_shift(d + 1)) & rand_mask(d));
         slot[d] = (on ? dim_slot0<DS>(d) + bin : L::kTrash) * 32 + c.lane;
     }
     // the dimensions own disjoint slot ranges (the trash slot is only ever a sink): load all,
@@ -1136,6 +1133,349 @@ __global__ void __launch_bounds__(RW * DS * 32) k_grid_random(RandParams rp, flo
     }
 }
 
+
+// ---- random-dimension bins, strip form -------------------------------------------------------------
+//
+// For uniform pushes over power-of-two node steps up to 32, where the bilinear weight of a pixel is
+// the exact product of its row's and its column's multiple of 1/step. A lane owns an image column
+// and walks down it: in a strip of `step` rows (between two node rows) it adds each sample to its
+// private bins twice, times the row factor of the node row above and of the one below: two
+// double-floats and one word of two 16-bit integer weights. At the
+// strip's end the node row above is complete: its nodes' sums are the columns' bins times the
+// column factors, and the node row below becomes the next strip's upper one. A sample is visited
+// once instead of once per node it supports (four), and the walk needs neither row tables nor
+// per-sample weights. A block's NC column warps cover NC * 32 columns and so NC * 32 / step - 1
+// whole nodes of each of its `len` node rows (neighbouring blocks overlap by one cell, one strip);
+// RG row groups split a strip's rows where there are too few blocks. Every sum is lane-private and
+// combined in a fixed order: deterministic, no atomics.
+// The bound is the shared-memory data path (for 32 samples, ten 128-byte wavefronts per dimension)
+// with two warps per scheduler to hide its latency: the dimensions are split over two warps of a
+// segment, whose bins share its 44 KB. At 1920x1080x16 without environment planes, one warp per
+// node visiting every sample four times took 0.795 ms, this 0.387 ms (2048x1152x64: 2.75 -> 1.89 ms);
+// with one warp for all dimensions and single updates 0.48 ms, with the two sets' warps on
+// different schedulers 0.44 ms.
+struct StripParams {
+    Geometry g;
+    int64_t first, count;
+    int ny0, ny1;          // node rows of the launch
+    int len;               // node rows of a block
+    int col_blocks;        // blocks per `len` node rows
+    int spp;
+    int sh;                // log2 of the node step
+    int fresh;             // the grid holds zeros (the frame's first push): nothing to read back
+};
+
+// slots of the dimensions in DIMS: each one's bins and a sink for samples without it
+__host__ __device__ constexpr int strip_bins(int d) { return d == 5 ? 3 : 17; }
+template <int DIMS>
+__host__ __device__ constexpr int strip_slot0(int d) {
+    int s = 0;
+    for (int k = 0; k < d; ++k)
+        if ((DIMS >> k) & 1) s += strip_bins(k);
+    return s;
+}
+// the dimensions of warp set DS of two: brdf, lens and rr, or the rest
+template <int DIMS>
+__host__ __device__ constexpr int strip_set(int ds) { return DIMS & (ds == 0 ? 0x23 : 0x1c); }
+template <int DIMS>
+struct StripLayout {
+    static constexpr int kSlots = strip_slot0<DIMS>(kRandDims);
+    static constexpr int kHalf = kSlots * 32;                          // double-floats of one node row
+    static constexpr int kSumBytes = 2 * kHalf * 8;
+    static constexpr int kWarpBytes = kSumBytes + kSlots * 32 * 4;     // and two 16-bit weights
+    // the segments' first and last node, shared with the next segment: (sum, weight) per slot,
+    // doubled by strip parity
+    static constexpr int edge_bytes(int nc) { return 2 * 2 * nc * kSlots * 12; }
+};
+
+// N (1 or 2) samples of one pixel in the dimensions of SET. Two samples' bins are all loaded before
+// either is updated, and the second takes the first one's result where they meet in a bin, so that
+// the two read-modify-writes overlap.
+// BOTH: both node rows' sums; else only the one `sums` points at (the other's weight is 0).
+template <int DIMS, int SET, int N, bool BOTH>
+__device__ __forceinline__ void strip_update(uint32_t* wgt, float2* sums, const uint32_t* key, const float* y, float wa,
+                                             float wb, uint32_t iw) {
+    constexpr int kHalf = StripLayout<DIMS>::kHalf;
+    float ya[N], yae[N], yb[N], ybe[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        ya[i] = wa * y[i];
+        yae[i] = __fmaf_rn(wa, y[i], -ya[i]);
+        yb[i] = wb * y[i];
+        ybe[i] = __fmaf_rn(wb, y[i], -yb[i]);
+    }
+    uint32_t p[kRandDims][N], w[kRandDims][N];
+    float2 s[kRandDims][N], r[kRandDims][N];
+    // the dimensions own disjoint slots
+#pragma unroll
+    for (int d = 0; d < kRandDims; ++d) {
+        if (!((SET >> d) & 1)) continue;
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            p[d][i] = (((key[i] >> key_shift(d + 1)) & (d == 5 ? 3u : 31u)) + uint32_t(strip_slot0<DIMS>(d))) * 32u;
+            w[d][i] = wgt[p[d][i]];
+            s[d][i] = sums[p[d][i]];
+            if (BOTH) r[d][i] = sums[p[d][i] + kHalf];
+        }
+    }
+#pragma unroll
+    for (int d = 0; d < kRandDims; ++d) {
+        if (!((SET >> d) & 1)) continue;
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            if (i > 0) {
+                const bool same = p[d][i] == p[d][i - 1];
+                w[d][i] = same ? w[d][i - 1] : w[d][i];
+                s[d][i].x = same ? s[d][i - 1].x : s[d][i].x;
+                s[d][i].y = same ? s[d][i - 1].y : s[d][i].y;
+                if (BOTH) {
+                    r[d][i].x = same ? r[d][i - 1].x : r[d][i].x;
+                    r[d][i].y = same ? r[d][i - 1].y : r[d][i].y;
+                }
+            }
+            w[d][i] += iw;
+            df_add(s[d][i].x, s[d][i].y, ya[i]);
+            s[d][i].y += yae[i];
+            wgt[p[d][i]] = w[d][i];
+            sums[p[d][i]] = s[d][i];
+            if (BOTH) {
+                df_add(r[d][i].x, r[d][i].y, yb[i]);
+                r[d][i].y += ybe[i];
+                sums[p[d][i] + kHalf] = r[d][i];
+            }
+        }
+    }
+}
+
+// U samples of one pixel: keys and luminances (U = 8, 4: 16-byte loads; 1: scalar)
+template <int U>
+struct StripUnit {
+    uint32_t key[U];
+    float y[U];
+};
+template <int U>
+__device__ __forceinline__ void strip_load(StripUnit<U>& u, const GridPrep& gp, int64_t k, bool in) {
+#pragma unroll
+    for (int i = 0; i < U; ++i) {
+        u.key[i] = kKeyNone;
+        u.y[i] = 0.0f;
+    }
+    if (!in) return;
+    if constexpr (U == 1) {
+        u.key[0] = gp.key[k];
+        u.y[0] = gp.lum[k];
+    } else {
+#pragma unroll
+        for (int i = 0; i < U; i += 4) {
+            const uint4 a = *reinterpret_cast<const uint4*>(gp.key + k + i);
+            const float4 b = *reinterpret_cast<const float4*>(gp.lum + k + i);
+            u.key[i] = a.x, u.key[i + 1] = a.y, u.key[i + 2] = a.z, u.key[i + 3] = a.w;
+            u.y[i] = b.x, u.y[i + 1] = b.y, u.y[i + 2] = b.z, u.y[i + 3] = b.w;
+        }
+    }
+}
+
+template <int NC, int RG, int U, int DIMS>
+__global__ void __launch_bounds__(NC * RG * 64) k_grid_strips(StripParams sp, float2* grid, GridPrep gp) {
+    using L = StripLayout<DIMS>;
+    constexpr int NT = NC * RG * 64;  // two dimension sets
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ int s_entry[L::kSlots];  // a slot's entry of a node's 13 x 36, -1 for a sink
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // the two sets' warps of a segment are NC * RG apart, on the same one of the SM's four schedulers:
+    // their unequal walks share its issue slots
+    const int ds = warp / (NC * RG), rg = (warp / NC) % RG, cw = warp % NC;
+    const Geometry& g = sp.g;
+    const int step = g.step, sh = sp.sh;
+    const int r0 = sp.ny0 + int(blockIdx.x / unsigned(sp.col_blocks)) * sp.len;  // the block's node rows
+    const int r1 = imins(r0 + sp.len, sp.ny1);
+    const int cells = 32 >> sh;                  // of a column warp (a segment)
+    const int nb = NC * cells - 1;               // the block's nodes with both of their cells in it
+    const int cb = int(blockIdx.x % unsigned(sp.col_blocks));
+    const int c0 = cb * nb;                      // its first cell, between nodes c0 and c0 + 1
+    const float inv_step = 1.0f / float(step);
+    auto sums_of = [&](int w) { return reinterpret_cast<float2*>(smem_raw + w * L::kWarpBytes); };
+    auto weights_of = [&](int w) { return reinterpret_cast<uint32_t*>(smem_raw + w * L::kWarpBytes + L::kSumBytes); };
+    float2* edge_s = reinterpret_cast<float2*>(smem_raw + NC * RG * L::kWarpBytes);  // [parity][left, right][NC][slot]
+    uint32_t* edge_w = reinterpret_cast<uint32_t*>(edge_s + 4 * NC * L::kSlots);
+    float2* sums = sums_of(rg * NC + cw) + lane;
+    uint32_t* wgt = weights_of(rg * NC + cw) + lane;
+#pragma unroll 4
+    for (int k = ds; k < L::kSlots; k += 2) {
+        wgt[k * 32] = 0u;
+        sums[k * 32] = sums[k * 32 + L::kHalf] = make_float2(0.0f, 0.0f);
+    }
+    for (int slot = threadIdx.x; slot < L::kSlots; slot += NT) {
+        int en = -1;
+#pragma unroll
+        for (int d = 0; d < kRandDims; ++d) {
+            if (!((DIMS >> d) & 1)) continue;
+            const int bin = slot - strip_slot0<DIMS>(d);
+            if (bin >= 0 && bin < strip_bins(d) - 1) en = rand_dep(d) * kDepStride + bin;
+        }
+        s_entry[slot] = en;
+    }
+    __syncthreads();
+
+    const int x = c0 * step + cw * 32 + lane;
+    const bool xin = x < g.w;
+    const int upr = sp.spp / U;  // units of a pixel
+    const int s0 = imaxs(r0 - 1, 0), s1 = r1;  // strips (the one below the last node row has no rows)
+    const int ylast = imins(g.h, s1 * step) - 1;  // the block's last image row
+    // the walk's next fetch: rows s0 * step + rg + RG j, the pixel's units of each
+    int fy = s0 * step + rg, fu = 0;
+    int64_t fp = int64_t(fy) * g.w + x - sp.first;
+    auto fetch = [&](StripUnit<U>& u) {
+        strip_load<U>(u, gp, fp * sp.spp + fu * U, xin && fy <= ylast && fp >= 0 && fp < sp.count);
+        if (++fu == upr) {
+            fu = 0;
+            fy += RG;
+            fp += int64_t(RG) * g.w;
+        }
+    };
+    const int cell = lane >> sh, sub = lane & (step - 1);
+    const int passes = (L::kSlots + step - 1) >> sh;
+    auto add = [&](float2* e, float2 prev, float h, float l) {
+        if (h == 0.0f && l == 0.0f) return;
+        df_add(prev.x, prev.y, h);
+        prev.y += l;
+        *e = prev;
+    };
+    const float inv_w = inv_step * inv_step;
+
+    StripUnit<U> a, b;
+    fetch(a);
+    fetch(b);
+    for (int s = s0; s < s1; ++s) {
+        // the node row above (s) uses the half s & 1 of every record, the one below the other half;
+        // rows outside [r0, r1) are left out
+        const int half = s & 1;
+        const bool up = s >= r0, down = s + 1 < r1;
+        for (int y = s * step + rg; y < imins((s + 1) * step, g.h); y += RG) {
+            const int k = y - s * step;
+            const uint32_t iu = up ? uint32_t(step - k) : 0u, id = down ? uint32_t(k) : 0u;
+            const uint32_t iw = half ? id | (iu << 16) : iu | (id << 16);
+            const float wu = float(iu) * inv_step, wd = float(id) * inv_step;
+            const float wa = half ? wd : wu, wb = half ? wu : wd;
+            constexpr int N = U >= 2 ? 2 : 1;
+            for (int t = 0; t < upr; ++t) {
+                const StripUnit<U> c = a;
+                a = b;
+                fetch(b);
+                // a node row's own image row, and the strips at the block's ends, feed one node row
+                auto go = [&](auto set, auto both, float2* to, float w0, float w1) {
+#pragma unroll
+                    for (int i = 0; i < U; i += N)
+                        strip_update<DIMS, decltype(set)::value, N, decltype(both)::value>(wgt, to, c.key + i, c.y + i, w0,
+                                                                                        w1, iw);
+                };
+                using Set0 = std::integral_constant<int, strip_set<DIMS>(0)>;
+                using Set1 = std::integral_constant<int, strip_set<DIMS>(1)>;
+                if (iu && id) {
+                    if (ds == 0) go(Set0{}, std::true_type{}, sums, wa, wb);
+                    else go(Set1{}, std::true_type{}, sums, wa, wb);
+                } else if (iu | id) {
+                    float2* to = sums + ((iu != 0) == (half == 0) ? 0 : L::kHalf);
+                    const float w0 = iu ? wu : wd;
+                    if (ds == 0) go(Set0{}, std::false_type{}, to, w0, 0.0f);
+                    else go(Set1{}, std::false_type{}, to, w0, 0.0f);
+                }
+            }
+        }
+        if (!up) continue;  // the strip above the block's first node row: nothing complete yet
+        // ---- node row s is complete. Lanes over the segment's cells and `step` slots at a time;
+        // column c of a cell adds (step - c) / step of its bin to the node on the cell's left and
+        // c / step to the one on its right (rotated by lane: the lanes read different banks), and
+        // the bin is cleared for the node row after the next. ----
+        __syncthreads();
+        float2* es = edge_s + half * 2 * NC * L::kSlots;
+        uint32_t* ew = edge_w + half * 2 * NC * L::kSlots;
+        float2* row = grid + int64_t(s) * g.nodes_x * kDeps * kDepStride;
+        const int node = c0 + cw * cells + cell;  // on the cell's left
+        for (int ps = rg * 2 + ds; ps < passes; ps += RG * 2) {
+            const int slot = (ps << sh) + sub;
+            const int en = slot < L::kSlots ? s_entry[slot] : -1;
+            const bool wr = en >= 0 && cell > 0 && node < g.nodes_x;
+            float2* e = row + int64_t(node) * kDeps * kDepStride + en;
+            float2 pw = make_float2(0.0f, 0.0f), py = pw;
+            if (wr && !sp.fresh) {
+                pw = e[0];
+                py = e[16];
+            }
+            uint32_t wl = 0, wr_ = 0;
+            float lh = 0.0f, ll = 0.0f, rh = 0.0f, rl = 0.0f;
+            if (en >= 0) {
+                for (int i = 0; i < step; ++i) {
+                    const int c = (i + lane) & (step - 1);
+                    const int at = slot * 32 + (cell << sh) + c;
+                    const float fr = float(c) * inv_step, fl = float(step - c) * inv_step;
+#pragma unroll
+                    for (int r = 0; r < RG; ++r) {
+                        float2* sv = sums_of(r * NC + cw) + half * L::kHalf + at;
+                        uint16_t* wv = reinterpret_cast<uint16_t*>(weights_of(r * NC + cw)) + 2 * at + half;
+                        const float2 v = *sv;
+                        const uint32_t w = *wv;
+                        *sv = make_float2(0.0f, 0.0f);
+                        *wv = 0;
+                        wl += w * uint32_t(step - c);
+                        wr_ += w * uint32_t(c);
+                        df_add_scaled(lh, ll, fl, v.x, v.y);
+                        df_add_scaled(rh, rl, fr, v.x, v.y);
+                    }
+                }
+            }
+            if (en >= 0 && cell == 0) {
+                es[cw * L::kSlots + slot] = make_float2(lh, ll);
+                ew[cw * L::kSlots + slot] = wl;
+            }
+            if (en >= 0 && cell == cells - 1) {
+                es[(NC + cw) * L::kSlots + slot] = make_float2(rh, rl);
+                ew[(NC + cw) * L::kSlots + slot] = wr_;
+            }
+            if (cells > 1) {  // the part of the cell on the node's left
+                const float ph = __shfl_up_sync(0xffffffffu, rh, step), pl = __shfl_up_sync(0xffffffffu, rl, step);
+                wl += __shfl_up_sync(0xffffffffu, wr_, step);
+                df_add(lh, ll, ph);
+                ll += pl;
+                if (wr) {
+                    const float2 v = int_weight_df(wl, inv_w);
+                    add(e, pw, v.x, v.y);
+                    add(e + 16, py, lh, ll);
+                }
+            }
+        }
+        __syncthreads();
+        // the nodes between two segments, and at the image's edges the block's first and last node
+        const bool last = (c0 + nb + 1) * step >= g.w;
+        for (int q = threadIdx.x; q < (NC + 1) * L::kSlots; q += NT) {
+            const int seg = q / L::kSlots, slot = q % L::kSlots;
+            const int en = s_entry[slot], nd = c0 + seg * cells;
+            if (en < 0 || nd >= g.nodes_x || (seg == 0 && cb > 0) || (seg == NC && !last)) continue;
+            float2* e = row + int64_t(nd) * kDeps * kDepStride + en;
+            float2 pw = make_float2(0.0f, 0.0f), py = pw;
+            if (!sp.fresh) {
+                pw = e[0];
+                py = e[16];
+            }
+            float2 v = make_float2(0.0f, 0.0f);
+            uint32_t w = 0;
+            if (seg > 0) {
+                v = es[(NC + seg - 1) * L::kSlots + slot];
+                w = ew[(NC + seg - 1) * L::kSlots + slot];
+            }
+            if (seg < NC) {
+                const float2 l = es[seg * L::kSlots + slot];
+                df_add(v.x, v.y, l.x);
+                v.y += l.y;
+                w += ew[seg * L::kSlots + slot];
+            }
+            const float2 wv = int_weight_df(w, inv_w);
+            add(e, pw, wv.x, wv.y);
+            add(e + 16, py, v.x, v.y);
+        }
+    }
+}
+
 }  // namespace
 
 namespace {
@@ -1195,6 +1535,67 @@ cudaError_t launch_random_shape(Job& j, const RandParams& rp, const GridPrep& gp
     }
 }
 
+template <int NC, int RG, int U, int DIMS>
+cudaError_t launch_strips_unit(Job& j, const StripParams& sp, unsigned blocks, float2* target, const GridPrep& gp) {
+    constexpr int smem = NC * RG * StripLayout<DIMS>::kWarpBytes + StripLayout<DIMS>::edge_bytes(NC);
+    const cudaError_t e = cudaFuncSetAttribute(k_grid_strips<NC, RG, U, DIMS>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    k_grid_strips<NC, RG, U, DIMS><<<blocks, NC * RG * 64, smem, j.stream>>>(sp, target, gp);
+    j.launches += 1;
+    return cudaGetLastError();
+}
+
+// Blocks of NC * 32 columns and `len` node rows (one more strip to walk than node rows), one block per
+// SM by shared memory: the len whose waves of blocks walk the fewest strips.
+constexpr int kStripSms = 152;
+template <int NC>
+int64_t strip_plan(StripParams& sp) {
+    const int nb = NC * 32 / sp.g.step - 1;
+    if (nb < 1) return INT64_MAX;
+    // blocks of nb + 1 cells, each overlapping the one before by a cell
+    const int cells = (sp.g.w + sp.g.step - 1) / sp.g.step;
+    sp.col_blocks = std::max(1, (cells - 1 + nb - 1) / nb);
+    const int rows = sp.ny1 - sp.ny0;
+    int64_t best = INT64_MAX;
+    for (int len = 1; len <= rows; ++len) {
+        const int64_t blocks = int64_t(sp.col_blocks) * ((rows + len - 1) / len);
+        const int64_t cost = (blocks + kStripSms - 1) / kStripSms * (len + 1);
+        if (cost < best) {
+            best = cost;
+            sp.len = len;
+        }
+    }
+    return best;
+}
+
+// Units of 8 samples (a 32-byte sector of keys and one of luminances per lane) or 4 where the samples
+// per pixel and the planes' alignment allow, else single samples.
+template <int NC, int RG, int DIMS>
+cudaError_t launch_strips_shape(Job& j, const StripParams& sp, float2* target, const GridPrep& gp) {
+    const bool aligned = (reinterpret_cast<uintptr_t>(gp.key) & 15u) == 0 && (reinterpret_cast<uintptr_t>(gp.lum) & 15u) == 0;
+    const int rows = sp.ny1 - sp.ny0;
+    const unsigned blocks = unsigned(sp.col_blocks) * unsigned((rows + sp.len - 1) / sp.len);
+    if (aligned && sp.spp % 8 == 0) return launch_strips_unit<NC, RG, 8, DIMS>(j, sp, blocks, target, gp);
+    if (aligned && sp.spp % 4 == 0) return launch_strips_unit<NC, RG, 4, DIMS>(j, sp, blocks, target, gp);
+    return launch_strips_unit<NC, RG, 1, DIMS>(j, sp, blocks, target, gp);
+}
+
+// NC column segments and RG row groups, two warps each (one per dimension set): bins of 44 KB per
+// segment and group without the environment dimension, 55 KB with it, so at most four (three).
+// Two row groups halve the rows a warp walks but their blocks repeat a cell in 8 (NC = 2) instead of
+// 16 columns: taken where they need no more strips than the wide blocks, on images of a few
+// blocks (64x48: 17 us, wide 26 us; 1080p16: 0.47 ms, wide 0.39 ms).
+template <int DIMS>
+cudaError_t launch_strips_dims(Job& j, const StripParams& sp, float2* target, const GridPrep& gp) {
+    constexpr int NC = DIMS == kAllDims ? 3 : 4;
+    StripParams wide = sp, tall = sp;
+    const int64_t cw = strip_plan<NC>(wide), ct = strip_plan<2>(tall);
+    if (NC == 4 && sp.g.step >= 2 && ct != INT64_MAX && ct <= cw)
+        return launch_strips_shape<2, NC == 4 ? 2 : 1, DIMS>(j, tall, target, gp);
+    return launch_strips_shape<NC, 1, DIMS>(j, wide, target, gp);
+}
+
 }  // namespace
 
 // Where a fast-mode push adds its bins. The reference adds each pass's grid to the frame grid at the
@@ -1223,6 +1624,7 @@ static cudaError_t grid_target(Job& j, float2** out) {
 cudaError_t launch_grid_fast(Job& j, const DeviceSamples& s, int64_t first, int64_t count, const GridPrep& gp,
                              int32_t spp, int32_t max_count, int64_t total_samples, const int64_t* d_max_count) {
     float2* target = nullptr;
+    const bool fresh = j.cfg.rpf_shrinkage_scale > 0.0f && j.grid_fresh;  // grid_target clears the frame grid
     if (const cudaError_t e0 = grid_target(j, &target); e0 != cudaSuccess) return e0;
     const int step = j.g.step;
     const bool pow2 = (step & (step - 1)) == 0;
@@ -1296,9 +1698,19 @@ cudaError_t launch_grid_fast(Job& j, const DeviceSamples& s, int64_t first, int6
     // a lane takes at most 1/32 of a chunk's (up to 32 segments) quads plus one, so at most
     // side^2 M / 32 + 10 samples per chunk of 32 support rows.
     const bool default_shape = j.grid_shape == 0 || j.grid_shape == 6;
-    const double side = double(2 * step + 3), units = double(step) * double(step);
+    const double units = double(step) * double(step);
+    const double side = double(2 * step + 3);
     const double chunks = std::ceil(side / 32.0);
     auto counts_fit = [&](double m) { return (side * side * m / 32.0 + 10.0 * chunks) * units < 65536.0; };
+    // 16-bit lane sums: a column's row factors sum to at most step^2 units per sample of a pixel
+    if (int_w && default_shape && spp > 0 && step <= 32 && units * double(spp) < 65536.0 &&
+        gpar.count_nodes < (int64_t(1) << 30)) {
+        int sh = 0;
+        while ((1 << sh) < step) ++sh;
+        const int ny0 = int(gpar.node0 / j.g.nodes_x), ny1 = ny0 + int(gpar.count_nodes / j.g.nodes_x);
+        const StripParams sp{j.g, first, count, ny0, ny1, 0, 0, spp, sh, fresh ? 1 : 0};
+        return env ? launch_strips_dims<kAllDims>(j, sp, target, gp) : launch_strips_dims<kNoEnvDims>(j, sp, target, gp);
+    }
     if (int_w && default_shape) {
         if (spp > 0) {
             if ((double(sup + 3) * double(sup + 3) * double(spp) / 32.0 + 8.0) * units < 65536.0)

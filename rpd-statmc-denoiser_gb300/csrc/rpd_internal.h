@@ -296,18 +296,18 @@ struct GridPrep {
                               // (null for uniform pushes, where the column follows from the index)
     int width;
 };
-// Sample key: bits 0-3 lens bin, 4-7 brdf bin, 8-11 light_uv bin, 12-15 environment bin,
-// 16-19 light index, 20 rr survived; bits 21-27 the valid flags of pixel, lens, brdf,
-// light_uv, light_select, environment, rr (after dropping flags whose plane is absent).
-constexpr int kKeyValidShift = 21;
-__host__ __device__ constexpr uint32_t key_valid_bit(int group) {
+// Sample key: one 5-bit field per random dimension in the order of the classes (brdf, lens, light_uv,
+// environment, light_select at bits 0, 5, 10, 15, 20): the bin 0-15, or 16 when the sample does not
+// carry the dimension (a flag whose plane is absent counts as clear); bits 25-26 rr: 0 ended, 1
+// survived, 2 not carried; bit 27 set when the screen position is not valid. A field indexes a
+// dimension's 17 bins directly, the last one a sink.
+__host__ __device__ constexpr int key_shift(int group) { return 5 * (group - 1); }  // groups 1-6
+__host__ __device__ constexpr uint32_t key_absent_bit(int group) {
     // group 0 pixel, 1 brdf, 2 lens, 3 light_uv, 4 environment, 5 light_select, 6 rr
-    return group == 0 ? 1u << 21 : group == 1 ? 1u << 23 : group == 2 ? 1u << 22 : group == 3 ? 1u << 24
-         : group == 4 ? 1u << 26 : group == 5 ? 1u << 25 : 1u << 27;
+    return group == 0 ? 1u << 27 : group == 6 ? 1u << 26 : 16u << key_shift(group);
 }
-__host__ __device__ constexpr int key_bin_shift(int group) {
-    return group == 1 ? 4 : group == 2 ? 0 : group == 3 ? 8 : group == 4 ? 12 : 16;
-}
+constexpr uint32_t kKeyNone = key_absent_bit(0) | key_absent_bit(1) | key_absent_bit(2) | key_absent_bit(3) |
+                              key_absent_bit(4) | key_absent_bit(5) | key_absent_bit(6);
 
 cudaError_t launch_encode_samples16(const DeviceSamples& in, int64_t n_samples, int64_t n_pixels,
                                     const DeviceSamples16& out, cudaStream_t stream);
