@@ -97,7 +97,7 @@ uint64_t plan(const Geometry& g, PixelPlanes& p, NodePlanes& n, float* (*cls)[5]
     L.add(p.slow, np);
     L.add(p.alloc_state, np);
     L.add(p.alloc_work, int64_t(allocator_work_bytes(np)));
-    L.add(p.counters, RPD_COUNTER_COUNT_);
+    L.add(p.counters, RPD_COUNTER_COUNT_ + 1);  // and the grid pass's odd-node count
     L.add(n.grid, nn * kDeps * kDepStride);
     L.add(n.pass_grid, nn * kDeps * kDepStride);
     for (int f = 0; f < N_FIELDS; ++f) L.add(n.field[f], nn);
@@ -1010,6 +1010,8 @@ static int push_tail(Job* j, DeviceSamples& d, int64_t first, int64_t count, int
     if (rpd && !d.category) return fail(RPD_ERR_INVALID_ARGUMENT, "category plane is required when RPD is enabled");
     GridPrep gp{};
     gp.width = j->g.w;
+    const int sup = j->g.support;
+    gp.bin_pixels = sup >= 4 && (sup & (sup - 1)) == 0 ? sup / 4 : 1;
     const bool fast_grid = rpd && !j->exact_grid;
     int64_t nsamp = total;
     if (fast_grid) {

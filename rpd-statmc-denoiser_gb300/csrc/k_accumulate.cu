@@ -155,18 +155,29 @@ __device__ __forceinline__ bool markstein_ok(float x) { return x == 0.0f || fabs
 // int(u * 4) = q >> 14, already within 0..3 (core/stats.h:166-168)
 __device__ __forceinline__ uint32_t bin2d_q(uint16_t qu, uint16_t qv) { return uint32_t(qv >> 14) * 4u + uint32_t(qu >> 14); }
 
+// The samples of one validity pattern (pat, 0: none yet): count, sum y and sum y^2 as double-floats.
+struct PatternSums {
+    uint32_t pat;
+    float c, s1h, s1l, s2h, s2l;
+    __device__ __forceinline__ void add(float y, float y2, float y2e) {
+        c += 1.0f;
+        df_add(s1h, s1l, y);
+        df_add(s2h, s2l, y2);
+        s2l += y2e;
+    }
+};
+
 // Per-pixel running state of the statistics pass.
 struct PixelAcc {
     float mean, m2;
     int n;
     float cm[3], sm[3], sq[3], rad[3], nor[3], alb[3], dep;
     int hits, nsamples;
-    // validity-class sums for the grid pass: samples whose class bits equal the pixel's
-    // pattern (the first nonzero class bits) share one set of sums; others go to per-class
-    // sums and make the pixel deviant
-    uint8_t pat;
-    bool have_pat, dev;
-    float pc, p1h, p1l, p2h, p2l;
+    // pattern sums for the grid pass: the samples with the same class bits share one set of sums,
+    // for the pixel's first kPatterns such patterns; samples of a further one go to per-class sums
+    // and make the pixel deviant
+    PatternSums pt[kPatterns];
+    bool dev;
     // the per-class sums [class][count, s1 hi, s1 lo, s2 hi, s2 lo] of a deviant pixel, in the
     // thread's local memory (written only once the pixel deviates, which is rare): held in
     // registers they would cost 35 registers through the whole sample loop
@@ -174,13 +185,121 @@ struct PixelAcc {
     uint8_t pflags;
 };
 
+// The packed random-dimension bins of a sample with (masked) flags fm (Dependency2D::add,
+// core/stats.h:166-168).
+template <bool COMPACT_IN>
+__device__ __forceinline__ uint32_t sample_key(const SampleIn& in, uint8_t fm) {
+    uint32_t key;
+    if (COMPACT_IN) {
+        key = (fm & RPD_SAMPLE_BRDF_VALID) ? in.bins & 0x1fu : key_absent_bit(1);
+        key |= (fm & RPD_SAMPLE_LENS_VALID) ? in.bins & (0x1fu << 5) : key_absent_bit(2);
+        key |= (fm & RPD_SAMPLE_LIGHT_VALID) ? in.bins & (0x1fu << 10) : key_absent_bit(3);
+        key |= (fm & RPD_SAMPLE_ENV_VALID) ? in.bins & (0x1fu << 15) : key_absent_bit(4);
+    } else {
+        key = (fm & RPD_SAMPLE_BRDF_VALID) ? uint32_t(bin2d_k(in.bu[0], in.bu[1])) : key_absent_bit(1);
+        key |= (fm & RPD_SAMPLE_LENS_VALID) ? uint32_t(bin2d_k(in.lu[0], in.lu[1])) << 5 : key_absent_bit(2);
+        key |= (fm & RPD_SAMPLE_LIGHT_VALID) ? uint32_t(bin2d_k(in.liu[0], in.liu[1])) << 10 : key_absent_bit(3);
+        key |= (fm & RPD_SAMPLE_ENV_VALID) ? uint32_t(bin2d_k(in.eu[0], in.eu[1])) << 15 : key_absent_bit(4);
+    }
+    key |= (fm & RPD_SAMPLE_LIGHT_SELECT_VALID) ? uint32_t(in.cat & RPD_CATEGORY_LIGHT_INDEX_MASK) << 20 : key_absent_bit(5);
+    key |= (fm & RPD_SAMPLE_RR_VALID) ? ((in.cat & RPD_CATEGORY_RR_SURVIVED) ? 1u << 25 : 0u) : key_absent_bit(6);
+    key |= (fm & RPD_SAMPLE_PIXEL_VALID) ? 0u : key_absent_bit(0);
+    return key;
+}
+
+// A finite sample's luminance into its pixel's pattern sums. A tracer's pixels hold a few patterns (all
+// dimensions, paths that ended before Russian roulette, paths that ended at the first hit): with
+// one pattern in registers and the rest added class by class in local memory, a 1920x1080x16
+// frame of such samples took 1.71 ms in this pass, with three patterns in registers 0.99 ms (0.64
+// ms for a frame of a single pattern).
+template <typename Acc>
+__device__ __forceinline__ void class_add(Acc& a, uint8_t fm, float lum) {
+    const uint32_t bits = fm & 0xfeu;
+    if (bits == 0u) return;  // no validity class: nothing for the grid's totals
+    const float y2 = lum * lum;
+    const float y2e = __fmaf_rn(lum, lum, -y2);
+    // (selects, not branches: the compiler would merge three branches into one over an array in local
+    // memory)
+    if (a.pt[0].pat == 0u) a.pt[0].pat = bits;
+    if (a.pt[0].pat == bits) {
+        a.pt[0].add(lum, y2, y2e);
+        return;
+    }
+    if (a.pt[1].pat == 0u) a.pt[1].pat = bits;
+    else if (a.pt[1].pat != bits && a.pt[2].pat == 0u) a.pt[2].pat = bits;
+    const bool one = a.pt[1].pat == bits;
+    if (one || a.pt[2].pat == bits) {
+        PatternSums t;
+        t.c = one ? a.pt[1].c : a.pt[2].c;
+        t.s1h = one ? a.pt[1].s1h : a.pt[2].s1h;
+        t.s1l = one ? a.pt[1].s1l : a.pt[2].s1l;
+        t.s2h = one ? a.pt[1].s2h : a.pt[2].s2h;
+        t.s2l = one ? a.pt[1].s2l : a.pt[2].s2l;
+        t.add(lum, y2, y2e);
+        a.pt[1].c = one ? t.c : a.pt[1].c;
+        a.pt[1].s1h = one ? t.s1h : a.pt[1].s1h;
+        a.pt[1].s1l = one ? t.s1l : a.pt[1].s1l;
+        a.pt[1].s2h = one ? t.s2h : a.pt[1].s2h;
+        a.pt[1].s2l = one ? t.s2l : a.pt[1].s2l;
+        a.pt[2].c = one ? a.pt[2].c : t.c;
+        a.pt[2].s1h = one ? a.pt[2].s1h : t.s1h;
+        a.pt[2].s1l = one ? a.pt[2].s1l : t.s1l;
+        a.pt[2].s2h = one ? a.pt[2].s2h : t.s2h;
+        a.pt[2].s2l = one ? a.pt[2].s2l : t.s2l;
+        return;
+    }
+    if (!a.dev) {
+        a.dev = true;
+        for (int q = 0; q < kClasses * 5; ++q) a.cs[q] = 0.0f;
+    }
+    for (int c = 0; c < kClasses; ++c) {
+        if (!(bits & class_bit(c))) continue;
+        float* e = a.cs + 5 * c;
+        float h1 = e[1], l1 = e[2], h2 = e[3], l2 = e[4];
+        df_add(h1, l1, lum);
+        df_add(h2, l2, y2);
+        l2 += y2e;
+        e[0] += 1.0f;
+        e[1] = h1;
+        e[2] = l1;
+        e[3] = h2;
+        e[4] = l2;
+    }
+}
+
+// Is a sample at offset f = fl(x + u) - x of pixel x in the pixel's own screen bin at every node? With a
+// power-of-two support 4 <= S <= 2^11 the bin is floor(fl(fl(x + u) - left) / (S/4)) (the division
+// and the x4 are power-of-two scalings; left is an integer): fl(X - left) is exact for left >= 0,
+// and for the first node row/column (left = -S/2, X + S/2 < 2^12) it moves by at most 2^-13
+// (main.cpp:352-356, core/stats.h:166-167). So it is whenever f lies in [0, 1 - 2^-12], or the
+// position at least a pixel inside the bin's bin_pixels pixels.
+__device__ __forceinline__ bool in_own_bin(float f, float x, int bin_pixels) {
+    const float at = float(int(x) & (bin_pixels - 1)) + f;
+    return (f >= 0.0f || at >= 1.0f) && (f <= kUniformMax || at <= float(bin_pixels - 1));
+}
+
+// A finite sample's screen position: does it stay in its pixel's bin, does a random dimension come
+// without one.
+__device__ __forceinline__ void screen_flags(const SampleIn& in, uint8_t fm, float fx, float fy, int bin_pixels,
+                                             uint8_t& pflags) {
+    if (fm & RPD_SAMPLE_PIXEL_VALID) {
+        const float jx = (fx + in.pu[0]) - fx, jy = (fy + in.pu[1]) - fy;
+        if (!(jx >= 0.0f && jx <= kUniformMax && jy >= 0.0f && jy <= kUniformMax)) {
+            if (!(in_own_bin(jx, fx, bin_pixels) && in_own_bin(jy, fy, bin_pixels))) pflags &= uint8_t(~kPixUniform);
+        }
+    } else if (fm & (RPD_SAMPLE_LENS_VALID | RPD_SAMPLE_BRDF_VALID | RPD_SAMPLE_LIGHT_VALID | RPD_SAMPLE_ENV_VALID |
+                     RPD_SAMPLE_LIGHT_SELECT_VALID | RPD_SAMPLE_RR_VALID)) {
+        pflags |= kPixMixed;  // a random dimension without the screen position
+    }
+}
+
 // COMPACT_IN: a sample decoded from the compact planes. Its radiance is the square of a
 // non-negative half, so sqrt(max(0, L)) is exactly that half (in.root), no quotient's dividend is
 // -0, and the random-dimension bins come with it (in.bins).
 template <bool COMPACT_IN = false>
 __device__ __forceinline__ void process_sample(PixelAcc& a, const SampleIn& in, bool per_sample_albedo,
                                                const float* palb, bool prep, uint8_t plane_mask, float fx,
-                                               float fy, float& lum_out, uint32_t& key_out) {
+                                               float fy, int bin_pixels, float& lum_out, uint32_t& key_out) {
     if (in.f & RPD_SAMPLE_HIT) {  // main.cpp:572-576
         ++a.hits;
         for (int c = 0; c < 3; ++c) a.nor[c] += in.n[c];
@@ -241,69 +360,9 @@ __device__ __forceinline__ void process_sample(PixelAcc& a, const SampleIn& in, 
     key_out = kKeyNone;
     if (!prep) return;
     const uint8_t fm = in.f & plane_mask;
-    // packed random-dimension bins (Dependency2D::add, core/stats.h:166-168)
-    uint32_t key;
-    if (COMPACT_IN) {
-        key = (fm & RPD_SAMPLE_BRDF_VALID) ? in.bins & 0x1fu : key_absent_bit(1);
-        key |= (fm & RPD_SAMPLE_LENS_VALID) ? in.bins & (0x1fu << 5) : key_absent_bit(2);
-        key |= (fm & RPD_SAMPLE_LIGHT_VALID) ? in.bins & (0x1fu << 10) : key_absent_bit(3);
-        key |= (fm & RPD_SAMPLE_ENV_VALID) ? in.bins & (0x1fu << 15) : key_absent_bit(4);
-    } else {
-        key = (fm & RPD_SAMPLE_BRDF_VALID) ? uint32_t(bin2d_k(in.bu[0], in.bu[1])) : key_absent_bit(1);
-        key |= (fm & RPD_SAMPLE_LENS_VALID) ? uint32_t(bin2d_k(in.lu[0], in.lu[1])) << 5 : key_absent_bit(2);
-        key |= (fm & RPD_SAMPLE_LIGHT_VALID) ? uint32_t(bin2d_k(in.liu[0], in.liu[1])) << 10 : key_absent_bit(3);
-        key |= (fm & RPD_SAMPLE_ENV_VALID) ? uint32_t(bin2d_k(in.eu[0], in.eu[1])) << 15 : key_absent_bit(4);
-    }
-    key |= (fm & RPD_SAMPLE_LIGHT_SELECT_VALID) ? uint32_t(in.cat & RPD_CATEGORY_LIGHT_INDEX_MASK) << 20 : key_absent_bit(5);
-    key |= (fm & RPD_SAMPLE_RR_VALID) ? ((in.cat & RPD_CATEGORY_RR_SURVIVED) ? 1u << 25 : 0u) : key_absent_bit(6);
-    key |= (fm & RPD_SAMPLE_PIXEL_VALID) ? 0u : key_absent_bit(0);
-    key_out = key;
-    const uint8_t cls_bits = fm & 0xfe;
-    const float y2 = lum * lum;
-    const float y2e = __fmaf_rn(lum, lum, -y2);
-    if (cls_bits != 0 && !a.have_pat) {
-        a.have_pat = true;
-        a.pat = cls_bits;
-    }
-    if (cls_bits == 0) {
-        // no validity class: nothing for the grid's totals
-    } else if (cls_bits == a.pat) {
-        a.pc += 1.0f;
-        df_add(a.p1h, a.p1l, lum);
-        df_add(a.p2h, a.p2l, y2);
-        a.p2l += y2e;
-    } else {
-        if (!a.dev) {
-            a.dev = true;
-            for (int q = 0; q < kClasses * 5; ++q) a.cs[q] = 0.0f;
-        }
-        for (int c = 0; c < kClasses; ++c) {
-            if (!(cls_bits & class_bit(c))) continue;
-            float* e = a.cs + 5 * c;
-            float h1 = e[1], l1 = e[2], h2 = e[3], l2 = e[4];
-            df_add(h1, l1, lum);
-            df_add(h2, l2, y2);
-            l2 += y2e;
-            e[0] += 1.0f;
-            e[1] = h1;
-            e[2] = l1;
-            e[3] = h2;
-            e[4] = l2;
-        }
-    }
-    if (fm & RPD_SAMPLE_PIXEL_VALID) {
-        // the screen position stays inside the pixel: with a power-of-two support 4 <= S <= 2^11
-        // the screen bin is floor(fl(fl(x + u) - left) / (S/4)) (the division and the x4 are
-        // power-of-two scalings; left is an integer), the pixel's own bin whenever
-        // f = fl(x + u) - x lies in [0, 1 - 2^-12]: fl(X - left) is exact for left >= 0, and for
-        // the first node row/column (left = -S/2, X + S/2 < 2^12) it moves by at most 2^-13
-        // (main.cpp:352-356, core/stats.h:166-167)
-        const float jx = (fx + in.pu[0]) - fx, jy = (fy + in.pu[1]) - fy;
-        if (!(jx >= 0.0f && jx <= kUniformMax && jy >= 0.0f && jy <= kUniformMax)) a.pflags &= uint8_t(~kPixUniform);
-    } else if (fm & (RPD_SAMPLE_LENS_VALID | RPD_SAMPLE_BRDF_VALID | RPD_SAMPLE_LIGHT_VALID | RPD_SAMPLE_ENV_VALID |
-                     RPD_SAMPLE_LIGHT_SELECT_VALID | RPD_SAMPLE_RR_VALID)) {
-        a.pflags |= kPixMixed;  // a random dimension without the screen position
-    }
+    key_out = sample_key<COMPACT_IN>(in, fm);
+    class_add(a, fm, lum);
+    screen_flags(in, fm, fx, fy, bin_pixels, a.pflags);
 }
 
 __device__ __forceinline__ float4 ld4(const float* p, int64_t k) { return *reinterpret_cast<const float4*>(p + k); }
@@ -318,10 +377,8 @@ __device__ __forceinline__ float sq(float v) { return v * v; }
 // A pixel's running state before its first sample of the push (the class sums start empty).
 __device__ __forceinline__ void acc_init(PixelAcc& a) {
     a.pflags = kPixUniform;
-    a.have_pat = false;
-    a.dev = false;
-    a.pat = 0;
-    a.pc = a.p1h = a.p1l = a.p2h = a.p2l = 0.0f;  // the class sums are cleared when the pixel deviates
+    a.dev = false;  // the class sums are cleared when the pixel deviates
+    for (int k = 0; k < kPatterns; ++k) a.pt[k] = PatternSums{0u, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
 }
 
 // The grid-pass sums of a pixel without samples in the push.
@@ -355,6 +412,52 @@ __device__ __forceinline__ void acc_load(PixelAcc& a, const PixelPlanes& p, int6
     a.nsamples = p.sample_count[idx];
 }
 
+// The grid-pass sums of a pixel (GridPrep): its first pattern's, and either its further patterns' or, for a
+// deviant pixel, the per-class sums.
+template <typename Acc>
+__device__ __forceinline__ void store_classes(const Acc& a, const GridPrep& gp, int64_t idx, uint8_t pflags) {
+    const PatternSums& p0 = a.pt[0];
+    gp.pat4[idx] = make_float4(p0.c, p0.s1h, p0.s1l, p0.s2h);
+    uint32_t bits = p0.pat | (uint32_t(pflags | (a.dev ? kPixDeviant : 0)) << 8);
+    if (!a.dev) {
+        for (int k = 1; k < kPatterns; ++k) bits |= a.pt[k].pat << (8 * (k + 1));
+    }
+    gp.pat2[idx] = make_float2(p0.s2l, __uint_as_float(bits));
+    if (!a.dev) {
+#pragma unroll
+        for (int k = 1; k < kPatterns; ++k) {
+            const PatternSums& t = a.pt[k];
+            if (t.pat == 0u) continue;
+            gp.cls[k - 1][0][idx] = t.c;
+            gp.cls[k - 1][1][idx] = t.s1h;
+            gp.cls[k - 1][2][idx] = t.s1l;
+            gp.cls[k - 1][3][idx] = t.s2h;
+            gp.cls[k - 1][4][idx] = t.s2l;
+        }
+        return;
+    }
+    // full per-class sums: the deviating samples plus the patterns'
+    for (int c = 0; c < kClasses; ++c) {
+        const float* e = a.cs + 5 * c;
+        float h1 = e[1], l1 = e[2], h2 = e[3], l2 = e[4], cnt = e[0];
+#pragma unroll
+        for (int k = 0; k < kPatterns; ++k) {
+            const PatternSums& t = a.pt[k];
+            if (!(t.pat & class_bit(c))) continue;
+            cnt += t.c;
+            df_add(h1, l1, t.s1h);
+            l1 += t.s1l;
+            df_add(h2, l2, t.s2h);
+            l2 += t.s2l;
+        }
+        gp.cls[c][0][idx] = cnt;
+        gp.cls[c][1][idx] = h1;
+        gp.cls[c][2][idx] = l1;
+        gp.cls[c][3][idx] = h2;
+        gp.cls[c][4][idx] = l2;
+    }
+}
+
 // The pixel's statistics back to its planes, and its grid-pass sums: the pattern class's, and
 // for a deviant pixel the full per-class sums.
 __device__ __forceinline__ void acc_store(const PixelAcc& a, const PixelPlanes& p, const GridPrep& gp, int64_t idx,
@@ -373,30 +476,100 @@ __device__ __forceinline__ void acc_store(const PixelAcc& a, const PixelPlanes& 
     p.depth[idx] = a.dep;
     p.hit_count[idx] = a.hits;
     p.sample_count[idx] = a.nsamples;
-    if (prep) {
-        gp.pat4[idx] = make_float4(a.pc, a.p1h, a.p1l, a.p2h);
-        const uint32_t bits = uint32_t(a.have_pat ? a.pat : 0) |
-                              (uint32_t(a.pflags | (a.dev ? kPixDeviant : 0)) << 8);
-        gp.pat2[idx] = make_float2(a.p2l, __uint_as_float(bits));
-        if (a.dev) {
-            // full per-class sums: the deviating samples plus the pattern's
-            for (int c = 0; c < kClasses; ++c) {
-                const float* e = a.cs + 5 * c;
-                float h1 = e[1], l1 = e[2], h2 = e[3], l2 = e[4], cnt = e[0];
-                if (a.have_pat && (a.pat & class_bit(c))) {
-                    cnt += a.pc;
-                    df_add(h1, l1, a.p1h);
-                    l1 += a.p1l;
-                    df_add(h2, l2, a.p2h);
-                    l2 += a.p2l;
-                }
-                gp.cls[c][0][idx] = cnt;
-                gp.cls[c][1][idx] = h1;
-                gp.cls[c][2][idx] = l1;
-                gp.cls[c][3][idx] = h2;
-                gp.cls[c][4][idx] = l2;
-            }
+    if (prep) store_classes(a, gp, idx, a.pflags);
+}
+
+__device__ __forceinline__ uint8_t plane_mask_of(bool pu, bool lu, bool bu, bool li, bool eu) {
+    return uint8_t(0xffu & ~((pu ? 0 : RPD_SAMPLE_PIXEL_VALID) | (lu ? 0 : RPD_SAMPLE_LENS_VALID) |
+                             (bu ? 0 : RPD_SAMPLE_BRDF_VALID) | (li ? 0 : RPD_SAMPLE_LIGHT_VALID) |
+                             (eu ? 0 : RPD_SAMPLE_ENV_VALID)));
+}
+
+// What the samples of a pixel share.
+struct PixelIn {
+    bool per_sample_albedo, prep;
+    float palb[3];
+    uint8_t plane_mask;  // the flags whose planes are present
+    float fx, fy;
+    int bin_pixels;
+};
+
+template <bool COMPACT>
+__device__ __forceinline__ void load_pixel_albedo(PixelIn& px, const DeviceSamples& s, int64_t local) {
+    if (COMPACT) {
+        if (s.c16.pixel_albedo[0])
+            for (int c = 0; c < 3; ++c) px.palb[c] = h2f(s.c16.pixel_albedo[c][local]);
+    } else if (!px.per_sample_albedo && s.pixel_albedo[0]) {
+        for (int c = 0; c < 3; ++c) px.palb[c] = s.pixel_albedo[c][local];
+    }
+}
+
+// Four FP32 samples of a pixel, each plane's as one 16-byte load; flags and categories one byte each.
+struct Quad32 {
+    float4 L[3], N[3], A[3], D, PU[2], LU[2], BU[2], LI[2], EU[2];
+    uint32_t F, C;
+};
+__device__ __forceinline__ void process_quad(PixelAcc& a, const Quad32& q, const PixelIn& px, float* lum, uint32_t* key) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        SampleIn in;
+        for (int c = 0; c < 3; ++c) {
+            in.L[c] = lane4(q.L[c], i);
+            in.n[c] = lane4(q.N[c], i);
+            in.alb[c] = lane4(q.A[c], i);
         }
+        in.d = lane4(q.D, i);
+        for (int c = 0; c < 2; ++c) {
+            in.pu[c] = lane4(q.PU[c], i);
+            in.lu[c] = lane4(q.LU[c], i);
+            in.bu[c] = lane4(q.BU[c], i);
+            in.liu[c] = lane4(q.LI[c], i);
+            in.eu[c] = lane4(q.EU[c], i);
+        }
+        in.f = uint8_t(q.F >> (8 * i));
+        in.cat = uint8_t(q.C >> (8 * i));
+        process_sample(a, in, px.per_sample_albedo, px.palb, px.prep, px.plane_mask, px.fx, px.fy, px.bin_pixels, lum[i], key[i]);
+    }
+}
+
+// V compact samples of a pixel (V = 4 or 8), two per 32-bit word of each plane.
+template <int V>
+struct Words {
+    uint32_t w[V / 2];
+    __device__ __forceinline__ uint16_t at(int i) const { return uint16_t(w[i >> 1] >> (16 * (i & 1))); }
+};
+template <int V>
+struct Group16 {
+    Words<V> L[3], N[3], D, PU[2], LU[2], BU[2], LI[2], EU[2];
+    uint32_t F[V / 4], C[V / 4];
+};
+template <int V>
+__device__ __forceinline__ void process_group(PixelAcc& a, const Group16<V>& q, const PixelIn& px, float dscale, float* lum,
+                                              uint32_t* key) {
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+        SampleIn in;
+        for (int c = 0; c < 3; ++c) {
+            in.root[c] = fabsf(h2f(q.L[c].at(i)));
+            in.L[c] = sq(in.root[c]);
+            in.n[c] = snorm16(int16_t(q.N[c].at(i)));
+            in.alb[c] = 0.0f;
+        }
+        in.d = h2f(q.D.at(i)) * dscale;
+        for (int c = 0; c < 2; ++c) in.pu[c] = unorm16(q.PU[c].at(i));
+        in.bins = bin2d_q(q.BU[0].at(i), q.BU[1].at(i)) | (bin2d_q(q.LU[0].at(i), q.LU[1].at(i)) << 5) |
+                  (bin2d_q(q.LI[0].at(i), q.LI[1].at(i)) << 10) | (bin2d_q(q.EU[0].at(i), q.EU[1].at(i)) << 15);
+        in.f = uint8_t(q.F[i >> 2] >> (8 * (i & 3)));
+        in.cat = uint8_t(q.C[i >> 2] >> (8 * (i & 3)));
+        process_sample<true>(a, in, false, px.palb, px.prep, px.plane_mask, px.fx, px.fy, px.bin_pixels, lum[i], key[i]);
+    }
+}
+template <int V>
+__device__ __forceinline__ void store_prep(const GridPrep& gp, int64_t k, const float* lum, const uint32_t* key) {
+#pragma unroll
+    for (int i = 0; i < V; i += 4) {
+        *reinterpret_cast<float4*>(gp.lum + k + i) = make_float4(lum[i], lum[i + 1], lum[i + 2], lum[i + 3]);
+        *reinterpret_cast<uint4*>(gp.key + k + i) = make_uint4(key[i], key[i + 1], key[i + 2], key[i + 3]);
     }
 }
 
@@ -419,12 +592,12 @@ __global__ void __launch_bounds__(128, MINB) k_accumulate_pixels(PixelPlanes p, 
     const bool has_bu = COMPACT ? s.c16.brdf_u[0] != nullptr : s.brdf_u[0] != nullptr;
     const bool has_li = COMPACT ? s.c16.light_u[0] != nullptr : s.light_u[0] != nullptr;
     const bool has_eu = COMPACT ? s.c16.env_u[0] != nullptr : s.env_u[0] != nullptr;
-    const uint8_t plane_mask = uint8_t(0xffu & ~((has_pu ? 0 : RPD_SAMPLE_PIXEL_VALID) |
-                                                 (has_lu ? 0 : RPD_SAMPLE_LENS_VALID) |
-                                                 (has_bu ? 0 : RPD_SAMPLE_BRDF_VALID) |
-                                                 (has_li ? 0 : RPD_SAMPLE_LIGHT_VALID) |
-                                                 (has_eu ? 0 : RPD_SAMPLE_ENV_VALID)));
-    const float fx = float(idx % gp.width), fy = float(idx / gp.width);
+    PixelIn px{};
+    px.prep = prep;
+    px.plane_mask = plane_mask_of(has_pu, has_lu, has_bu, has_li, has_eu);
+    px.fx = float(idx % gp.width);
+    px.fy = float(idx / gp.width);
+    px.bin_pixels = gp.bin_pixels;
     PixelAcc a;
     // the class sums' local array, addressed through an offset the compiler cannot fold, so that
     // it stays in local memory instead of registers
@@ -438,14 +611,8 @@ __global__ void __launch_bounds__(128, MINB) k_accumulate_pixels(PixelPlanes p, 
     // fresh: the frame's first push over every pixel, whose statistics the frame start zeroed
     if (fresh) acc_zero(a);
     else acc_load(a, p, idx);
-    const bool per_sample_albedo = !COMPACT && s.albedo[0] != nullptr;
-    float palb[3] = {0.0f, 0.0f, 0.0f};
-    if (COMPACT) {
-        if (s.c16.pixel_albedo[0])
-            for (int c = 0; c < 3; ++c) palb[c] = h2f(s.c16.pixel_albedo[c][local]);
-    } else if (!per_sample_albedo && s.pixel_albedo[0]) {
-        for (int c = 0; c < 3; ++c) palb[c] = s.pixel_albedo[c][local];
-    }
+    px.per_sample_albedo = !COMPACT && s.albedo[0] != nullptr;
+    load_pixel_albedo<COMPACT>(px, s, local);
     const bool dims = prep;  // the random dimensions are only read for the grid pass
 
     if (COMPACT) {
@@ -454,10 +621,8 @@ __global__ void __launch_bounds__(128, MINB) k_accumulate_pixels(PixelPlanes p, 
         if (VEC4) {
             // V samples per plane load: 8 (16-byte loads) when WIDE, else 4 (8-byte loads)
             constexpr int V = WIDE ? 8 : 4;
-            constexpr int NW = V / 2;  // 32-bit words per load
-            struct Wv { uint32_t w[NW]; };
             auto ldv = [](const void* ptr, int64_t k) {
-                Wv r;
+                Words<V> r;
                 if constexpr (WIDE) {
                     const uint4 v = *reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(ptr) + k);
                     r.w[0] = v.x;
@@ -471,57 +636,29 @@ __global__ void __launch_bounds__(128, MINB) k_accumulate_pixels(PixelPlanes p, 
                 }
                 return r;
             };
-            auto lane16 = [](const Wv& v, int i) { return uint16_t(v.w[i >> 1] >> (16 * (i & 1))); };
             for (int64_t k = k0; k < k1; k += V) {
-                Wv L[3], N[3], D, PU[2], LU[2], BU[2], LI[2], EU[2];
+                Group16<V> q;
+                const Words<V> z{};
                 for (int c = 0; c < 3; ++c) {
-                    L[c] = ldv(h.sqrt_radiance[c], k);
-                    N[c] = ldv(h.normal[c], k);
+                    q.L[c] = ldv(h.sqrt_radiance[c], k);
+                    q.N[c] = ldv(h.normal[c], k);
                 }
-                D = ldv(h.depth, k);
-                Wv z;
-                for (int q = 0; q < NW; ++q) z.w[q] = 0u;
+                q.D = ldv(h.depth, k);
                 for (int c = 0; c < 2; ++c) {
-                    PU[c] = (dims && has_pu) ? ldv(h.pixel_u[c], k) : z;
-                    LU[c] = (dims && has_lu) ? ldv(h.lens_u[c], k) : z;
-                    BU[c] = (dims && has_bu) ? ldv(h.brdf_u[c], k) : z;
-                    LI[c] = (dims && has_li) ? ldv(h.light_u[c], k) : z;
-                    EU[c] = (dims && has_eu) ? ldv(h.env_u[c], k) : z;
+                    q.PU[c] = (dims && has_pu) ? ldv(h.pixel_u[c], k) : z;
+                    q.LU[c] = (dims && has_lu) ? ldv(h.lens_u[c], k) : z;
+                    q.BU[c] = (dims && has_bu) ? ldv(h.brdf_u[c], k) : z;
+                    q.LI[c] = (dims && has_li) ? ldv(h.light_u[c], k) : z;
+                    q.EU[c] = (dims && has_eu) ? ldv(h.env_u[c], k) : z;
                 }
-                uint32_t F[NW / 2 > 0 ? NW / 2 : 1], Cg[NW / 2 > 0 ? NW / 2 : 1];
-                for (int q = 0; q < V / 4; ++q) {
-                    F[q] = *reinterpret_cast<const uint32_t*>(s.flags + k + 4 * q);
-                    Cg[q] = (dims && s.category) ? *reinterpret_cast<const uint32_t*>(s.category + k + 4 * q) : 0u;
+                for (int i = 0; i < V / 4; ++i) {
+                    q.F[i] = *reinterpret_cast<const uint32_t*>(s.flags + k + 4 * i);
+                    q.C[i] = (dims && s.category) ? *reinterpret_cast<const uint32_t*>(s.category + k + 4 * i) : 0u;
                 }
-                float lumv[V];
-                uint32_t keyv[V];
-                #pragma unroll
-                for (int i = 0; i < V; ++i) {
-                    SampleIn in;
-                    for (int c = 0; c < 3; ++c) {
-                        in.root[c] = fabsf(h2f(lane16(L[c], i)));
-                        in.L[c] = sq(in.root[c]);
-                        in.n[c] = snorm16(int16_t(lane16(N[c], i)));
-                        in.alb[c] = 0.0f;
-                    }
-                    in.d = h2f(lane16(D, i)) * dscale;
-                    for (int c = 0; c < 2; ++c) in.pu[c] = unorm16(lane16(PU[c], i));
-                    in.bins = bin2d_q(lane16(BU[0], i), lane16(BU[1], i)) |
-                              (bin2d_q(lane16(LU[0], i), lane16(LU[1], i)) << 5) |
-                              (bin2d_q(lane16(LI[0], i), lane16(LI[1], i)) << 10) |
-                              (bin2d_q(lane16(EU[0], i), lane16(EU[1], i)) << 15);
-                    in.f = uint8_t(F[i >> 2] >> (8 * (i & 3)));
-                    in.cat = uint8_t(Cg[i >> 2] >> (8 * (i & 3)));
-                    process_sample<true>(a, in, false, palb, prep, plane_mask, fx, fy, lumv[i], keyv[i]);
-                }
-                if (prep) {
-                    for (int q = 0; q < V / 4; ++q) {
-                        *reinterpret_cast<float4*>(gp.lum + k + 4 * q) =
-                            make_float4(lumv[4 * q], lumv[4 * q + 1], lumv[4 * q + 2], lumv[4 * q + 3]);
-                        *reinterpret_cast<uint4*>(gp.key + k + 4 * q) =
-                            make_uint4(keyv[4 * q], keyv[4 * q + 1], keyv[4 * q + 2], keyv[4 * q + 3]);
-                    }
-                }
+                float lum[V];
+                uint32_t key[V];
+                process_group<V>(a, q, px, dscale, lum, key);
+                if (prep) store_prep<V>(gp, k, lum, key);
             }
         } else {
             for (int64_t k = k0; k < k1; ++k) {
@@ -547,7 +684,7 @@ __global__ void __launch_bounds__(128, MINB) k_accumulate_pixels(PixelPlanes p, 
                 in.cat = (dims && s.category) ? s.category[k] : 0;
                 float lum;
                 uint32_t key;
-                process_sample<true>(a, in, false, palb, prep, plane_mask, fx, fy, lum, key);
+                process_sample<true>(a, in, false, px.palb, prep, px.plane_mask, px.fx, px.fy, px.bin_pixels, lum, key);
                 if (prep) {
                     gp.lum[k] = lum;
                     gp.key[k] = key;
@@ -557,49 +694,27 @@ __global__ void __launch_bounds__(128, MINB) k_accumulate_pixels(PixelPlanes p, 
         }
     } else if (VEC4) {
         for (int64_t k = k0; k < k1; k += 4) {
-            float4 L[3], N[3], A[3], D, PU[2], LU[2], BU[2], LI[2], EU[2];
-            for (int c = 0; c < 3; ++c) {
-                L[c] = ld4(s.radiance[c], k);
-                N[c] = ld4(s.normal[c], k);
-                A[c] = per_sample_albedo ? ld4(s.albedo[c], k) : make_float4(0, 0, 0, 0);
-            }
-            D = ld4(s.depth, k);
+            Quad32 q;
             const float4 z4 = make_float4(0, 0, 0, 0);
+            for (int c = 0; c < 3; ++c) {
+                q.L[c] = ld4(s.radiance[c], k);
+                q.N[c] = ld4(s.normal[c], k);
+                q.A[c] = px.per_sample_albedo ? ld4(s.albedo[c], k) : z4;
+            }
+            q.D = ld4(s.depth, k);
             for (int c = 0; c < 2; ++c) {
-                PU[c] = (dims && s.pixel_u[0]) ? ld4(s.pixel_u[c], k) : z4;
-                LU[c] = (dims && s.lens_u[0]) ? ld4(s.lens_u[c], k) : z4;
-                BU[c] = (dims && s.brdf_u[0]) ? ld4(s.brdf_u[c], k) : z4;
-                LI[c] = (dims && s.light_u[0]) ? ld4(s.light_u[c], k) : z4;
-                EU[c] = (dims && s.env_u[0]) ? ld4(s.env_u[c], k) : z4;
+                q.PU[c] = (dims && s.pixel_u[0]) ? ld4(s.pixel_u[c], k) : z4;
+                q.LU[c] = (dims && s.lens_u[0]) ? ld4(s.lens_u[c], k) : z4;
+                q.BU[c] = (dims && s.brdf_u[0]) ? ld4(s.brdf_u[c], k) : z4;
+                q.LI[c] = (dims && s.light_u[0]) ? ld4(s.light_u[c], k) : z4;
+                q.EU[c] = (dims && s.env_u[0]) ? ld4(s.env_u[c], k) : z4;
             }
-            const uint32_t F4 = *reinterpret_cast<const uint32_t*>(s.flags + k);
-            const uint32_t C4 = (dims && s.category) ? *reinterpret_cast<const uint32_t*>(s.category + k) : 0u;
-            float lum4[4];
-            uint32_t key4[4];
-            #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                SampleIn in;
-                for (int c = 0; c < 3; ++c) {
-                    in.L[c] = lane4(L[c], i);
-                    in.n[c] = lane4(N[c], i);
-                    in.alb[c] = lane4(A[c], i);
-                }
-                in.d = lane4(D, i);
-                for (int c = 0; c < 2; ++c) {
-                    in.pu[c] = lane4(PU[c], i);
-                    in.lu[c] = lane4(LU[c], i);
-                    in.bu[c] = lane4(BU[c], i);
-                    in.liu[c] = lane4(LI[c], i);
-                    in.eu[c] = lane4(EU[c], i);
-                }
-                in.f = uint8_t(F4 >> (8 * i));
-                in.cat = uint8_t(C4 >> (8 * i));
-                process_sample(a, in, per_sample_albedo, palb, prep, plane_mask, fx, fy, lum4[i], key4[i]);
-            }
-            if (prep) {
-                *reinterpret_cast<float4*>(gp.lum + k) = make_float4(lum4[0], lum4[1], lum4[2], lum4[3]);
-                *reinterpret_cast<uint4*>(gp.key + k) = make_uint4(key4[0], key4[1], key4[2], key4[3]);
-            }
+            q.F = *reinterpret_cast<const uint32_t*>(s.flags + k);
+            q.C = (dims && s.category) ? *reinterpret_cast<const uint32_t*>(s.category + k) : 0u;
+            float lum[4];
+            uint32_t key[4];
+            process_quad(a, q, px, lum, key);
+            if (prep) store_prep<4>(gp, k, lum, key);
         }
     } else {
         for (int64_t k = k0; k < k1; ++k) {
@@ -607,7 +722,7 @@ __global__ void __launch_bounds__(128, MINB) k_accumulate_pixels(PixelPlanes p, 
             for (int c = 0; c < 3; ++c) {
                 in.L[c] = s.radiance[c][k];
                 in.n[c] = s.normal[c][k];
-                in.alb[c] = per_sample_albedo ? s.albedo[c][k] : 0.0f;
+                in.alb[c] = px.per_sample_albedo ? s.albedo[c][k] : 0.0f;
             }
             in.d = s.depth[k];
             for (int c = 0; c < 2; ++c) {
@@ -621,7 +736,7 @@ __global__ void __launch_bounds__(128, MINB) k_accumulate_pixels(PixelPlanes p, 
             in.cat = (dims && s.category) ? s.category[k] : 0;
             float lum;
             uint32_t key;
-            process_sample(a, in, per_sample_albedo, palb, prep, plane_mask, fx, fy, lum, key);
+            process_sample(a, in, px.per_sample_albedo, px.palb, prep, px.plane_mask, px.fx, px.fy, px.bin_pixels, lum, key);
             if (prep) {
                 gp.lum[k] = lum;
                 gp.key[k] = key;

@@ -32,6 +32,7 @@ namespace rpd {
 namespace {
 
 constexpr int kGroups = 7;
+constexpr int kStripSms = 152;  // GB300's SMs
 
 __device__ __forceinline__ void df_add(float& hi, float& lo, float x) {
     const float s = hi + x;
@@ -226,16 +227,16 @@ __device__ __forceinline__ float axis_factor(const GridParams& gp, int c, int n,
     return 0.0f;
 }
 
-// A pixel's pattern sums, pattern and flags (see GridPrep).
+// A pixel's first pattern's sums, its patterns and flags (see GridPrep).
 struct PixPattern {
     float c, s1h, s1l, s2h, s2l;
-    uint8_t pat, pf;
+    uint8_t pat, pf, more[kPatterns - 1];
 };
 __device__ __forceinline__ PixPattern load_pattern(const GridPrep& gp, int64_t idx) {
     const float4 a = gp.pat4[idx];
     const float2 b = gp.pat2[idx];
     const uint32_t bits = __float_as_uint(b.y);
-    return PixPattern{a.x, a.y, a.z, a.w, b.x, uint8_t(bits & 0xffu), uint8_t(bits >> 8)};
+    return PixPattern{a.x, a.y, a.z, a.w, b.x, uint8_t(bits), uint8_t(bits >> 8), {uint8_t(bits >> 16), uint8_t(bits >> 24)}};
 }
 
 // The (count, sum y hi/lo, sum y^2 hi/lo) of class c for pixel idx (see GridPrep).
@@ -243,15 +244,33 @@ __device__ __forceinline__ void class_sums(const GridPrep& gp, int c, int64_t id
                                            float* out) {
     if (pp.pf & kPixDeviant) {
         for (int f = 0; f < 5; ++f) out[f] = gp.cls[c][f][idx];
-    } else if (pp.pat & class_bit(c)) {
+        return;
+    }
+    for (int f = 0; f < 5; ++f) out[f] = 0.0f;
+    if (pp.pat & class_bit(c)) {
         out[0] = pp.c;
         out[1] = pp.s1h;
         out[2] = pp.s1l;
         out[3] = pp.s2h;
         out[4] = pp.s2l;
-    } else {
-        for (int f = 0; f < 5; ++f) out[f] = 0.0f;
     }
+    for (int k = 0; k < kPatterns - 1; ++k) {
+        if (!(pp.more[k] & class_bit(c))) continue;
+        out[0] += gp.cls[k][0][idx];
+        df_add(out[1], out[2], gp.cls[k][1][idx]);
+        out[2] += gp.cls[k][2][idx];
+        df_add(out[3], out[4], gp.cls[k][3][idx]);
+        out[4] += gp.cls[k][4][idx];
+    }
+}
+
+// The key bits that mark absent dimensions, of a sample with exactly pattern `pat`.
+__device__ __forceinline__ uint32_t pattern_absent(uint32_t pat) {
+    uint32_t a = 0u;
+#pragma unroll
+    for (int c = 0; c < kClasses; ++c)
+        if (!(pat & class_bit(c))) a |= key_absent_bit(c);
+    return a;
 }
 
 template <bool INT_W>
@@ -356,13 +375,13 @@ __global__ void __launch_bounds__(kGroups * 32) k_grid_fast(GridParams gpar, flo
     reduce_totals_into(tot_x, base + dep_x * kDepStride);
 }
 
-// ---- totals and screen bins, pattern form (the default) ----------------------------------
+// ---- totals and screen bins, pattern form (small images, other supports) ------------------
 //
 // One warp per node. Pixels of the node's pattern P0 (the pattern of its first non-deviant
 // support pixel) carry the same class sums for every class in P0, so their totals are formed
 // once (TP) and their screen bins once (bins A: per pixel for uniform pixels, sample by sample
-// otherwise); each class then takes TP and bins A if it is in P0. Every other pixel (deviant,
-// or of another pattern) goes to a list handled class by class as the per-class kernel does
+// otherwise); each class then takes TP and bins A if it is in P0. Every other pixel (of
+// several patterns, or of another one) goes to a list handled class by class as the per-class kernel does
 // (bins B). All sums are lane-private and combined in a fixed order: deterministic.
 __device__ __forceinline__ int axis_ifactor(int c, int n, int nodes, int sh) {
     // x factor * step of a power-of-two step (c < (nodes - 1) * step for every image pixel)
@@ -438,7 +457,7 @@ __global__ void __launch_bounds__(32) k_grid_screen(GridParams gpar, float2* pas
             const int64_t idx = int64_t(ylo + q / cols) * g.w + xlo + q % cols;
             if (idx >= gpar.first && idx < gpar.first + gpar.count) {
                 const uint32_t bits = __float_as_uint(gp.pat2[idx].y);
-                if (!((bits >> 8) & kPixDeviant)) pat = uint8_t(bits & 0xffu);
+                if (!((bits >> 8) & kPixDeviant) && (bits >> 16) == 0u) pat = uint8_t(bits & 0xffu);
             }
         }
         const unsigned m = __ballot_sync(0xffffffffu, pat != 0);
@@ -459,7 +478,7 @@ __global__ void __launch_bounds__(32) k_grid_screen(GridParams gpar, float2* pas
         const int64_t idx = int64_t(py) * g.w + px;
         in = q < npix && idx >= gpar.first && idx < gpar.first + gpar.count;
         if (in) pp = load_pattern(gp, idx);
-        else pp = PixPattern{0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0, 0};
+        else pp = PixPattern{0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0, 0, {0, 0}};
     };
     PixPattern nxt;
     bool nin;
@@ -480,7 +499,7 @@ __global__ void __launch_bounds__(32) k_grid_screen(GridParams gpar, float2* pas
         if (in) {
             w = weight(cx, cy);
             if (w > 1e-8f) {  // BinnedDependency::add skips w <= 1e-8 (core/stats.h:103)
-                const bool dev = (pp.pf & kPixDeviant) != 0;
+                const bool dev = (pp.pf & kPixDeviant) != 0 || pp.more[0] != 0;  // several patterns
                 if (!dev && pp.pat == P0 && pp.pat != 0) {
                     add_class(TP, w, pp.c, pp.s1h, pp.s1l, pp.s2h, pp.s2l);
                     if (p0pix) {
@@ -637,6 +656,478 @@ __global__ void __launch_bounds__(32) k_grid_screen(GridParams gpar, float2* pas
             tv.y += tl;
             *te = tv;
         }
+    }
+}
+
+// ---- totals and screen bins, strip form ----------------------------------------------------------
+//
+// For power-of-two node steps from 2 to 16 (supports from 4). A pixel's samples then share the pixel's
+// nominal screen bin (see uniform_ok), which is its quarter of the node's support in x and in y:
+// the pixels of half a cell (step / 2 rows and columns) fall in one bin of each of the cell's four
+// nodes. A lane owns a column and walks down it through the pixels' pattern sums: per half strip
+// (step / 2 rows) it sums them times the row factors of the node rows above and below, and the lanes of
+// a half cell add up their column-weighted sums, which are then one finished bin of four nodes. The
+// totals add up over the strip's two halves and the node's two cells. Each pixel is visited once (and
+// once more for the cell that neighbouring warps share) instead of once per node it supports, in
+// registers instead of lane-private bins in shared memory; warps are independent of each other.
+// A validity pattern at a time: its sums enter every class it holds. Samples outside their pixel's
+// nominal bin, and pixels with more patterns than the statistics pass keeps (deviant), are
+// k_grid_odd's. The bound is load latency (18 warps per SM, one pass over 24 bytes a pixel): with
+// k_grid_odd 0.119 ms at 1920x1080 against 0.213 ms for the pattern form; where a pixel's samples
+// hold three patterns, 0.30 against 0.82 ms.
+struct TotalsParams {
+    Geometry g;
+    int64_t first, count;
+    int ny0, ny1;    // node rows of the launch
+    int len;         // node rows of a warp
+    int col_warps;   // warps per `len` node rows
+    int sh;          // log2 of the node step
+    int fresh;       // the grid holds zeros (the frame's first push)
+    // the nodes with work for k_grid_odd: how many, and their indices
+    unsigned* odd_count;
+    int32_t* odd_nodes;
+};
+
+__host__ __device__ constexpr int dep_random(int c) { return c == 0 ? 0 : 2 * c - 1; }
+__host__ __device__ constexpr int dep_screen(int c) { return 2 * c; }
+
+// Does k_grid_odd look at a pixel with these bits (pat2.y)?
+__device__ __forceinline__ bool odd_pixel(uint32_t bits) {
+    const uint32_t pats = bits | (bits >> 16) | (bits >> 24);
+    return ((bits >> 8) & kPixDeviant) || (!((bits >> 8) & kPixUniform) && (pats & RPD_SAMPLE_PIXEL_VALID));
+}
+
+// A set of patterns, one bit each (patterns are even: bit p / 2).
+struct PatternSet {
+    uint32_t w[4] = {0u, 0u, 0u, 0u};
+    __device__ __forceinline__ void add(uint32_t p) {
+        if (p == 0u) return;
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+            if (int(p >> 6) == t) w[t] |= 1u << ((p >> 1) & 31u);
+    }
+    __device__ __forceinline__ void unite_warp() {
+#pragma unroll
+        for (int t = 0; t < 4; ++t) w[t] = __reduce_or_sync(0xffffffffu, w[t]);
+    }
+    __device__ __forceinline__ uint32_t pop() {  // the smallest, 0: empty
+        uint32_t p = 0;
+#pragma unroll
+        for (int t = 3; t >= 0; --t)
+            if (w[t]) p = uint32_t(t) * 64u + 2u * uint32_t(__ffs(w[t]) - 1);
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+            if (p && int(p >> 6) == t) w[t] &= w[t] - 1u;
+        return p;
+    }
+};
+
+// the sum of (h, l) over groups of `lanes` lanes (a power of two), in every lane
+__device__ __forceinline__ void df_group_sum(float& h, float& l, int lanes) {
+    for (int o = 1; o < lanes; o <<= 1) {
+        const float oh = __shfl_xor_sync(0xffffffffu, h, o), ol = __shfl_xor_sync(0xffffffffu, l, o);
+        df_add(h, l, oh);
+        l += ol;
+    }
+}
+__device__ __forceinline__ DF df_scaled(float a, DF b) {  // a * b
+    DF r;
+    r.h = a * b.h;
+    r.l = __fmaf_rn(a, b.l, __fmaf_rn(a, b.h, -r.h));
+    return r;
+}
+
+__global__ void __launch_bounds__(128) k_grid_totals(TotalsParams tp, float2* grid, GridPrep gp) {
+    const int lane = threadIdx.x & 31;
+    const int64_t gw = int64_t(blockIdx.x) * 4 + (threadIdx.x >> 5);
+    const Geometry& g = tp.g;
+    const int sh = tp.sh, step = g.step, half = step >> 1;
+    const int r0 = tp.ny0 + int(gw / tp.col_warps) * tp.len;
+    if (r0 >= tp.ny1) return;  // the whole warp
+    const int r1 = imins(r0 + tp.len, tp.ny1);
+    const int cells = 32 >> sh;
+    const int c0 = int(gw % tp.col_warps) * (cells - 1);  // its first cell, between nodes c0 and c0 + 1
+    const int x = c0 * step + lane;
+    const int cell = lane >> sh, col = lane & (step - 1);
+    const bool xin = x < g.w;
+    const bool last = (c0 + cells) * step >= g.w;
+    // node c0 + j, complete in this warp: both its cells are, or lie outside the image
+    auto owned = [&](int j) { return (j > 0 || c0 == 0) && (j < cells || last) && c0 + j < g.nodes_x; };
+    const float inv_step = 1.0f / float(step), inv_w = inv_step * inv_step;
+    auto inside = [&](int64_t p) { return p >= tp.first && p < tp.first + tp.count; };
+    const int s0 = imaxs(r0 - 1, 0), s1 = r1;
+    // the patterns of the warp's pixels, and the nodes (of its rows r0 .. r1 - 1) with odd pixels: the
+    // lanes' strips first, then the cells'
+    PatternSet set;
+    bool odd_prev = false;
+    for (int s = s0; s < s1; ++s) {
+        bool odd = false;
+        for (int k0 = 0; k0 < step; k0 += 4) {
+            uint32_t bits[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int y = s * step + k0 + i;
+                const int64_t p = int64_t(y) * g.w + x;
+                bits[i] = k0 + i < step && xin && y < g.h && inside(p) ? __float_as_uint(gp.pat2[p].y) : uint32_t(kPixUniform) << 8;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                odd = odd || odd_pixel(bits[i]);
+                if ((bits[i] >> 8) & kPixDeviant) continue;
+                set.add(bits[i] & 0xffu);
+                set.add((bits[i] >> 16) & 0xffu);
+                set.add(bits[i] >> 24);
+            }
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, odd || odd_prev);  // strips s - 1 and s: node row s
+        odd_prev = odd;
+        if (s < r0 || m == 0u || lane > cells || !owned(lane)) continue;
+        // node `lane`: the cells on its left and right
+        const unsigned cell_lanes = cells == 1 ? 0xffffffffu : (1u << step) - 1u;
+        const bool l = lane > 0 && ((m >> ((lane - 1) << sh)) & cell_lanes);
+        const bool r = lane < cells && ((m >> (lane << sh)) & cell_lanes);
+        if (l || r) tp.odd_nodes[atomicAdd(tp.odd_count, 1u)] = int32_t(int64_t(s) * g.nodes_x + c0 + lane);
+    }
+    set.unite_warp();
+    // column factors (in units of 1 / step) of the cell's left and right node
+    const uint32_t il = uint32_t(step - col), ir = uint32_t(col);
+    const float fl = float(il) * inv_step, fr = float(ir) * inv_step;
+    bool store_only = tp.fresh != 0;  // the grid is still zero: write instead of add
+    for (uint32_t P = set.pop(); P != 0u; P = set.pop()) {
+        const bool pix = (P & RPD_SAMPLE_PIXEL_VALID) != 0;
+        // the column's part of the next node row's totals: weights, squared weights, y, y^2
+        uint32_t nw = 0u;
+        unsigned long long nw2 = 0ull;
+        DF ny, nz;
+        for (int s = s0; s < s1; ++s) {
+            const bool up = s >= r0, down = s + 1 < r1;
+            uint32_t tw = nw;  // node row s
+            unsigned long long tw2 = nw2;
+            DF ty = ny, tz = nz;
+            nw = 0u;
+            nw2 = 0ull;
+            ny = nz = DF{};
+            for (int hs = 0; hs < 2; ++hs) {
+                uint32_t bw[2] = {0u, 0u};  // [0] the node row above, [1] below
+                DF by[2];
+                // rows in fours, their records loaded before any is used
+                for (int k0 = hs * half; k0 < (hs + 1) * half; k0 += 4) {
+                    float4 A[4];
+                    float2 B[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const int y = s * step + k0 + i;
+                        const int64_t p = int64_t(y) * g.w + x;
+                        A[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                        B[i] = make_float2(0.0f, 0.0f);
+                        if (k0 + i < (hs + 1) * half && xin && y < g.h && inside(p)) {
+                            A[i] = gp.pat4[p];
+                            B[i] = gp.pat2[p];
+                        }
+                    }
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const uint32_t bits = __float_as_uint(B[i].y);
+                        if ((bits >> 8) & kPixDeviant) continue;
+                        float4 a = A[i];
+                        float s2l = B[i].x;
+                        if ((bits & 0xffu) != P) {
+                            const int more = ((bits >> 16) & 0xffu) == P ? 0 : (bits >> 24) == P ? 1 : -1;
+                            if (more < 0) continue;
+                            const int64_t p = int64_t(s * step + k0 + i) * g.w + x;
+                            a = make_float4(gp.cls[more][0][p], gp.cls[more][1][p], gp.cls[more][2][p], gp.cls[more][3][p]);
+                            s2l = gp.cls[more][4][p];
+                        }
+                        const int k = k0 + i;
+                        const uint32_t n = uint32_t(a.x), i0 = uint32_t(step - k), i1 = uint32_t(k);
+                        const float f0 = float(i0) * inv_step, f1 = float(i1) * inv_step;
+                        bw[0] += i0 * n;
+                        bw[1] += i1 * n;
+                        tw2 += i0 * i0 * n;
+                        nw2 += i1 * i1 * n;
+                        df_add_scaled(by[0].h, by[0].l, f0, a.y, a.z);
+                        df_add_scaled(by[1].h, by[1].l, f1, a.y, a.z);
+                        df_add_scaled(tz.h, tz.l, f0, a.w, s2l);
+                        df_add_scaled(nz.h, nz.l, f1, a.w, s2l);
+                    }
+                }
+                if (!__any_sync(0xffffffffu, bw[0] != 0u)) continue;
+                tw += bw[0];
+                nw += bw[1];
+                df_add(ty.h, ty.l, by[0].h);
+                ty.l += by[0].l;
+                df_add(ny.h, ny.l, by[1].h);
+                ny.l += by[1].l;
+                if (!pix) continue;
+                // the half cell's bin of each node: quarter v * 2 + t (t: 0 left, 1 right)
+                uint32_t qw[4];
+                DF qy[4];
+#pragma unroll
+                for (int v = 0; v < 2; ++v) {
+                    qw[2 * v] = bw[v] * il;
+                    qw[2 * v + 1] = bw[v] * ir;
+                    qy[2 * v] = df_scaled(fl, by[v]);
+                    qy[2 * v + 1] = df_scaled(fr, by[v]);
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    for (int o = 1; o < half; o <<= 1) qw[q] += __shfl_xor_sync(0xffffffffu, qw[q], o);
+                    df_group_sum(qy[q].h, qy[q].l, half);
+                }
+                const int hcell = (lane >> (sh - 1)) & 1;  // left or right half of the cell
+                for (int q = lane & (half - 1); q < 4; q += half) {
+                    const int node = cell + (q & 1), row = s + (q >> 1);
+                    if (!owned(node) || !(q < 2 ? up : down)) continue;
+                    const uint32_t W = q == 0 ? qw[0] : q == 1 ? qw[1] : q == 2 ? qw[2] : qw[3];
+                    DF Y;
+                    Y.h = q == 0 ? qy[0].h : q == 1 ? qy[1].h : q == 2 ? qy[2].h : qy[3].h;
+                    Y.l = q == 0 ? qy[0].l : q == 1 ? qy[1].l : q == 2 ? qy[2].l : qy[3].l;
+                    if (W == 0u) continue;
+                    const int bin = ((q < 2 ? 2 : 0) + hs) * 4 + ((q & 1) ? 0 : 2) + hcell;
+                    const float2 wv = int_weight_df(W, inv_w);
+                    float2* e = grid + (int64_t(row) * g.nodes_x + c0 + node) * kDeps * kDepStride + bin;
+                    float2 pw[kClasses], py[kClasses];
+#pragma unroll
+                    for (int c = 0; c < kClasses; ++c) {
+                        pw[c] = py[c] = make_float2(0.0f, 0.0f);
+                        if (!(P & class_bit(c)) || store_only) continue;
+                        pw[c] = e[dep_screen(c) * kDepStride];
+                        py[c] = e[dep_screen(c) * kDepStride + 16];
+                    }
+#pragma unroll
+                    for (int c = 0; c < kClasses; ++c) {
+                        if (!(P & class_bit(c))) continue;
+                        df_add(pw[c].x, pw[c].y, wv.x);
+                        pw[c].y += wv.y;
+                        df_add(py[c].x, py[c].y, Y.h);
+                        py[c].y += Y.l;
+                        e[dep_screen(c) * kDepStride] = pw[c];
+                        e[dep_screen(c) * kDepStride + 16] = py[c];
+                    }
+                }
+            }
+            if (!up || !__any_sync(0xffffffffu, tw != 0u)) continue;
+            // node row s: per cell and side, then per node (its left cell's right part and its right
+            // cell's left part)
+            uint32_t wl = tw * il, wr = tw * ir;
+            unsigned long long w2l = tw2 * (il * il), w2r = tw2 * (ir * ir);
+            DF yl = df_scaled(fl, ty), yr = df_scaled(fr, ty), zl = df_scaled(fl, tz), zr = df_scaled(fr, tz);
+            for (int o = 1; o < step; o <<= 1) {
+                wl += __shfl_xor_sync(0xffffffffu, wl, o);
+                wr += __shfl_xor_sync(0xffffffffu, wr, o);
+                w2l += __shfl_xor_sync(0xffffffffu, w2l, o);
+                w2r += __shfl_xor_sync(0xffffffffu, w2r, o);
+            }
+            df_group_sum(yl.h, yl.l, step);
+            df_group_sum(yr.h, yr.l, step);
+            df_group_sum(zl.h, zl.l, step);
+            df_group_sum(zr.h, zr.l, step);
+            // node `cell`, on this cell's left; the lanes of the last cell also take the one on its right
+            const uint32_t aw = __shfl_up_sync(0xffffffffu, wr, step);
+            const unsigned long long aw2 = __shfl_up_sync(0xffffffffu, w2r, step);
+            const float ayh = __shfl_up_sync(0xffffffffu, yr.h, step), ayl = __shfl_up_sync(0xffffffffu, yr.l, step);
+            const float azh = __shfl_up_sync(0xffffffffu, zr.h, step), azl = __shfl_up_sync(0xffffffffu, zr.l, step);
+            for (int t = 0; t < (cell == cells - 1 ? 2 : 1); ++t) {
+                const int node = cell + t;
+                if (!owned(node)) continue;
+                uint32_t W = t ? wr : wl;
+                unsigned long long W2 = t ? w2r : w2l;
+                DF Y = t ? yr : yl, Z = t ? zr : zl;
+                if (!t && cell > 0) {
+                    W += aw;
+                    W2 += aw2;
+                    df_add(Y.h, Y.l, ayh);
+                    Y.l += ayl;
+                    df_add(Z.h, Z.l, azh);
+                    Z.l += azl;
+                }
+                if (W == 0u) continue;
+                const float w2h = __ull2float_rz(W2);
+                const float w2m = float(W2 - (unsigned long long)(w2h));
+                const float2 add[4] = {int_weight_df(W, inv_w),
+                                       make_float2(w2h * (inv_w * inv_w), w2m * (inv_w * inv_w)),
+                                       make_float2(Y.h, Y.l), make_float2(Z.h, Z.l)};
+                float2* e = grid + (int64_t(s) * g.nodes_x + c0 + node) * kDeps * kDepStride + 32;
+                for (int d = col; d < kDeps; d += step) {  // the cell's lanes take a dependency each
+                    const int c = (d + 1) >> 1;  // its class: dep_random(c) and dep_screen(c) in order
+                    if (!(P & class_bit(c)) || ((d & 1) == 0 && !pix)) continue;
+                    float2* ed = e + d * kDepStride;
+                    float2 o[4];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) o[k] = store_only ? make_float2(0.0f, 0.0f) : ed[k];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        df_add(o[k].x, o[k].y, add[k].x);
+                        o[k].y += add[k].y;
+                        ed[k] = o[k];
+                    }
+                }
+            }
+            __syncwarp();
+        }
+        store_only = false;
+    }
+}
+
+// What k_grid_totals leaves out, one warp per node. It takes every sample of a pixel in the pixel's
+// nominal screen bin: a pixel some of whose samples may not be (a position within 2^-12 of the
+// pixel's end, or outside it) is looked over sample by sample here, and a sample that the reference
+// bins elsewhere is moved (very few are). Deviant pixels are summed class by class.
+// Blocks of one warp take the listed nodes in turn; each node is one warp's, in a fixed order.
+__device__ void odd_node(const GridParams& gpar, float2* grid, const DeviceSamples& s, const int64_t* offsets,
+                         const GridPrep& gp, int64_t node, float* sm) {
+    const int lane = threadIdx.x;
+    const Geometry& g = gpar.g;
+    const int nx = int(node % g.nodes_x), ny = int(node / g.nodes_x);
+    const int step = g.step, sh = __ffs(step) - 1;
+    const float wscale = float(step) * float(step), inv_wscale = 1.0f / wscale;
+    LaneBins<false> bins{sm, lane, wscale};
+    uint16_t* list = reinterpret_cast<uint16_t*>(sm + LaneBins<false>::kSlots * 32);
+    float2* base = grid + node * kDeps * kDepStride;
+    const float support = float(g.support);
+    const float half_support = 0.5f * support;
+    const float support_left = float(nx * step) - half_support;
+    const float support_top = float(ny * step) - half_support;
+    // the pixels the node weighs: strictly within a step of it
+    const int xlo = imaxs(0, (nx - 1) * step + 1), xhi = imins(g.w - 1, (nx + 1) * step - 1);
+    const int ylo = imaxs(0, (ny - 1) * step + 1), yhi = imins(g.h - 1, (ny + 1) * step - 1);
+    int nodd = 0;
+    bool deviants = false;
+    // one row of 2 step - 1 pixels (or two, for steps up to 8) at a time
+    const int lw = step <= 8 ? 16 : 32, rows = 32 / lw;
+    const int lx = lane & (lw - 1), lr = lane / lw;
+    for (int y0 = ylo; y0 <= yhi; y0 += rows) {
+        const int x = xlo + lx, y = y0 + lr;
+        const int64_t idx = int64_t(y) * g.w + x;
+        bool odd = false;
+        if (x <= xhi && y <= yhi && idx >= gpar.first && idx < gpar.first + gpar.count) {
+            const uint32_t bits = __float_as_uint(gp.pat2[idx].y);
+            odd = odd_pixel(bits);
+            deviants = deviants || ((bits >> 8) & kPixDeviant);
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, odd);
+        if (odd) list[nodd + __popc(m & ((1u << lane) - 1))] = uint16_t((y - ylo) * 64 + x - xlo);
+        nodd += __popc(m);
+    }
+    if (nodd == 0) return;
+    __syncwarp();
+    deviants = __any_sync(0xffffffffu, deviants);
+    auto pixel = [&](int i, int& x, int& y, int64_t& idx) {
+        x = xlo + (list[i] & 63);
+        y = ylo + (list[i] >> 6);
+        idx = int64_t(y) * g.w + x;
+    };
+    auto weight = [&](int x, int y) {
+        return float(axis_ifactor(x, nx, g.nodes_x, sh) * axis_ifactor(y, ny, g.nodes_y, sh)) * inv_wscale;
+    };
+    auto exact_bin = [&](int x, int y, int64_t k) {  // main.cpp:352-357
+        const float su = fclamps((float(x) + sample_pu(s, 0, k) - support_left) / support, 0.0f, 1.0f);
+        const float sv = fclamps((float(y) + sample_pu(s, 1, k) - support_top) / support, 0.0f, 1.0f);
+        return bin2d(su, sv);
+    };
+    auto nominal_bin = [&](int x, int y) {
+        return ((y - (ny - 1) * step) >> (sh - 1)) * 4 + ((x - (nx - 1) * step) >> (sh - 1));
+    };
+    auto is_deviant = [&](int64_t idx) { return ((__float_as_uint(gp.pat2[idx].y) >> 8) & kPixDeviant) != 0; };
+    auto pattern_of = [](uint32_t key) {
+        uint32_t p = 0u;
+#pragma unroll
+        for (int c = 0; c < kClasses; ++c)
+            if (!(key & key_absent_bit(c))) p |= class_bit(c);
+        return p;
+    };
+    // the patterns of the samples to move
+    PatternSet set;
+    for (int i = 0; i < nodd; ++i) {
+        int x, y;
+        int64_t idx;
+        pixel(i, x, y, idx);
+        if (is_deviant(idx)) continue;
+        const int b0 = nominal_bin(x, y);
+        const int64_t local = idx - gpar.first, kend = offsets[local + 1];
+        for (int64_t k = offsets[local] + lane; k < kend; k += 32) {
+            const uint32_t key = gp.key[k];
+            if (!(key & key_absent_bit(0)) && exact_bin(x, y, k) != b0) set.add(pattern_of(key));
+        }
+    }
+    set.unite_warp();
+    Totals unused;
+    for (uint32_t P = set.pop(); P != 0u; P = set.pop()) {
+        bins.clear();
+        __syncwarp();
+        for (int i = 0; i < nodd; ++i) {
+            int x, y;
+            int64_t idx;
+            pixel(i, x, y, idx);
+            if (is_deviant(idx)) continue;
+            const int b0 = nominal_bin(x, y);
+            const float w = weight(x, y);
+            const int64_t local = idx - gpar.first, kend = offsets[local + 1];
+            for (int64_t k = offsets[local] + lane; k < kend; k += 32) {
+                const uint32_t key = gp.key[k];
+                if ((key & key_absent_bit(0)) || pattern_of(key) != P) continue;
+                const int b = exact_bin(x, y, k);
+                if (b == b0) continue;
+                const float yv = gp.lum[k];
+                bins.add_weight(b, w, 1.0f);
+                bins.add_sum(b, w, yv, 0.0f);
+                bins.add_weight(b0, -w, 1.0f);
+                bins.add_sum(b0, -w, yv, 0.0f);
+            }
+        }
+        const float2 v = bins.reduce_value();
+        if (v.x == 0.0f && v.y == 0.0f) continue;
+#pragma unroll
+        for (int c = 0; c < kClasses; ++c)
+            if (P & class_bit(c)) df_accum(base + dep_screen(c) * kDepStride + lane, v.x, v.y);
+    }
+    __syncwarp();
+    if (!deviants) return;
+    for (int c = 0; c < kClasses; ++c) {
+        const uint32_t absent = key_absent_bit(c) | key_absent_bit(0);
+        Totals tx, ts;
+        bins.clear();
+        __syncwarp();
+        for (int i = 0; i < nodd; ++i) {
+            int x, y;
+            int64_t idx;
+            pixel(i, x, y, idx);
+            const PixPattern pp = load_pattern(gp, idx);
+            if (!(pp.pf & kPixDeviant)) continue;
+            float cs[5];
+            class_sums(gp, c, idx, pp, cs);
+            if (cs[0] == 0.0f) continue;
+            const float w = weight(x, y);
+            const bool mixed = c > 0 && (pp.pf & kPixMixed);
+            if (lane == 0) {
+                add_class(tx, w, cs[0], cs[1], cs[2], cs[3], cs[4]);
+                if (!mixed) add_class(ts, w, cs[0], cs[1], cs[2], cs[3], cs[4]);
+            }
+            const int64_t local = idx - gpar.first, kend = offsets[local + 1];
+            for (int64_t k = offsets[local] + lane; k < kend; k += 32) {
+                const uint32_t key = gp.key[k];
+                if (key & absent) continue;
+                const float yv = gp.lum[k];
+                const int b = exact_bin(x, y, k);
+                bins.add_weight(b, w, 1.0f);
+                bins.add_sum(b, w, yv, 0.0f);
+                if (mixed) add_sample(ts, w, yv);
+            }
+        }
+        const float2 v = bins.reduce_value();
+        if (v.x != 0.0f || v.y != 0.0f) df_accum(base + dep_screen(c) * kDepStride + lane, v.x, v.y);
+        reduce_totals_into(ts, base + dep_screen(c) * kDepStride);
+        if (c > 0) reduce_totals_into(tx, base + dep_random(c) * kDepStride);
+    }
+}
+
+__global__ void __launch_bounds__(32) k_grid_odd(GridParams gpar, float2* grid, DeviceSamples s, const int64_t* offsets,
+                                                 GridPrep gp, const unsigned* odd_count, const int32_t* odd_nodes) {
+    extern __shared__ float sm[];
+    const unsigned n = *odd_count;
+    for (unsigned k = blockIdx.x; k < n; k += gridDim.x) {
+        odd_node(gpar, grid, s, offsets, gp, odd_nodes[k], sm);
+        __syncwarp();
     }
 }
 
@@ -1548,7 +2039,6 @@ cudaError_t launch_strips_unit(Job& j, const StripParams& sp, unsigned blocks, f
 
 // Blocks of NC * 32 columns and `len` node rows (one more strip to walk than node rows), one block per
 // SM by shared memory: the len whose waves of blocks walk the fewest strips.
-constexpr int kStripSms = 152;
 template <int NC>
 int64_t strip_plan(StripParams& sp) {
     const int nb = NC * 32 / sp.g.step - 1;
@@ -1648,6 +2138,32 @@ cudaError_t launch_grid_fast(Job& j, const DeviceSamples& s, int64_t first, int6
     cudaError_t e;
     {
         KernelScope ks(j, RPD_KERNEL_GRID);
+        int sh = 0;
+        while ((1 << sh) < step) ++sh;
+        // (images of a few nodes fill the GPU with neither form, and the one launch of the pattern form
+        // is shorter than the two: 64x48, 63 nodes, 21 against 29 us; 256x256, 1089 nodes, 76 against 72)
+        if (gpar.uniform_ok && int_w && step >= 2 && step <= 16 && gpar.count_nodes > 512) {
+            const int ny0 = int(gpar.node0 / j.g.nodes_x), ny1 = ny0 + int(gpar.count_nodes / j.g.nodes_x);
+            // (scratch: a node plane that recompute_sensitivity writes before it reads)
+            unsigned* odd_count = reinterpret_cast<unsigned*>(j.p.counters + RPD_COUNTER_COUNT_);
+            int32_t* odd_nodes = reinterpret_cast<int32_t*>(j.n.prior[0]);
+            if ((e = cudaMemsetAsync(odd_count, 0, sizeof(unsigned), j.stream)) != cudaSuccess) return e;
+            TotalsParams tp{j.g, first, count, ny0, ny1, 1, 1, sh, fresh ? 1 : 0, odd_count, odd_nodes};
+            const int cells = 32 / step, image_cells = (j.g.w + step - 1) / step;
+            tp.col_warps = std::max(1, (image_cells - 1 + cells - 2) / (cells - 1));
+            // node rows per warp: one more strip than node rows is walked, so as many as leave
+            // 16 warps per SM
+            const int64_t warps16 = int64_t(kStripSms) * 16;
+            tp.len = int(std::min<int64_t>(16, std::max<int64_t>(1, int64_t(tp.col_warps) * (ny1 - ny0) / warps16)));
+            const int64_t warps = int64_t(tp.col_warps) * ((ny1 - ny0 + tp.len - 1) / tp.len);
+            k_grid_totals<<<unsigned((warps + 3) / 4), 128, 0, j.stream>>>(tp, target, gp);
+            if ((e = cudaGetLastError()) != cudaSuccess) return e;
+            const size_t smem = size_t(LaneBins<false>::kSlots) * 32 * sizeof(float) + size_t(4) * step * step * sizeof(uint16_t);
+            const unsigned odd_blocks = std::min<unsigned>(nblocks, unsigned(kStripSms) * 16);
+            k_grid_odd<<<odd_blocks, 32, smem, j.stream>>>(gpar, target, s, j.offsets, gp, odd_count, odd_nodes);
+            j.launches += 2;
+            if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        } else {
         const int side = 2 * step + 3;
         const size_t list_bytes = size_t(side) * size_t(side) * sizeof(int);
         if (list_bytes <= size_t(64) * 1024) {
@@ -1676,6 +2192,7 @@ cudaError_t launch_grid_fast(Job& j, const DeviceSamples& s, int64_t first, int6
         }
         j.launches += 1;
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        }
     }
     KernelScope ks(j, RPD_KERNEL_GRID_RANDOM);
     RandParams rp{gpar, 0u, -1, 2 * step + 3, nullptr, 0, 0, target};

@@ -156,9 +156,9 @@ struct Job {
     int64_t band_bytes = int64_t(768) << 20;  // target size of a band (RPD_TUNE_HOST_BAND_MB)
     float* lum = nullptr;        // per-sample luminance of the current push (fast grid pass)
     uint64_t lum_cap = 0;
-    float* cls[kClasses][5]{};   // per-pixel validity-class sums of deviant pixels (arena)
-    float4* pat4 = nullptr;      // per-pixel pattern sums (count, sum y hi, lo, sum y^2 hi) (arena)
-    float2* pat2 = nullptr;      // per-pixel (sum y^2 lo, pattern | flags << 8 as bits) (arena)
+    float* cls[kClasses][5]{};   // per-pixel sums of further patterns, or per class (GridPrep) (arena)
+    float4* pat4 = nullptr;      // per-pixel sums of the first pattern (count, sum y hi, lo, sum y^2 hi) (arena)
+    float2* pat2 = nullptr;      // per-pixel (sum y^2 lo, patterns and flags as bits) (arena)
     int64_t* offsets = nullptr;  // per-pixel sample offsets of the current push
     int64_t offsets_cap = 0;
     bool exact_grid = false;     // RPD_EXACT_GRID: double-precision grid in the reference's order
@@ -271,9 +271,9 @@ struct DeviceSamples {           // rpd_sample_soa with pointers in HBM
 // Class 0: pixel_valid samples; classes 1-6: samples with the brdf, lens, light_uv,
 // environment, light_select and rr dimension valid. Each class holds count, sum y
 // (hi, lo) and sum y^2 (hi, lo) over the pixel's finite samples.
-constexpr uint8_t kPixUniform = 0x1;  // every screen position lies inside its pixel
+constexpr uint8_t kPixUniform = 0x1;  // every sample lies in its pixel's screen bin, at every node
 constexpr uint8_t kPixMixed = 0x2;    // some sample has a random dimension but no screen position
-constexpr uint8_t kPixDeviant = 0x4;  // some sample's validity pattern differs from the pixel's pattern
+constexpr uint8_t kPixDeviant = 0x4;  // the pixel's samples have more than kPatterns validity patterns
 constexpr float kUniformMax = 1.0f - 1.0f / 4096.0f;  // largest in-pixel offset of a uniform pixel
 __host__ __device__ constexpr uint8_t class_bit(int c) {
     return c == 0 ? RPD_SAMPLE_PIXEL_VALID : c == 1 ? RPD_SAMPLE_BRDF_VALID : c == 2 ? RPD_SAMPLE_LENS_VALID
@@ -281,11 +281,13 @@ __host__ __device__ constexpr uint8_t class_bit(int c) {
          : RPD_SAMPLE_RR_VALID;
 }
 // Per-pixel inputs of the grid pass, written by the statistics pass for the pixels of a push.
-// A pixel's pattern is the validity-class bits (flags & 0xfe) of its first finite sample that
-// has any; pat4/pat2 hold the (count, sum y, sum y^2) double-float sums over its finite samples
-// with exactly that pattern, and the pattern and the pixel flags (kPix*) as the bits of
-// pat2.y: pattern | flags << 8. A pixel with other patterns too is deviant (kPixDeviant) and
-// then also has full per-class sums in cls[0..6].
+// A pixel's patterns are the validity-class bits (flags & 0xfe) of its finite samples that have any, in
+// the order they first appear; pat4/pat2 hold the (count, sum y, sum y^2) double-float sums over its
+// samples with exactly the first pattern, and the patterns and the pixel flags (kPix*) as the bits
+// of pat2.y: pattern 0 | flags << 8 | pattern 1 << 16 | pattern 2 << 24 (0: none). The sums of
+// patterns 1 and 2 are in cls[0] and cls[1]. A pixel with more patterns is deviant (kPixDeviant): no
+// pattern 1 and 2, and full per-class sums in cls[0..6].
+constexpr int kPatterns = 3;
 struct GridPrep {
     float* cls[kClasses][5];  // W*H planes
     float4* pat4;             // W*H
@@ -295,6 +297,7 @@ struct GridPrep {
     uint16_t* col;            // per sample of a push with per-pixel counts: the pixel's column
                               // (null for uniform pushes, where the column follows from the index)
     int width;
+    int bin_pixels;           // pixels per screen bin in x and y (a quarter of a power-of-two support of at least 4), else 1
 };
 // Sample key: one 5-bit field per random dimension in the order of the classes (brdf, lens, light_uv,
 // environment, light_select at bits 0, 5, 10, 15, 20): the bin 0-15, or 16 when the sample does not
