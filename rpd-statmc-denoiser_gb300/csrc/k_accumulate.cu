@@ -16,6 +16,7 @@
 
 #include "rpd_internal.h"
 #include "device_math.cuh"
+#include "tma.cuh"
 
 namespace rpd {
 
@@ -748,6 +749,355 @@ __global__ void __launch_bounds__(128, MINB) k_accumulate_pixels(PixelPlanes p, 
     acc_store(a, p, gp, idx, prep);
 }
 
+// ---- the statistics pass on staged rows ------------------------------------------------------------
+//
+// For uniform pushes of many samples per pixel: a plane is a matrix of one row of spp samples per pixel.
+// A block owns 32 pixels and fetches, into one of two buffers in turn, 32 bytes of their rows of
+// every plane into shared memory, one tensor copy per plane (cp.async.bulk.tensor, completion on an mbarrier).
+// Its five warps split a pixel's quantities, which are independent chains over its samples: one
+// warp per colour channel (colour and square-root mean and variance, radiance, normal and albedo
+// sums), one for the luminance statistics and the grid pass's class sums, one for the sample keys;
+// lane i of each is pixel i, walking the samples in order with the operations of
+// k_accumulate_pixels, so the results are the same bits. A thread that walks all of a pixel's planes
+// has a line of each plane in flight per pixel, 61 KB a warp from 64 compact samples on: the lines
+// of 12 warps on each SM do not survive in L2 until their next sectors are read (DRAM read 3.5 times the planes); with
+// a pixel's work on five warps a quarter of the pixels keeps an SM busy. 2048x1152x64: 4.22 -> 2.7 ms
+// compact; 1920x1080x64: 7.1 -> 2.25 ms FP32 (3.6 TB/s).
+struct RowsArgs {
+    CUtensorMap map[20];
+    int planes;                      // present planes, in the order of the offsets below
+    int albedo, pu, lu, bu, li, eu;  // a plane group's byte offset in a buffer, or -1
+};
+constexpr int kRowRoles = 5;
+constexpr int kRowPixels = 32;
+constexpr int kRowBytes = 32;  // of a pixel's row per step
+
+// The luminance warp's state (class_add's fields).
+struct LumAcc {
+    float mean, m2, dep;
+    int n, hits, nsamples;
+    PatternSums pt[kPatterns];
+    bool dev;
+    float* cs;
+};
+
+// x / n and y / n, IEEE quotients (the compact pass's by one reciprocal where that is exact)
+template <bool COMPACT>
+__device__ __forceinline__ void quotients(float x, float y, int n, float& qx, float& qy) {
+    const float fn = float(n);
+    if (COMPACT && n < (1 << 23) && markstein_ok(x) && markstein_ok(y)) {
+        const float rn = 1.0f / fn;
+        qx = div_markstein(x, fn, rn);
+        qy = div_markstein(y, fn, rn);
+    } else {
+        qx = x / fn;
+        qy = y / fn;
+    }
+}
+
+// w[i] of a small register array by selects (i is a loop counter the compiler does not unroll)
+template <int N>
+__device__ __forceinline__ uint32_t pick(const uint32_t (&w)[N], int i) {
+    uint32_t r = w[0];
+#pragma unroll
+    for (int k = 1; k < N; ++k) r = i == k ? w[k] : r;
+    return r;
+}
+
+template <bool COMPACT>
+__global__ void __launch_bounds__(kRowRoles * 32, 4)
+    k_accumulate_rows(PixelPlanes p, DeviceSamples s, int32_t spp, int64_t first, int64_t count, GridPrep gp, int fresh,
+                      const __grid_constant__ RowsArgs ra) {
+    constexpr int ES = COMPACT ? 2 : 4;
+    constexpr int RB = kRowBytes;
+    constexpr int CH = RB / ES;        // samples per step
+    constexpr int V = 4;               // samples per group
+    constexpr int PLANE = kRowPixels * RB;
+    extern __shared__ unsigned char smem_raw[];
+    __shared__ __align__(8) unsigned long long bars[2];
+    __shared__ uint8_t s_pflags[kRowPixels];
+    __shared__ int s_fail;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // (a block's warps go to the SM's schedulers by index: the roles rotate over the blocks)
+    const int role = (warp + int(blockIdx.x)) % kRowRoles;
+    const int64_t row0 = int64_t(blockIdx.x) * kRowPixels;
+    const uint32_t pad = (1024u - (smem_addr(smem_raw) & 1023u)) & 1023u;
+    const int stage = (ra.planes * PLANE + 1023) & ~1023;
+    unsigned char* buf = smem_raw + pad;
+    const int steps = spp / CH;
+    auto issue = [&](int c) {  // warp 0: lane 0 arms the barrier, lanes 0 .. planes-1 issue one plane's copy each
+        const uint32_t bar = smem_addr(&bars[c & 1]);
+        if (lane == 0) mbar_expect_tx(bar, uint32_t(ra.planes) * PLANE);
+        __syncwarp();
+        if (lane < ra.planes)
+            tma_load_2d(smem_addr(buf + (c & 1) * stage + lane * PLANE), &ra.map[lane], c * CH, int(row0), bar);
+    };
+    if (threadIdx.x == 0) {
+        mbar_init(smem_addr(&bars[0]), 1);
+        mbar_init(smem_addr(&bars[1]), 1);
+        s_fail = 0;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        issue(0);
+        if (steps > 1) issue(1);
+    }
+    const int64_t local = row0 + lane;
+    const bool mine = local < count;
+    const int64_t idx = first + local;
+    const int64_t k0 = local * spp;
+    const bool prep = gp.lum != nullptr;
+    // step c's samples are in place; false: they did not arrive in time, the block gives up
+    auto arrived = [&](int c) { return mbar_wait_bounded(smem_addr(&bars[c & 1]), (c >> 1) & 1); };
+    auto done = [&](int c, bool ok) -> bool {  // step c is read: its buffer takes step c + 2
+        if (!ok) s_fail = 1;
+        __syncthreads();
+        if (s_fail) {
+            if (threadIdx.x == 0) atomicAdd(p.counters + RPD_COUNTER_DEVICE_WAIT_TIMEOUTS, 1ull);
+            arrived(c);  // let the copies land (bounded) before the shared memory is released
+            if (c + 1 < steps) arrived(c + 1);
+            return false;
+        }
+        if (warp == 0 && c + 2 < steps) issue(c + 2);
+        return true;
+    };
+    auto flag_words = [&](const uint8_t* plane, int c, uint32_t* w) {
+#pragma unroll
+        for (int i = 0; i < CH / 4; ++i) w[i] = mine && plane ? *reinterpret_cast<const uint32_t*>(plane + k0 + c * CH + 4 * i) : 0u;
+    };
+    // group q of the pixel's row in the plane at byte offset off of step c
+    auto chunk = [&](int c, int off, int q) -> uint4 {
+        const unsigned char* at = buf + (c & 1) * stage + off + lane * RB;
+        if constexpr (COMPACT) {
+            const uint2 v = *reinterpret_cast<const uint2*>(at + 16 * swizzled_chunk<RB>(q >> 1, lane) + 8 * (q & 1));
+            return make_uint4(v.x, v.y, 0u, 0u);
+        } else {
+            return *reinterpret_cast<const uint4*>(at + 16 * swizzled_chunk<RB>(q, lane));
+        }
+    };
+    // sample i of a chunk: its float (FP32 planes), or its 16 bits
+    auto f32 = [](const uint4& v, int i) { return __uint_as_float(i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w); };
+    auto u16 = [](const uint4& v, int i) {
+        const uint32_t w = (i >> 1) == 0 ? v.x : (i >> 1) == 1 ? v.y : (i >> 1) == 2 ? v.z : v.w;
+        return uint16_t(w >> (16 * (i & 1)));
+    };
+    auto finite = [&](const uint4* L, int i) {
+        if constexpr (COMPACT) {
+            bool ok = true;
+            for (int d = 0; d < 3; ++d) ok = ok && (u16(L[d], i) & 0x7c00u) != 0x7c00u;
+            return ok;
+        } else {
+            return finite3(f32(L[0], i), f32(L[1], i), f32(L[2], i));
+        }
+    };
+
+    if (role < 3) {  // colour channel `role`
+        float cm = 0.0f, sm = 0.0f, sq_ = 0.0f, rad = 0.0f, nor = 0.0f, alb = 0.0f, palb = 0.0f;
+        int n = 0;
+        const bool per_sample = !COMPACT && ra.albedo >= 0;
+        if (mine) {
+            if (!fresh) {
+                n = p.n[idx];
+                cm = p.color_mean[role][idx];
+                sm = p.sqrt_mean[role][idx];
+                sq_ = p.sqrt_sq[role][idx];
+                rad = p.radiance[role][idx];
+                nor = p.normal[role][idx];
+                alb = p.albedo[role][idx];
+            }
+            if (COMPACT) {
+                if (s.c16.pixel_albedo[0]) palb = h2f(s.c16.pixel_albedo[role][local]);
+            } else if (!per_sample && s.pixel_albedo[0]) {
+                palb = s.pixel_albedo[role][local];
+            }
+        }
+        for (int c = 0; c < steps; ++c) {
+            uint32_t F[CH / 4];
+            flag_words(s.flags, c, F);
+            const bool ok = arrived(c);
+            if (ok && mine) {
+#pragma unroll 1
+                for (int q = 0; q < CH / V; ++q) {
+                    uint4 L[3];
+                    for (int d = 0; d < 3; ++d) L[d] = chunk(c, d * PLANE, q);
+                    const uint4 N = chunk(c, (3 + role) * PLANE, q);
+                    uint4 A = make_uint4(0u, 0u, 0u, 0u);
+                    if (per_sample) A = chunk(c, ra.albedo + role * PLANE, q);
+                    uint32_t f4[V / 4];
+                    for (int i = 0; i < V / 4; ++i) f4[i] = pick(F, q * (V / 4) + i);
+                    const uint4 mineL = role == 0 ? L[0] : role == 1 ? L[1] : L[2];
+#pragma unroll
+                    for (int i = 0; i < V; ++i) {
+                        const uint32_t f = f4[i >> 2] >> (8 * (i & 3));
+                        if (f & RPD_SAMPLE_HIT) {  // main.cpp:572-576
+                            nor += COMPACT ? snorm16(int16_t(u16(N, i))) : f32(N, i);
+                            alb += per_sample ? f32(A, i) : palb;
+                        }
+                        if (!finite(L, i)) continue;  // main.cpp:707
+                        float v, root;
+                        if constexpr (COMPACT) {
+                            root = fabsf(h2f(u16(mineL, i)));
+                            v = sq(root);
+                        } else {
+                            v = f32(mineL, i);
+                            root = sqrtf(fmaxs(0.0f, v));
+                        }
+                        // accumulate_sample (core/stats.h:25-41), this channel
+                        ++n;
+                        const float cd = v - cm, sd = root - sm;
+                        float qc, qs;
+                        quotients<COMPACT>(cd, sd, n, qc, qs);
+                        cm += qc;
+                        sm += qs;
+                        sq_ += sd * (root - sm);
+                        rad += v;
+                    }
+                }
+            }
+            if (!done(c, ok)) return;
+        }
+        if (mine) {
+            p.color_mean[role][idx] = cm;
+            p.sqrt_mean[role][idx] = sm;
+            p.sqrt_sq[role][idx] = sq_;
+            p.radiance[role][idx] = rad;
+            p.normal[role][idx] = nor;
+            p.albedo[role][idx] = alb;
+        }
+        __syncthreads();
+    } else if (role == 3) {  // luminance, depth, counts, class sums
+        const uint8_t mask = plane_mask_of(ra.pu >= 0, ra.lu >= 0, ra.bu >= 0, ra.li >= 0, ra.eu >= 0);
+        LumAcc a{};
+        float cls_local[kClasses * 5];
+        a.cs = cls_local + (uint32_t(gp.width) >> 31);  // in local memory (k_accumulate_pixels)
+        if (mine && !fresh) {
+            a.mean = p.mean[idx];
+            a.m2 = p.square_diff[idx];
+            a.n = p.n[idx];
+            a.dep = p.depth[idx];
+            a.hits = p.hit_count[idx];
+            a.nsamples = p.sample_count[idx];
+        }
+        for (int c = 0; c < steps; ++c) {
+            uint32_t F[CH / 4];
+            flag_words(s.flags, c, F);
+            const bool ok = arrived(c);
+            if (ok && mine) {
+#pragma unroll 1
+                for (int q = 0; q < CH / V; ++q) {
+                    uint4 L[3];
+                    for (int d = 0; d < 3; ++d) L[d] = chunk(c, d * PLANE, q);
+                    const uint4 D = chunk(c, 6 * PLANE, q);
+                    uint32_t f4[V / 4];
+                    for (int i = 0; i < V / 4; ++i) f4[i] = pick(F, q * (V / 4) + i);
+                    float lum_out[V];
+#pragma unroll
+                    for (int i = 0; i < V; ++i) {
+                        const uint32_t f = f4[i >> 2] >> (8 * (i & 3));
+                        if (f & RPD_SAMPLE_HIT) {
+                            ++a.hits;
+                            a.dep += COMPACT ? h2f(u16(D, i)) * s.c16.depth_scale : f32(D, i);
+                        }
+                        lum_out[i] = __int_as_float(0x7fc00000);  // NaN: dropped by the grid pass
+                        if (!finite(L, i)) continue;
+                        float v[3];
+                        for (int d = 0; d < 3; ++d) v[d] = COMPACT ? sq(fabsf(h2f(u16(L[d], i)))) : f32(L[d], i);
+                        const float lum = luminance(v[0], v[1], v[2]);
+                        const float delta = lum - a.mean;
+                        ++a.n;
+                        float qd, unused;
+                        quotients<COMPACT>(delta, delta, a.n, qd, unused);
+                        a.mean += qd;
+                        a.m2 += delta * (lum - a.mean);
+                        ++a.nsamples;
+                        lum_out[i] = lum;
+                        if (prep) class_add(a, uint8_t(f) & mask, lum);
+                    }
+                    if (prep) {
+#pragma unroll
+                        for (int i = 0; i < V; i += 4)
+                            *reinterpret_cast<float4*>(gp.lum + k0 + c * CH + q * V + i) =
+                                make_float4(lum_out[i], lum_out[i + 1], lum_out[i + 2], lum_out[i + 3]);
+                    }
+                }
+            }
+            if (!done(c, ok)) return;
+        }
+        if (mine) {
+            p.mean[idx] = a.mean;
+            p.square_diff[idx] = a.m2;
+            p.n[idx] = a.n;
+            p.depth[idx] = a.dep;
+            p.hit_count[idx] = a.hits;
+            p.sample_count[idx] = a.nsamples;
+        }
+        __syncthreads();  // the key warp's pixel flags
+        if (mine && prep) store_classes(a, gp, idx, s_pflags[lane]);
+    } else {  // keys and pixel flags
+        const uint8_t mask = plane_mask_of(ra.pu >= 0, ra.lu >= 0, ra.bu >= 0, ra.li >= 0, ra.eu >= 0);
+        uint8_t pflags = kPixUniform;
+        const float fx = float(idx % gp.width), fy = float(idx / gp.width);
+        for (int c = 0; c < steps; ++c) {
+            uint32_t F[CH / 4], C[CH / 4];
+            flag_words(s.flags, c, F);
+            flag_words(s.category, c, C);
+            const bool ok = arrived(c);
+            if (ok && mine && prep) {
+#pragma unroll 1
+                for (int q = 0; q < CH / V; ++q) {
+                    uint4 L[3], U[5][2];
+                    const int offs[5] = {ra.pu, ra.bu, ra.lu, ra.li, ra.eu};
+                    for (int d = 0; d < 3; ++d) L[d] = chunk(c, d * PLANE, q);
+#pragma unroll
+                    for (int g = 0; g < 5; ++g)
+                        for (int d = 0; d < 2; ++d)
+                            U[g][d] = offs[g] >= 0 ? chunk(c, offs[g] + d * PLANE, q) : make_uint4(0u, 0u, 0u, 0u);
+                    uint32_t f4[V / 4], c4[V / 4];
+                    for (int i = 0; i < V / 4; ++i) {
+                        f4[i] = pick(F, q * (V / 4) + i);
+                        c4[i] = pick(C, q * (V / 4) + i);
+                    }
+                    uint32_t key[V];
+#pragma unroll
+                    for (int i = 0; i < V; ++i) {
+                        const uint8_t fm = uint8_t(f4[i >> 2] >> (8 * (i & 3))) & mask;
+                        key[i] = kKeyNone;
+                        if (!finite(L, i)) continue;
+                        SampleIn in;
+                        in.cat = uint8_t(c4[i >> 2] >> (8 * (i & 3)));
+                        for (int d = 0; d < 2; ++d) {
+                            if constexpr (COMPACT) {
+                                in.pu[d] = unorm16(u16(U[0][d], i));
+                            } else {
+                                in.pu[d] = f32(U[0][d], i);
+                                in.bu[d] = f32(U[1][d], i);
+                                in.lu[d] = f32(U[2][d], i);
+                                in.liu[d] = f32(U[3][d], i);
+                                in.eu[d] = f32(U[4][d], i);
+                            }
+                        }
+                        if constexpr (COMPACT) {
+                            in.bins = 0u;
+#pragma unroll
+                            for (int g = 0; g < 4; ++g)
+                                in.bins |= bin2d_q(u16(U[g + 1][0], i), u16(U[g + 1][1], i)) << (5 * g);
+                        }
+                        key[i] = sample_key<COMPACT>(in, fm);
+                        screen_flags(in, fm, fx, fy, gp.bin_pixels, pflags);
+                    }
+#pragma unroll
+                    for (int i = 0; i < V; i += 4)
+                        *reinterpret_cast<uint4*>(gp.key + k0 + c * CH + q * V + i) =
+                            make_uint4(key[i], key[i + 1], key[i + 2], key[i + 3]);
+                }
+            }
+            if (!done(c, ok)) return;
+        }
+        s_pflags[lane] = pflags;
+        __syncthreads();
+    }
+}
+
 // Valid-flag bit each dependency needs, and whether it bins the screen position.
 __device__ __forceinline__ uint8_t dep_flag(int d) {
     switch (d) {
@@ -1056,6 +1406,88 @@ cudaError_t run_accumulate(Job& j, unsigned blocks, const DeviceSamples& s, int6
     return cudaSuccess;
 }
 
+// The staged form of the statistics pass, if the push allows it: uniform samples per pixel, 16-byte
+// aligned planes, a pixel's row of each plane a multiple of 32 bytes. *taken: it ran. From 32 samples
+// per pixel: up to 16 the general form reads each line in few enough steps and executes a third
+// fewer instructions (1920x1080, general / staged: FP32 8 spp 0.33 / 0.45 ms, 16 spp 0.64 / 0.90, 32
+// spp 3.03 / 1.43, 64 spp 7.1 / 2.25; compact 16 spp 0.43 / 0.78, 32 spp 1.40 / 1.30, 64 spp 3.75 /
+// 2.26). Below a million samples its tensor maps' encoding on the host would show.
+constexpr int kRowMinSpp = 32;
+template <bool COMPACT>
+cudaError_t run_rows(Job& j, const DeviceSamples& s, int64_t first, int64_t count, const GridPrep& gp, int32_t spp,
+                     int fresh, const void* const* planes, RowsArgs& ra) {
+    constexpr int ES = COMPACT ? 2 : 4, RB = kRowBytes;
+    for (int i = 0; i < ra.planes; ++i) {
+        const cudaError_t e = encode_rows_map(&ra.map[i], planes[i], ES, spp, count, RB / ES, kRowPixels);
+        if (e != cudaSuccess) return e;
+    }
+    for (int* off : {&ra.albedo, &ra.pu, &ra.lu, &ra.bu, &ra.li, &ra.eu})
+        if (*off >= 0) *off *= kRowPixels * RB;
+    const int smem = 1024 + 2 * ((ra.planes * kRowPixels * RB + 1023) & ~1023);
+    const cudaError_t e =
+        cudaFuncSetAttribute(k_accumulate_rows<COMPACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    k_accumulate_rows<COMPACT><<<grid_for(count, kRowPixels), kRowRoles * 32, smem, j.stream>>>(j.p, s, spp, first, count, gp, fresh, ra);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_accumulate_rows(Job& j, const DeviceSamples& s, int64_t first, int64_t count, const GridPrep& gp,
+                                   int32_t spp, int fresh, bool* taken) {
+    *taken = false;
+    const int es = s.compact ? 2 : 4;
+    if (spp < kRowMinSpp || (int64_t(spp) * es) % kRowBytes || count * int64_t(spp) < (int64_t(1) << 20) ||
+        count > INT32_MAX)
+        return cudaSuccess;
+    const void* planes[20];
+    RowsArgs ra{};
+    ra.albedo = ra.pu = ra.lu = ra.bu = ra.li = ra.eu = -1;
+    bool ok = (reinterpret_cast<uintptr_t>(s.flags) & 15u) == 0 && (reinterpret_cast<uintptr_t>(s.category) & 15u) == 0 &&
+              (!gp.lum || ((reinterpret_cast<uintptr_t>(gp.lum) | reinterpret_cast<uintptr_t>(gp.key)) & 15u) == 0);
+    auto add = [&](const void* ptr) {
+        ok = ok && ptr && (reinterpret_cast<uintptr_t>(ptr) & 15u) == 0;
+        planes[ra.planes++] = ptr;
+    };
+    auto group = [&](const void* a, const void* b, int* off) {
+        if (!a || !gp.lum) return;
+        *off = ra.planes;
+        add(a);
+        add(b);
+    };
+    if (s.compact) {
+        const DeviceSamples16& h = s.c16;
+        for (int c = 0; c < 3; ++c) add(h.sqrt_radiance[c]);
+        for (int c = 0; c < 3; ++c) add(h.normal[c]);
+        add(h.depth);
+        group(h.pixel_u[0], h.pixel_u[1], &ra.pu);
+        group(h.lens_u[0], h.lens_u[1], &ra.lu);
+        group(h.brdf_u[0], h.brdf_u[1], &ra.bu);
+        group(h.light_u[0], h.light_u[1], &ra.li);
+        group(h.env_u[0], h.env_u[1], &ra.eu);
+    } else {
+        for (int c = 0; c < 3; ++c) add(s.radiance[c]);
+        for (int c = 0; c < 3; ++c) add(s.normal[c]);
+        add(s.depth);
+        if (s.albedo[0]) {
+            ra.albedo = ra.planes;
+            for (int c = 0; c < 3; ++c) add(s.albedo[c]);
+        }
+        group(s.pixel_u[0], s.pixel_u[1], &ra.pu);
+        group(s.lens_u[0], s.lens_u[1], &ra.lu);
+        group(s.brdf_u[0], s.brdf_u[1], &ra.bu);
+        group(s.light_u[0], s.light_u[1], &ra.li);
+        group(s.env_u[0], s.env_u[1], &ra.eu);
+    }
+    if (!ok) return cudaSuccess;
+    cudaError_t e = s.compact ? run_rows<true>(j, s, first, count, gp, spp, fresh, planes, ra)
+                              : run_rows<false>(j, s, first, count, gp, spp, fresh, planes, ra);
+    if (e == cudaErrorNotSupported || e == cudaErrorInvalidValue) {  // no tensor-map encoder: the general form runs
+        cudaGetLastError();
+        return cudaSuccess;
+    }
+    *taken = e == cudaSuccess;
+    return e;
+}
+
 cudaError_t launch_accumulate_pixels(Job& j, const DeviceSamples& s, int64_t first, int64_t count,
                                      const GridPrep& gp, int32_t spp) {
     KernelScope ks(j, RPD_KERNEL_ACCUMULATE_PIXELS);
@@ -1063,6 +1495,13 @@ cudaError_t launch_accumulate_pixels(Job& j, const DeviceSamples& s, int64_t fir
     // instead of reading them
     const int fresh = (j.acc_zero && first == 0 && count == j.g.np) ? 1 : 0;
     j.acc_zero = false;
+    bool taken = false;
+    if (const cudaError_t er = launch_accumulate_rows(j, s, first, count, gp, spp, fresh, &taken); er != cudaSuccess)
+        return er;
+    if (taken) {
+        j.launches += 1;
+        return cudaSuccess;
+    }
     auto aligned = [](const void* ptr, uintptr_t a) { return (reinterpret_cast<uintptr_t>(ptr) & (a - 1)) == 0; };
     bool vec4 = spp > 0 && spp % 4 == 0 && aligned(s.flags, 16) && (!s.category || aligned(s.category, 16));
     if (s.compact) {

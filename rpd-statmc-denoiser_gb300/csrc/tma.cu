@@ -56,4 +56,25 @@ cudaError_t encode_plane_map(CUtensorMap* map, const float* base, int w, int h, 
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
+cudaError_t encode_rows_map(CUtensorMap* map, const void* base, int elem, int64_t cols, int64_t rows, int box_cols,
+                            int box_rows) {
+    const int row_bytes = box_cols * elem;
+    if ((elem != 2 && elem != 4) || cols < box_cols || rows < 1 || (cols * elem) % 16 || box_rows < 1 || box_rows > 256 ||
+        (row_bytes != 16 && row_bytes != 32 && row_bytes != 64) || rows > (int64_t(1) << 31) || cols > (int64_t(1) << 31))
+        return cudaErrorInvalidValue;
+    const EncodeTiled fn = encoder();
+    if (!fn) return cudaErrorNotSupported;
+    const cuuint64_t dims[2] = {cuuint64_t(cols), cuuint64_t(rows)};
+    const cuuint64_t strides[1] = {cuuint64_t(cols) * elem};
+    const cuuint32_t box[2] = {cuuint32_t(box_cols), cuuint32_t(box_rows)};
+    const cuuint32_t estride[2] = {1, 1};
+    const CUtensorMapSwizzle sw = row_bytes == 64   ? CU_TENSOR_MAP_SWIZZLE_64B
+                                  : row_bytes == 32 ? CU_TENSOR_MAP_SWIZZLE_32B
+                                                    : CU_TENSOR_MAP_SWIZZLE_NONE;
+    const CUresult r = fn(map, elem == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_UINT16, 2,
+                          const_cast<void*>(base), dims, strides, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
+                          CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
 }  // namespace rpd

@@ -87,5 +87,16 @@ cudaError_t encode_record_map(CUtensorMap* map, const void* base, int w, int h, 
 // of 4, so rows start 16 bytes apart), for boxes of bw x bh floats (bw a multiple of 4, <= 256).
 // Columns from w to the pitch lie outside the tensor: a box reading them gets zeros.
 cudaError_t encode_plane_map(CUtensorMap* map, const float* base, int w, int h, int pitch, int bw, int bh);
+// Host: the tensor map of a plane of `rows` rows of `cols` elements of 2 or 4 bytes (a row a multiple
+// of 16 bytes), for boxes of box_rows rows of 16, 32 or 64 bytes. 32- and 64-byte rows land swizzled
+// in shared memory, so that lanes reading the same 16-byte chunk of consecutive rows hit different
+// banks (swizzled_chunk).
+cudaError_t encode_rows_map(CUtensorMap* map, const void* base, int elem, int64_t cols, int64_t rows, int box_cols,
+                            int box_rows);
+// Where 16-byte chunk c of row r of such a box lies in its row.
+template <int ROW_BYTES>
+__device__ __forceinline__ int swizzled_chunk(int c, int r) {
+    return ROW_BYTES == 64 ? c ^ ((r >> 1) & 3) : ROW_BYTES == 32 ? c ^ ((r >> 2) & 1) : c;
+}
 
 }  // namespace rpd
