@@ -1567,11 +1567,9 @@ int rpd_atrous_wavelet(rpd_ctx* ctx, const float* raw, const float* normal, cons
     RPD_CUDA(cudaSetDevice(c->device));
     cudaStream_t st = c->util_stream;
     const uint64_t bytes = uint64_t(w) * h * 12;
-    float *d_raw = nullptr, *d_n = nullptr, *d_a = nullptr, *b0 = nullptr, *b1 = nullptr;
-    float4* records = nullptr;
-    RPD_CUDA(cudaMallocAsync(&b0, bytes, st));
-    RPD_CUDA(cudaMallocAsync(&b1, bytes, st));
-    RPD_CUDA(cudaMallocAsync(&records, uint64_t(w) * h * 2 * sizeof(float4), st));
+    float *d_raw = nullptr, *d_n = nullptr, *d_a = nullptr;
+    void* scratch = nullptr;
+    RPD_CUDA(cudaMallocAsync(&scratch, atrous_scratch_bytes(w, h), st));
     if (where == RPD_MEM_HOST) {
         RPD_CUDA(cudaMallocAsync(&d_raw, bytes, st));
         RPD_CUDA(cudaMallocAsync(&d_n, bytes, st));
@@ -1583,14 +1581,12 @@ int rpd_atrous_wavelet(rpd_ctx* ctx, const float* raw, const float* normal, cons
     const float* r_in = where == RPD_MEM_HOST ? d_raw : raw;
     const float* n_in = where == RPD_MEM_HOST ? d_n : normal;
     const float* a_in = where == RPD_MEM_HOST ? d_a : albedo;
-    float* result = nullptr;
+    // a host call's result goes over its copy of the raw image
+    float* d_out = where == RPD_MEM_HOST ? d_raw : out;
     uint64_t launches = 0;
-    RPD_CUDA(launch_atrous(r_in, n_in, a_in, w, h, sigma_c, sigma_n, sigma_a, iterations, b0, b1, records, &result, st,
-                           &launches));
-    RPD_CUDA(cudaMemcpyAsync(out, result, bytes, where == RPD_MEM_HOST ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice, st));
-    RPD_CUDA(cudaFreeAsync(b0, st));
-    RPD_CUDA(cudaFreeAsync(b1, st));
-    RPD_CUDA(cudaFreeAsync(records, st));
+    RPD_CUDA(launch_atrous(r_in, n_in, a_in, w, h, sigma_c, sigma_n, sigma_a, iterations, scratch, d_out, st, &launches));
+    if (where == RPD_MEM_HOST) RPD_CUDA(cudaMemcpyAsync(out, d_out, bytes, cudaMemcpyDeviceToHost, st));
+    RPD_CUDA(cudaFreeAsync(scratch, st));
     if (d_raw) RPD_CUDA(cudaFreeAsync(d_raw, st));
     if (d_n) RPD_CUDA(cudaFreeAsync(d_n, st));
     if (d_a) RPD_CUDA(cudaFreeAsync(d_a, st));

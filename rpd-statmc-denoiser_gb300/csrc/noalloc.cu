@@ -76,10 +76,9 @@ extern "C" int rpd_atrous_wavelet_noalloc(const float* raw, const float* normal,
     float* first = (iterations & 1) ? out : scratch;
     float* second = (iterations & 1) ? scratch : out;
     float* result = nullptr;
-    uint64_t launches = 0;
     // no records scratch: the passes renormalise each tap's normal from the caller's buffer
-    RPD_CUDA(rpd::launch_atrous(raw, normal, albedo, width, height, sigma_c, sigma_n, sigma_a, iterations, first,
-                                second, nullptr, &result, s, &launches));
+    RPD_CUDA(rpd::launch_atrous_plain(raw, normal, albedo, width, height, sigma_c, sigma_n, sigma_a, iterations, first,
+                                      second, &result, s));
     if (result != out) return fail(RPD_ERR_STATE, "a-trous passes did not end in the output buffer");
     return RPD_OK;
 }

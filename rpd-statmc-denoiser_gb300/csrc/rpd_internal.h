@@ -352,12 +352,17 @@ cudaError_t allocator_stats(Job& j, int32_t* out);
 int allocator_timeline(Job& j, uint64_t* ns, int32_t max, int32_t* n);
 cudaError_t launch_finalize(Job& j);
 cudaError_t launch_expand(Job& j, const float* node_field, float* out);
-// `iterations` a-trous passes ping-ponging between buf_a and buf_b (interleaved RGB); *result
-// gets the buffer holding the last pass (raw for 0 passes). records: scratch for 2 * w * h float4
-// normal and albedo records, or nullptr to renormalise the normals at every tap instead.
-cudaError_t launch_atrous(const float* raw, const float* normal, const float* albedo, int w, int h,
-                          float sigma_c, float sigma_n, float sigma_a, int iterations, float* buf_a,
-                          float* buf_b, float4* records, float** result, cudaStream_t stream, uint64_t* launches);
+// `iterations` a-trous passes over records in `scratch` (atrous_scratch_bytes), the last one writing
+// the interleaved RGB `out`, which may be one of the inputs.
+uint64_t atrous_scratch_bytes(int w, int h);
+cudaError_t launch_atrous(const float* raw, const float* normal, const float* albedo, int w, int h, float sigma_c,
+                          float sigma_n, float sigma_a, int iterations, void* scratch, float* out, cudaStream_t stream,
+                          uint64_t* launches);
+// The same without records, ping-ponging between buf_a and buf_b (interleaved RGB); *result gets the
+// buffer holding the last pass (raw for 0 passes).
+cudaError_t launch_atrous_plain(const float* raw, const float* normal, const float* albedo, int w, int h, float sigma_c,
+                                float sigma_n, float sigma_a, int iterations, float* buf_a, float* buf_b, float** result,
+                                cudaStream_t stream);
 // The joint bilateral filter's scratch (its records and a copy-timeout flag), and the filter.
 // The flag (an unsigned after the records) is non-zero when a tile copy's bounded wait gave up.
 uint64_t joint_bilateral_scratch_bytes(int w, int h);
