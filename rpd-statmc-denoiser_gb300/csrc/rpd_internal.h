@@ -125,6 +125,7 @@ struct Ctx {
     std::atomic<uint64_t> in_use{0};
     std::mutex mu;
     cudaStream_t util_stream = nullptr;
+    cudaMemPool_t pool = nullptr;  // scratch of the post-filters and metrics, see kPoolKeep
     std::unordered_map<void*, uint64_t> user_allocs;  // rpd_device_alloc bookkeeping
 };
 
