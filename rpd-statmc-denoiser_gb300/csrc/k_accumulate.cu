@@ -211,8 +211,8 @@ __device__ __forceinline__ uint32_t sample_key(const SampleIn& in, uint8_t fm) {
 // A finite sample's luminance into its pixel's pattern sums. A tracer's pixels hold a few patterns (all
 // dimensions, paths that ended before Russian roulette, paths that ended at the first hit): with
 // one pattern in registers and the rest added class by class in local memory, a 1920x1080x16
-// frame of such samples took 1.71 ms in this pass, with three patterns in registers 0.99 ms (0.64
-// ms for a frame of a single pattern).
+// frame of such samples took 1.71 ms in this pass, with three patterns in registers 0.99 ms (0.76
+// with one reciprocal per sample; 0.64 ms for a frame of a single pattern).
 template <typename Acc>
 __device__ __forceinline__ void class_add(Acc& a, uint8_t fm, float lum) {
     const uint32_t bits = fm & 0xfeu;
@@ -294,68 +294,80 @@ __device__ __forceinline__ void screen_flags(const SampleIn& in, uint8_t fm, flo
     }
 }
 
+// What a thread of the statistics pass keeps of its pixel: everything, or one of two parts that share
+// nothing but the radiance they read (kColour: the channels' statistics, normal and albedo sums;
+// kLuminance: the luminance statistics, depth, counts, sample keys and the grid pass's sums).
+enum Part { kWhole = 0, kColour = 1, kLuminance = 2 };
+
 // COMPACT_IN: a sample decoded from the compact planes. Its radiance is the square of a
-// non-negative half, so sqrt(max(0, L)) is exactly that half (in.root), no quotient's dividend is
-// -0, and the random-dimension bins come with it (in.bins).
-template <bool COMPACT_IN = false>
+// non-negative half, so sqrt(max(0, L)) is exactly that half (in.root) and no dividend is infinite,
+// and the random-dimension bins come with it (in.bins).
+template <bool COMPACT_IN, Part PART>
 __device__ __forceinline__ void process_sample(PixelAcc& a, const SampleIn& in, bool per_sample_albedo,
                                                const float* palb, bool prep, uint8_t plane_mask, float fx,
                                                float fy, int bin_pixels, float& lum_out, uint32_t& key_out) {
+    constexpr bool colour = PART != kLuminance, lumi = PART != kColour;
     if (in.f & RPD_SAMPLE_HIT) {  // main.cpp:572-576
-        ++a.hits;
-        for (int c = 0; c < 3; ++c) a.nor[c] += in.n[c];
-        for (int c = 0; c < 3; ++c) a.alb[c] += per_sample_albedo ? in.alb[c] : palb[c];
-        a.dep += in.d;
+        if (lumi) {
+            ++a.hits;
+            a.dep += in.d;
+        }
+        if (colour) {
+            for (int c = 0; c < 3; ++c) a.nor[c] += in.n[c];
+            for (int c = 0; c < 3; ++c) a.alb[c] += per_sample_albedo ? in.alb[c] : palb[c];
+        }
     }
     if (!finite3(in.L[0], in.L[1], in.L[2])) {  // main.cpp:707
         lum_out = __int_as_float(0x7fc00000);  // NaN: dropped by the grid pass
         key_out = kKeyNone;
         return;
     }
-    // accumulate_sample (core/stats.h:25-41)
-    const float lum = luminance(in.L[0], in.L[1], in.L[2]);
-    const float delta = lum - a.mean;
+    // accumulate_sample (core/stats.h:25-41). The quotients by n come from one reciprocal where
+    // that is exact (div_markstein): the dividends are known before any of the updates. (Of a -0
+    // it makes +0, which the running means, never -0, add the same.) FP32 planes took seven
+    // divisions: 1920x1080x16 of path-like samples 0.98 -> 0.76 ms, adaptive counts 541 -> 469 us.
     ++a.n;
-    if (COMPACT_IN) {
-        // the seven quotients by n from one reciprocal, each still the IEEE quotient (the
-        // dividends are known before any of the updates)
-        const float fn = float(a.n);
-        float cd[3], sd[3];
-        bool fast = a.n < (1 << 23) && markstein_ok(delta);
+    const float fn = float(a.n);
+    float lum = 0.0f, delta = 0.0f, cd[3], root[3], sd[3];
+    bool fast = a.n < (1 << 23);
+    float size = 0.0f;  // FP32 radiance near the type's limits: a dividend may be infinite
+    if (lumi) {
+        lum = luminance(in.L[0], in.L[1], in.L[2]);
+        delta = lum - a.mean;
+        size += fabsf(delta);
+        fast = fast && markstein_ok(delta);
+    }
+    if (colour) {
         for (int c = 0; c < 3; ++c) {
+            root[c] = COMPACT_IN ? in.root[c] : sqrtf(fmaxs(0.0f, in.L[c]));
             cd[c] = in.L[c] - a.cm[c];
-            sd[c] = in.root[c] - a.sm[c];
+            sd[c] = root[c] - a.sm[c];
+            size += fabsf(cd[c]);
             fast = fast && markstein_ok(cd[c]) && markstein_ok(sd[c]);
         }
-        if (fast) {
-            const float rn = 1.0f / fn;
-            a.mean += div_markstein(delta, fn, rn);
+    }
+    if (!COMPACT_IN) fast = fast && size < INFINITY;
+    if (fast) {
+        const float rn = 1.0f / fn;
+        if (lumi) a.mean += div_markstein(delta, fn, rn);
+        if (colour) {
             for (int c = 0; c < 3; ++c) a.cm[c] += div_markstein(cd[c], fn, rn);
             for (int c = 0; c < 3; ++c) a.sm[c] += div_markstein(sd[c], fn, rn);
-        } else {
-            a.mean += delta / fn;
+        }
+    } else {
+        if (lumi) a.mean += delta / fn;
+        if (colour) {
             for (int c = 0; c < 3; ++c) a.cm[c] += cd[c] / fn;
             for (int c = 0; c < 3; ++c) a.sm[c] += sd[c] / fn;
         }
-        const float delta2 = lum - a.mean;
-        a.m2 += delta * delta2;
-        for (int c = 0; c < 3; ++c) a.sq[c] += sd[c] * (in.root[c] - a.sm[c]);
-    } else {
-        a.mean += delta / float(a.n);
-        const float delta2 = lum - a.mean;
-        a.m2 += delta * delta2;
-        for (int c = 0; c < 3; ++c) {
-            const float cd = in.L[c] - a.cm[c];
-            a.cm[c] += cd / float(a.n);
-        }
-        for (int c = 0; c < 3; ++c) {
-            const float sc = sqrtf(fmaxs(0.0f, in.L[c]));
-            const float sd = sc - a.sm[c];
-            a.sm[c] += sd / float(a.n);
-            a.sq[c] += sd * (sc - a.sm[c]);
-        }
     }
-    for (int c = 0; c < 3; ++c) a.rad[c] += in.L[c];
+    if (colour) {
+        for (int c = 0; c < 3; ++c) a.sq[c] += sd[c] * (root[c] - a.sm[c]);
+        for (int c = 0; c < 3; ++c) a.rad[c] += in.L[c];
+    }
+    if (!lumi) return;
+    const float delta2 = lum - a.mean;
+    a.m2 += delta * delta2;
     ++a.nsamples;
     lum_out = lum;
     key_out = kKeyNone;
@@ -396,21 +408,26 @@ __device__ __forceinline__ void acc_zero(PixelAcc& a) {
     a.hits = a.nsamples = 0;
 }
 
+template <Part PART>
 __device__ __forceinline__ void acc_load(PixelAcc& a, const PixelPlanes& p, int64_t idx) {
-    a.mean = p.mean[idx];
-    a.m2 = p.square_diff[idx];
     a.n = p.n[idx];
-    for (int c = 0; c < 3; ++c) {
-        a.cm[c] = p.color_mean[c][idx];
-        a.sm[c] = p.sqrt_mean[c][idx];
-        a.sq[c] = p.sqrt_sq[c][idx];
-        a.rad[c] = p.radiance[c][idx];
-        a.nor[c] = p.normal[c][idx];
-        a.alb[c] = p.albedo[c][idx];
+    if (PART != kLuminance) {
+        for (int c = 0; c < 3; ++c) {
+            a.cm[c] = p.color_mean[c][idx];
+            a.sm[c] = p.sqrt_mean[c][idx];
+            a.sq[c] = p.sqrt_sq[c][idx];
+            a.rad[c] = p.radiance[c][idx];
+            a.nor[c] = p.normal[c][idx];
+            a.alb[c] = p.albedo[c][idx];
+        }
     }
-    a.dep = p.depth[idx];
-    a.hits = p.hit_count[idx];
-    a.nsamples = p.sample_count[idx];
+    if (PART != kColour) {
+        a.mean = p.mean[idx];
+        a.m2 = p.square_diff[idx];
+        a.dep = p.depth[idx];
+        a.hits = p.hit_count[idx];
+        a.nsamples = p.sample_count[idx];
+    }
 }
 
 // The grid-pass sums of a pixel (GridPrep): its first pattern's, and either its further patterns' or, for a
@@ -461,23 +478,28 @@ __device__ __forceinline__ void store_classes(const Acc& a, const GridPrep& gp, 
 
 // The pixel's statistics back to its planes, and its grid-pass sums: the pattern class's, and
 // for a deviant pixel the full per-class sums.
+template <Part PART>
 __device__ __forceinline__ void acc_store(const PixelAcc& a, const PixelPlanes& p, const GridPrep& gp, int64_t idx,
                                           bool prep) {
-    p.mean[idx] = a.mean;
-    p.square_diff[idx] = a.m2;
-    p.n[idx] = a.n;
-    for (int c = 0; c < 3; ++c) {
-        p.color_mean[c][idx] = a.cm[c];
-        p.sqrt_mean[c][idx] = a.sm[c];
-        p.sqrt_sq[c][idx] = a.sq[c];
-        p.radiance[c][idx] = a.rad[c];
-        p.normal[c][idx] = a.nor[c];
-        p.albedo[c][idx] = a.alb[c];
+    if (PART != kLuminance) {
+        for (int c = 0; c < 3; ++c) {
+            p.color_mean[c][idx] = a.cm[c];
+            p.sqrt_mean[c][idx] = a.sm[c];
+            p.sqrt_sq[c][idx] = a.sq[c];
+            p.radiance[c][idx] = a.rad[c];
+            p.normal[c][idx] = a.nor[c];
+            p.albedo[c][idx] = a.alb[c];
+        }
     }
-    p.depth[idx] = a.dep;
-    p.hit_count[idx] = a.hits;
-    p.sample_count[idx] = a.nsamples;
-    if (prep) store_classes(a, gp, idx, a.pflags);
+    if (PART != kColour) {
+        p.mean[idx] = a.mean;
+        p.square_diff[idx] = a.m2;
+        p.n[idx] = a.n;
+        p.depth[idx] = a.dep;
+        p.hit_count[idx] = a.hits;
+        p.sample_count[idx] = a.nsamples;
+        if (prep) store_classes(a, gp, idx, a.pflags);
+    }
 }
 
 __device__ __forceinline__ uint8_t plane_mask_of(bool pu, bool lu, bool bu, bool li, bool eu) {
@@ -510,6 +532,7 @@ struct Quad32 {
     float4 L[3], N[3], A[3], D, PU[2], LU[2], BU[2], LI[2], EU[2];
     uint32_t F, C;
 };
+template <Part PART>
 __device__ __forceinline__ void process_quad(PixelAcc& a, const Quad32& q, const PixelIn& px, float* lum, uint32_t* key) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -529,7 +552,7 @@ __device__ __forceinline__ void process_quad(PixelAcc& a, const Quad32& q, const
         }
         in.f = uint8_t(q.F >> (8 * i));
         in.cat = uint8_t(q.C >> (8 * i));
-        process_sample(a, in, px.per_sample_albedo, px.palb, px.prep, px.plane_mask, px.fx, px.fy, px.bin_pixels, lum[i], key[i]);
+        process_sample<false, PART>(a, in, px.per_sample_albedo, px.palb, px.prep, px.plane_mask, px.fx, px.fy, px.bin_pixels, lum[i], key[i]);
     }
 }
 
@@ -544,7 +567,7 @@ struct Group16 {
     Words<V> L[3], N[3], D, PU[2], LU[2], BU[2], LI[2], EU[2];
     uint32_t F[V / 4], C[V / 4];
 };
-template <int V>
+template <int V, Part PART>
 __device__ __forceinline__ void process_group(PixelAcc& a, const Group16<V>& q, const PixelIn& px, float dscale, float* lum,
                                               uint32_t* key) {
 #pragma unroll
@@ -562,7 +585,7 @@ __device__ __forceinline__ void process_group(PixelAcc& a, const Group16<V>& q, 
                   (bin2d_q(q.LI[0].at(i), q.LI[1].at(i)) << 10) | (bin2d_q(q.EU[0].at(i), q.EU[1].at(i)) << 15);
         in.f = uint8_t(q.F[i >> 2] >> (8 * (i & 3)));
         in.cat = uint8_t(q.C[i >> 2] >> (8 * (i & 3)));
-        process_sample<true>(a, in, false, px.palb, px.prep, px.plane_mask, px.fx, px.fy, px.bin_pixels, lum[i], key[i]);
+        process_sample<true, PART>(a, in, false, px.palb, px.prep, px.plane_mask, px.fx, px.fy, px.bin_pixels, lum[i], key[i]);
     }
 }
 template <int V>
@@ -577,16 +600,13 @@ __device__ __forceinline__ void store_prep(const GridPrep& gp, int64_t k, const 
 // VEC4: every present plane is 16-byte aligned at the pixel's first sample and the pixel's
 // sample count is a multiple of 4, so each plane is read four samples per load. COMPACT: the
 // planes are rpd_sample_soa16's (s.c16), decoded to float here; WIDE reads them 8 samples (16
-// bytes) per load. MINB: resident blocks per SM the register allocation must allow.
-template <bool VEC4, bool COMPACT, bool WIDE, int MINB>
-__global__ void __launch_bounds__(128, MINB) k_accumulate_pixels(PixelPlanes p, DeviceSamples s, const int64_t* offsets,
-                                                           int32_t spp, int64_t first, int64_t count, GridPrep gp,
-                                                           int fresh) {
-    const int64_t local = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (local >= count) return;
+// bytes) per load. PART: what the thread keeps of its pixel.
+template <bool VEC4, bool COMPACT, bool WIDE, Part PART>
+__device__ __forceinline__ void accumulate_pixel(const PixelPlanes& p, const DeviceSamples& s, const int64_t* offsets,
+                                                 int64_t local, int64_t first, const GridPrep& gp, int fresh) {
+    constexpr bool colour = PART != kLuminance, lumi = PART != kColour;
     const int64_t idx = first + local;
-    const int64_t k0 = offsets ? offsets[local] : local * spp;
-    const int64_t k1 = offsets ? offsets[local + 1] : (local + 1) * spp;
+    const int64_t k0 = offsets[local], k1 = offsets[local + 1];
     const bool prep = gp.lum != nullptr;
     const bool has_pu = COMPACT ? s.c16.pixel_u[0] != nullptr : s.pixel_u[0] != nullptr;
     const bool has_lu = COMPACT ? s.c16.lens_u[0] != nullptr : s.lens_u[0] != nullptr;
@@ -606,15 +626,15 @@ __global__ void __launch_bounds__(128, MINB) k_accumulate_pixels(PixelPlanes p, 
     a.cs = cls_local + (uint32_t(gp.width) >> 31);  // the width is positive: offset 0
     acc_init(a);
     if (k0 == k1) {
-        if (prep) acc_store_empty(gp, idx);
+        if (prep && lumi) acc_store_empty(gp, idx);
         return;
     }
     // fresh: the frame's first push over every pixel, whose statistics the frame start zeroed
     if (fresh) acc_zero(a);
-    else acc_load(a, p, idx);
+    else acc_load<PART>(a, p, idx);
     px.per_sample_albedo = !COMPACT && s.albedo[0] != nullptr;
     load_pixel_albedo<COMPACT>(px, s, local);
-    const bool dims = prep;  // the random dimensions are only read for the grid pass
+    const bool dims = prep && lumi;  // the random dimensions are only read for the grid pass
 
     if (COMPACT) {
         const DeviceSamples16& h = s.c16;
@@ -642,9 +662,9 @@ __global__ void __launch_bounds__(128, MINB) k_accumulate_pixels(PixelPlanes p, 
                 const Words<V> z{};
                 for (int c = 0; c < 3; ++c) {
                     q.L[c] = ldv(h.sqrt_radiance[c], k);
-                    q.N[c] = ldv(h.normal[c], k);
+                    q.N[c] = colour ? ldv(h.normal[c], k) : z;
                 }
-                q.D = ldv(h.depth, k);
+                q.D = lumi ? ldv(h.depth, k) : z;
                 for (int c = 0; c < 2; ++c) {
                     q.PU[c] = (dims && has_pu) ? ldv(h.pixel_u[c], k) : z;
                     q.LU[c] = (dims && has_lu) ? ldv(h.lens_u[c], k) : z;
@@ -658,8 +678,8 @@ __global__ void __launch_bounds__(128, MINB) k_accumulate_pixels(PixelPlanes p, 
                 }
                 float lum[V];
                 uint32_t key[V];
-                process_group<V>(a, q, px, dscale, lum, key);
-                if (prep) store_prep<V>(gp, k, lum, key);
+                process_group<V, PART>(a, q, px, dscale, lum, key);
+                if (dims) store_prep<V>(gp, k, lum, key);
             }
         } else {
             for (int64_t k = k0; k < k1; ++k) {
@@ -667,10 +687,10 @@ __global__ void __launch_bounds__(128, MINB) k_accumulate_pixels(PixelPlanes p, 
                 for (int c = 0; c < 3; ++c) {
                     in.root[c] = fabsf(h2f(h.sqrt_radiance[c][k]));
                     in.L[c] = sq(in.root[c]);
-                    in.n[c] = snorm16(h.normal[c][k]);
+                    in.n[c] = colour ? snorm16(h.normal[c][k]) : 0.0f;
                     in.alb[c] = 0.0f;
                 }
-                in.d = h2f(h.depth[k]) * dscale;
+                in.d = lumi ? h2f(h.depth[k]) * dscale : 0.0f;
                 uint16_t q[4][2];
                 for (int c = 0; c < 2; ++c) {
                     in.pu[c] = (dims && has_pu) ? unorm16(h.pixel_u[c][k]) : 0.0f;
@@ -685,8 +705,8 @@ __global__ void __launch_bounds__(128, MINB) k_accumulate_pixels(PixelPlanes p, 
                 in.cat = (dims && s.category) ? s.category[k] : 0;
                 float lum;
                 uint32_t key;
-                process_sample<true>(a, in, false, px.palb, prep, px.plane_mask, px.fx, px.fy, px.bin_pixels, lum, key);
-                if (prep) {
+                process_sample<true, PART>(a, in, false, px.palb, prep, px.plane_mask, px.fx, px.fy, px.bin_pixels, lum, key);
+                if (dims) {
                     gp.lum[k] = lum;
                     gp.key[k] = key;
                     if (gp.col) gp.col[k] = uint16_t(idx % gp.width);
@@ -699,10 +719,10 @@ __global__ void __launch_bounds__(128, MINB) k_accumulate_pixels(PixelPlanes p, 
             const float4 z4 = make_float4(0, 0, 0, 0);
             for (int c = 0; c < 3; ++c) {
                 q.L[c] = ld4(s.radiance[c], k);
-                q.N[c] = ld4(s.normal[c], k);
-                q.A[c] = px.per_sample_albedo ? ld4(s.albedo[c], k) : z4;
+                q.N[c] = colour ? ld4(s.normal[c], k) : z4;
+                q.A[c] = colour && px.per_sample_albedo ? ld4(s.albedo[c], k) : z4;
             }
-            q.D = ld4(s.depth, k);
+            q.D = lumi ? ld4(s.depth, k) : z4;
             for (int c = 0; c < 2; ++c) {
                 q.PU[c] = (dims && s.pixel_u[0]) ? ld4(s.pixel_u[c], k) : z4;
                 q.LU[c] = (dims && s.lens_u[0]) ? ld4(s.lens_u[c], k) : z4;
@@ -714,18 +734,18 @@ __global__ void __launch_bounds__(128, MINB) k_accumulate_pixels(PixelPlanes p, 
             q.C = (dims && s.category) ? *reinterpret_cast<const uint32_t*>(s.category + k) : 0u;
             float lum[4];
             uint32_t key[4];
-            process_quad(a, q, px, lum, key);
-            if (prep) store_prep<4>(gp, k, lum, key);
+            process_quad<PART>(a, q, px, lum, key);
+            if (dims) store_prep<4>(gp, k, lum, key);
         }
     } else {
         for (int64_t k = k0; k < k1; ++k) {
             SampleIn in;
             for (int c = 0; c < 3; ++c) {
                 in.L[c] = s.radiance[c][k];
-                in.n[c] = s.normal[c][k];
-                in.alb[c] = px.per_sample_albedo ? s.albedo[c][k] : 0.0f;
+                in.n[c] = colour ? s.normal[c][k] : 0.0f;
+                in.alb[c] = colour && px.per_sample_albedo ? s.albedo[c][k] : 0.0f;
             }
-            in.d = s.depth[k];
+            in.d = lumi ? s.depth[k] : 0.0f;
             for (int c = 0; c < 2; ++c) {
                 in.pu[c] = (dims && s.pixel_u[0]) ? s.pixel_u[c][k] : 0.0f;
                 in.lu[c] = (dims && s.lens_u[0]) ? s.lens_u[c][k] : 0.0f;
@@ -737,8 +757,8 @@ __global__ void __launch_bounds__(128, MINB) k_accumulate_pixels(PixelPlanes p, 
             in.cat = (dims && s.category) ? s.category[k] : 0;
             float lum;
             uint32_t key;
-            process_sample(a, in, px.per_sample_albedo, px.palb, prep, px.plane_mask, px.fx, px.fy, px.bin_pixels, lum, key);
-            if (prep) {
+            process_sample<false, PART>(a, in, px.per_sample_albedo, px.palb, prep, px.plane_mask, px.fx, px.fy, px.bin_pixels, lum, key);
+            if (dims) {
                 gp.lum[k] = lum;
                 gp.key[k] = key;
                 if (gp.col) gp.col[k] = uint16_t(idx % gp.width);
@@ -746,7 +766,28 @@ __global__ void __launch_bounds__(128, MINB) k_accumulate_pixels(PixelPlanes p, 
         }
     }
 
-    acc_store(a, p, gp, idx, prep);
+    acc_store<PART>(a, p, gp, idx, prep);
+}
+
+// MINB: resident blocks per SM the register allocation must allow. SPLIT: two warps of a block share 32
+// pixels, one part each. The general form is bound by the latency of its loads and of the chain of
+// updates (40 % of the issue slots at 12 warps per SM, 156 registers a thread). Single samples per load
+// leave registers to halve: 16 warps' worth of pixels in 32 warps, 1283x717x6 168 -> 134 us, compact
+// 1920x1080x6 267 -> 226, adaptive counts over 1280x720 469 -> 426 us per frame. Four samples
+// per load do not: 24 split warps read more lines at a time than L1 holds (1920x1080x16 0.64 -> 0.72 ms).
+template <bool VEC4, bool COMPACT, bool WIDE, int MINB, bool SPLIT>
+__global__ void __launch_bounds__(128, MINB) k_accumulate_pixels(PixelPlanes p, DeviceSamples s, const int64_t* offsets,
+                                                                 int64_t first, int64_t count, GridPrep gp, int fresh) {
+    if constexpr (SPLIT) {
+        const int64_t local = int64_t(blockIdx.x) * 64 + (threadIdx.x & 63);
+        if (local >= count) return;
+        if (threadIdx.x < 64) accumulate_pixel<VEC4, COMPACT, WIDE, kLuminance>(p, s, offsets, local, first, gp, fresh);
+        else accumulate_pixel<VEC4, COMPACT, WIDE, kColour>(p, s, offsets, local, first, gp, fresh);
+    } else {
+        const int64_t local = int64_t(blockIdx.x) * 128 + threadIdx.x;
+        if (local >= count) return;
+        accumulate_pixel<VEC4, COMPACT, WIDE, kWhole>(p, s, offsets, local, first, gp, fresh);
+    }
 }
 
 // ---- the statistics pass on staged rows ------------------------------------------------------------
@@ -1395,14 +1436,13 @@ const int64_t* offsets_count_max(const Job& j, int64_t count) {
 // The statistics pass uses no shared memory: its launches ask for the whole unified array as L1,
 // which keeps more of the sample sectors a thread reads again a step later (3 % more throughput
 // on the served stream, where other requests' kernels share the SMs).
-template <bool VEC4, bool COMPACT, bool WIDE, int MINB>
-cudaError_t run_accumulate(Job& j, unsigned blocks, const DeviceSamples& s, int64_t first, int64_t count,
-                           const GridPrep& gp, int fresh) {
-    const cudaError_t e = cudaFuncSetAttribute(k_accumulate_pixels<VEC4, COMPACT, WIDE, MINB>,
+template <bool VEC4, bool COMPACT, bool WIDE, int MINB, bool SPLIT>
+cudaError_t run_accumulate(Job& j, const DeviceSamples& s, int64_t first, int64_t count, const GridPrep& gp, int fresh) {
+    const cudaError_t e = cudaFuncSetAttribute(k_accumulate_pixels<VEC4, COMPACT, WIDE, MINB, SPLIT>,
                                                cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxL1);
     if (e != cudaSuccess) return e;
-    k_accumulate_pixels<VEC4, COMPACT, WIDE, MINB><<<blocks, 128, 0, j.stream>>>(j.p, s, j.offsets, 0, first, count, gp,
-                                                                              fresh);
+    k_accumulate_pixels<VEC4, COMPACT, WIDE, MINB, SPLIT><<<grid_for(count, SPLIT ? 64 : 128), 128, 0, j.stream>>>(
+        j.p, s, j.offsets, first, count, gp, fresh);
     return cudaSuccess;
 }
 
@@ -1522,10 +1562,9 @@ cudaError_t launch_accumulate_pixels(Job& j, const DeviceSamples& s, int64_t fir
                    (!s.env_u[0] || aligned(s.env_u[c], 16));
     }
     vec4 = vec4 && (!gp.lum || (aligned(gp.lum, 16) && aligned(gp.key, 16)));
-    const unsigned blocks = grid_for(count, 128);
     // Shapes measured on GB300 at 1920x1080. Up to 16 samples per pixel, more resident pixels
-    // hide the per-pixel latency (compact planes 4 blocks per SM, FP32 planes 3; per-pixel counts
-    // 4 over compact planes, 5 over FP32 planes). From 32 on, a thread's sample run spans more bytes per plane than L1 keeps between its
+    // hide the per-pixel latency (four samples per load: compact planes 4 blocks per SM, FP32 planes
+    // 3; single samples, the pixel split over two warps: 8). From 32 on, a thread's sample run spans more bytes per plane than L1 keeps between its
     // loads, and a block's registers are not capped; from 64 on, compact planes are read 16 bytes
     // (8 samples) per load.
     const bool many = spp > 16;
@@ -1540,20 +1579,20 @@ cudaError_t launch_accumulate_pixels(Job& j, const DeviceSamples& s, int64_t fir
                    (!h.brdf_u[0] || aligned(h.brdf_u[c], 16)) && (!h.light_u[0] || aligned(h.light_u[c], 16)) &&
                    (!h.env_u[0] || aligned(h.env_u[c], 16));
         if (wide)
-            e = run_accumulate<true, true, true, 1>(j, blocks, s, first, count, gp, fresh);
+            e = run_accumulate<true, true, true, 1, false>(j, s, first, count, gp, fresh);
         else if (vec4 && many)
-            e = run_accumulate<true, true, false, 1>(j, blocks, s, first, count, gp, fresh);
+            e = run_accumulate<true, true, false, 1, false>(j, s, first, count, gp, fresh);
         else if (vec4)
-            e = run_accumulate<true, true, false, 4>(j, blocks, s, first, count, gp, fresh);
+            e = run_accumulate<true, true, false, 4, false>(j, s, first, count, gp, fresh);
         else
-            e = run_accumulate<false, true, false, 4>(j, blocks, s, first, count, gp, fresh);
+            e = run_accumulate<false, true, false, 8, true>(j, s, first, count, gp, fresh);
     } else {
         if (vec4 && many)
-            e = run_accumulate<true, false, false, 1>(j, blocks, s, first, count, gp, fresh);
+            e = run_accumulate<true, false, false, 1, false>(j, s, first, count, gp, fresh);
         else if (vec4)
-            e = run_accumulate<true, false, false, 3>(j, blocks, s, first, count, gp, fresh);
+            e = run_accumulate<true, false, false, 3, false>(j, s, first, count, gp, fresh);
         else
-            e = run_accumulate<false, false, false, 5>(j, blocks, s, first, count, gp, fresh);
+            e = run_accumulate<false, false, false, 8, true>(j, s, first, count, gp, fresh);
     }
     if (e != cudaSuccess) return e;
     j.launches += 1;
