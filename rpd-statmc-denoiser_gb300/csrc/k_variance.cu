@@ -1,16 +1,18 @@
 // variance_denoise (main.cpp:1166-1268): Jacobi iterations of the gated neighbour mean
-// with the upward-only update, ping-ponging two planes, then max with the raw variance.
+// with the upward-only update, ping-ponging two planes, the last into the denoised variance.
 // Single precision throughout, in the reference's order, so the result is bit-identical.
 //
 // The ping-pong planes carry the hit test in their sign: a pixel with a primary hit holds its
 // variance (>= EPS_SMALL), a pixel without one the negated clamped variance, which the
-// iterations copy unchanged (main.cpp:1198-1201) and the final max with the clamped raw
-// variance turns back into the value the reference keeps. A block's halo tile is then the
+// iterations copy unchanged (main.cpp:1198-1201) and the last one turns back into the value
+// the reference keeps. A block's halo tile is then the
 // plane's box as it lies in HBM — the tensor copy's zero fill past the image edges reads as
 // "no neighbour" like a pixel without a hit — so each iteration stages its tile with one
 // tiled tensor copy (cp.async.bulk.tensor) instead of per-thread gathers, and the gate records
 // (unit normal, depth) with a second one. Rows of the ping-pong planes are padded to 4 floats,
 // the 16-byte row pitch tensor copies need.
+#include <cmath>
+
 #include "rpd_internal.h"
 #include "device_math.cuh"
 #include "tma.cuh"
@@ -40,6 +42,10 @@ __global__ void k_var_init(PixelPlanes p, int w, int h, int pitch, float max_var
 struct VarParams {
     int w, h, radius, pitch;
     float normal_threshold, depth_threshold, compat_sigma, shrinkage_k;
+    float depth_half_ulp;  // half an ulp of the depth threshold
+    // |1 - x| / sqrt(x) > compat_sigma for the ratio x of two variances: surely not for
+    // lo_in <= x <= hi_in, surely for x < lo_out and x > hi_out (ratio_bounds)
+    float lo_out, lo_in, hi_in, hi_out;
 };
 
 // rpf::conservative_variance_update (core/stats.h:85-91)
@@ -48,7 +54,8 @@ __device__ __forceinline__ float conservative_variance_update(float value, float
     return lerp_std(value, neighbor, blend);
 }
 
-constexpr int kVarTx = 32, kVarTy = 16;
+constexpr int kVarTx = 32, kVarTy = 16;  // a block's pixels
+constexpr int kVarRows = 2;              // pixels of a thread, one above the other
 constexpr float kGateBand = 1.0f / 1048576.0f;  // 2^-20
 constexpr int kVarPad = 4;  // the variance box starts 4 floats left of the block (a 16-byte boundary)
 
@@ -65,6 +72,13 @@ __device__ __forceinline__ bool depth_far(float dabs_i, float di, float dj, floa
     if (tm >= 1e-30f && (d_hi || d_lo)) return d_hi;
     return num / m > dthr;
 }
+// The same decision by one exact fused difference (k_statmc.cu's depth_far, with its reasons), for
+// thresholds of at least 1e-21. dm: max(|d_i|, EPS_SMALL).
+__device__ __forceinline__ bool depth_far_fused(float di, float dm, float dj, float dthr, float half_ulp) {
+    float m = dm;
+    if (m < fabsf(dj)) m = fabsf(dj);
+    return __fmaf_rn(-dthr, m, fabsf(di - dj)) > m * half_ulp;
+}
 
 // |var_i - var_j| / max(EPS_SMALL, sqrt(var_i * var_j)) > compat_sigma (main.cpp:1228-1232),
 // by a reciprocal square root away from the threshold and the IEEE quotient near it.
@@ -76,21 +90,67 @@ __device__ __forceinline__ bool incompatible(float var_i, float var_j, float sig
     return diff / fmaxs(1e-8f, sqrtf(prod)) > sigma;
 }
 
+// A thread's pixel: its variance, the bounds of the variances it is compatible with, its feature gate
+// and the sums over its window.
+template <int R>
+struct VarPixel {
+    static constexpr int kWords = ((2 * R + 1) * (2 * R + 1) - 1 + 31) / 32;
+    float var, lo_out, lo_in, hi_in, hi_out;
+    float4 g;
+    float dm;                // max(|depth|, EPS_SMALL)
+    uint32_t gate[kWords];   // the neighbours the hit, normal and depth gates pass, in window order
+    float weighted, weight;  // over the surely compatible neighbours
+    float may_weight;        // over those that may be: more than `weight` if a ratio lies between the bounds
+};
+
+// The pixel's sums again, every ratio by the reference's quotient.
+template <int R>
+__device__ __noinline__ float2 var_exact_sums(const float* V, int vw, float var_i, uint32_t g0, uint32_t g1, uint32_t g2,
+                                            float sigma) {
+    constexpr int side = 2 * R + 1, n = side * side - 1;
+    float weighted = 0.0f, weight = 0.0f;
+    for (int b = 0; b < n; ++b) {
+        if (!(((b < 32 ? g0 : b < 64 ? g1 : g2) >> (b & 31)) & 1u)) continue;
+        const int e = b < n / 2 ? b : b + 1;
+        const int dy = e / side - R, dx = e % side - R;
+        const float var_j = V[dy * vw + dx];
+        if (incompatible(var_i, var_j, sigma)) continue;
+        const float w_j = 1.0f / (1.0f + float(dx * dx + dy * dy));
+        weighted += w_j * var_j;
+        weight += w_j;
+    }
+    return make_float2(weighted, weight);
+}
+
 // One Jacobi iteration (main.cpp:1198-1249) with the radius fixed at compile time. A 32 x 16
 // block's halo tile arrives by tensor copies: the variance box (the 4-float-aligned
 // (32 + 8) x (16 + 2R) floats) and, unless MODE 2, the gate records' (32 + 2R) x (16 + 2R) box.
-// The window is unrolled, every gate is evaluated as a predicate (the lanes of a warp stay
-// converged; the quotient gates branch only within the bands of their thresholds), and the
-// accepted neighbours are added in the reference's order; a rejected neighbour adds nothing, as
-// the reference's `continue` does.
+// The window is unrolled; a thread's two pixels read each of its rows once; every gate is a
+// predicate (the lanes of a warp stay converged), and the accepted neighbours are added in the
+// reference's order; a rejected neighbour adds nothing, as the reference's `continue` does.
 //
 // The hit, normal and depth gates depend on the features only, which the iterations do not
 // change. MODE 0 evaluates every gate; MODE 1 also writes each pixel's geometric-gate bits (one
 // per neighbour, in window order) to var_mask; MODE 2 reads them and evaluates only the
 // variance-compatibility gate of the neighbours they pass.
+//
+// That gate compares |var_i - var_j| / max(EPS_SMALL, sqrt(var_i var_j)) with sigma, which for a given
+// var_i is a test of var_j against two bounds. Within 2^-19 of a bound, where the quotient's rounding
+// decides, the pixel's sums are taken again with the quotient itself (var_exact_sums). Passed neighbours are at
+// least EPS_SMALL, as is every value of the planes for a pixel with a hit (the update only raises it), so
+// the reference's maxima with EPS_SMALL change nothing.
+//
+// LAST: the iteration's result is the denoised variance itself. The reference takes the maximum with the
+// clamped raw variance (main.cpp:1252-1261), where the iterations began and below which none falls;
+// a pixel without a hit holds its negative.
+//
+// Bound by instruction issue. At 1920x1080, radius 3: MODE 1 184 us and MODE 2 94 us with one pixel per
+// thread, an rsqrt and two guarded quotients per neighbour, 17 us for the
+// final maximum; 119 and 62 us with the bounds, two pixels per thread and the fused depth gate (124 and 67 with
+// an uncertainty flag per neighbour instead of a second weight sum).
 template <int R, int MODE>
-__global__ void __launch_bounds__(kVarTx * kVarTy)
-    k_var_smooth_r(PixelPlanes p, VarParams prm, float* dst, unsigned long long* timeouts,
+__global__ void __launch_bounds__(kVarTx * kVarTy / kVarRows)
+    k_var_smooth_r(PixelPlanes p, VarParams prm, float* dst, int dst_pitch, bool last, unsigned long long* timeouts,
                    const __grid_constant__ CUtensorMap gmap, const __grid_constant__ CUtensorMap vmap) {
     static_assert(R <= kVarPad, "the variance box covers a halo of at most 4 columns");
     static_assert(MODE == 0 || (2 * R + 1) * (2 * R + 1) - 1 <= 64, "the gate bits fit one word");
@@ -121,61 +181,100 @@ __global__ void __launch_bounds__(kVarTx * kVarTy)
         }
         return;
     }
-    const int x = x0 + threadIdx.x, y = y0 + threadIdx.y;
+    const int x = x0 + threadIdx.x, y = y0 + threadIdx.y * kVarRows;
     if (x >= prm.w || y >= prm.h) return;
-    const int64_t idx = int64_t(y) * prm.w + x;
-    const int64_t pidx = int64_t(y) * prm.pitch + x;
-    const int vi = (threadIdx.y + R) * vw + threadIdx.x + kVarPad;
-    const float src_i = V[vi];
-    if (!(src_i > 0.0f)) {  // no primary hit (hit_count == 0): copied unchanged
-        dst[pidx] = src_i;
-        return;
-    }
-    const float var_i = fmaxs(1e-8f, src_i);
-    const float sigma = prm.compat_sigma;
-    float weight_sum = 0.0f, weighted_sum = 0.0f;
-    uint64_t gates = MODE == 2 ? p.var_mask[idx] : 0ull;
-    float4 gi = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    const int gi_e = (threadIdx.y + R) * gw + threadIdx.x + R;
-    if (MODE != 2) gi = G[gi_e];
-    const float dabs_i = fabsf(gi.w);
-    int bit = 0;
+    // the first row and column of the thread's windows
+    const float* Vw = V + threadIdx.y * kVarRows * vw + threadIdx.x + kVarPad - R;
+    const float4* Gw = G + threadIdx.y * kVarRows * gw + threadIdx.x;
+    VarPixel<R> px[kVarRows];
+    float src[kVarRows];
 #pragma unroll
-    for (int dy = -R; dy <= R; ++dy) {
+    for (int k = 0; k < kVarRows; ++k) {
+        VarPixel<R>& q = px[k];
+        src[k] = Vw[(R + k) * vw + R];  // 0 below the image's last row
+        q.var = src[k];
+        q.lo_out = q.var * prm.lo_out;
+        q.lo_in = q.var * prm.lo_in;
+        q.hi_in = q.var * prm.hi_in;
+        q.hi_out = q.var * prm.hi_out;
+        q.weighted = q.weight = q.may_weight = 0.0f;
 #pragma unroll
-        for (int dx = -R; dx <= R; ++dx) {
-            if (dx == 0 && dy == 0) continue;
-            const float src_j = V[vi + dy * vw + dx];
-            bool ok;
-            if (MODE == 2) {
-                ok = (gates >> bit) & 1ull;
-            } else {
-                // outside the image (zero fill) or no primary hit (negative)
-                const float4 gj = G[gi_e + dy * gw + dx];
-                ok = src_j > 0.0f && !(dot3(gi.x, gi.y, gi.z, gj.x, gj.y, gj.z) < prm.normal_threshold);
-                ok = ok && !depth_far(dabs_i, gi.w, gj.w, prm.depth_threshold);
-                if (MODE == 1 && ok) gates |= 1ull << bit;
+        for (int b = 0; b < VarPixel<R>::kWords; ++b) q.gate[b] = 0u;
+        if (MODE == 2) {
+            if (y + k < prm.h) {
+                const uint64_t m = p.var_mask[int64_t(y + k) * prm.w + x];
+                q.gate[0] = uint32_t(m);
+                if (VarPixel<R>::kWords > 1) q.gate[VarPixel<R>::kWords > 1 ? 1 : 0] = uint32_t(m >> 32);
             }
-            ++bit;
-            const float var_j = fmaxs(1e-8f, src_j);
-            ok = ok && !incompatible(var_i, var_j, sigma);
-            const float w_j = 1.0f / (1.0f + float(dx * dx + dy * dy));
-            if (ok) {
-                weighted_sum += w_j * var_j;
-                weight_sum += w_j;
+        } else {
+            q.g = Gw[(R + k) * gw + R];
+            q.dm = fmaxs(fabsf(q.g.w), 1e-8f);
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 2 * R + kVarRows; ++j) {
+#pragma unroll
+        for (int i = 0; i <= 2 * R; ++i) {
+            const float var_j = Vw[j * vw + i];
+            float4 gj = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (MODE != 2) gj = Gw[j * gw + i];
+#pragma unroll
+            for (int k = 0; k < kVarRows; ++k) {
+                const int dy = j - k - R, dx = i - R;
+                if (dy < -R || dy > R || (dx == 0 && dy == 0)) continue;
+                const int e = (dy + R) * (2 * R + 1) + i, bit = e - (e > (2 * R + 1) * R + R ? 1 : 0);
+                VarPixel<R>& q = px[k];
+                bool ok;
+                if (MODE == 2) {
+                    ok = (q.gate[bit >> 5] >> (bit & 31)) & 1u;
+                } else {
+                    // outside the image (zero fill) or no primary hit (negative)
+                    ok = var_j > 0.0f && !(dot3(q.g.x, q.g.y, q.g.z, gj.x, gj.y, gj.z) < prm.normal_threshold);
+                    ok = ok && !depth_far_fused(q.g.w, q.dm, gj.w, prm.depth_threshold, prm.depth_half_ulp);
+                    if (ok) q.gate[bit >> 5] |= 1u << (bit & 31);
+                }
+                const float w_j = 1.0f / (1.0f + float(dx * dx + dy * dy));
+                if (ok && var_j >= q.lo_out && var_j <= q.hi_out) q.may_weight += w_j;
+                if (ok && var_j >= q.lo_in && var_j <= q.hi_in) {
+                    q.weighted += w_j * var_j;
+                    q.weight += w_j;
+                }
             }
         }
     }
-    if (MODE == 1) p.var_mask[idx] = gates;
-    float neighbor_mean = var_i;
-    if (weight_sum > 1e-8f) neighbor_mean = weighted_sum / weight_sum;
-    dst[pidx] = conservative_variance_update(var_i, neighbor_mean, prm.shrinkage_k);
+#pragma unroll
+    for (int k = 0; k < kVarRows; ++k) {
+        VarPixel<R>& q = px[k];
+        if (y + k >= prm.h) continue;
+        if (MODE == 1) {
+            uint64_t m = q.gate[0];
+            if (VarPixel<R>::kWords > 1) m |= uint64_t(q.gate[VarPixel<R>::kWords > 1 ? 1 : 0]) << 32;
+            p.var_mask[int64_t(y + k) * prm.w + x] = m;
+        }
+        float out = src[k];
+        if (src[k] > 0.0f) {
+            if (q.may_weight != q.weight) {
+                constexpr int n = VarPixel<R>::kWords;
+                const float2 s = var_exact_sums<R>(Vw + (R + k) * vw + R, vw, q.var, q.gate[0], q.gate[n > 1 ? 1 : 0],
+                                                   q.gate[n > 2 ? 2 : 0], prm.compat_sigma);
+                q.weighted = s.x;
+                q.weight = s.y;
+            }
+            float neighbor_mean = q.var;
+            if (q.weight > 1e-8f) neighbor_mean = q.weighted / q.weight;
+            out = conservative_variance_update(q.var, neighbor_mean, prm.shrinkage_k);
+        } else if (last) {
+            out = -src[k];  // no primary hit (hit_count == 0): its clamped raw variance
+        }
+        dst[int64_t(y + k) * dst_pitch + x] = out;
+    }
 }
 
-// The same iteration for radii above 4 (the radius at run time): the halo is gathered by the
+// The same iteration for radii above 4 (the radius at run time) and for parameters outside the bounds'
+// reasoning (launch_variance): the halo is gathered by the
 // threads into dynamic shared memory, the window loops at run time.
 __global__ void __launch_bounds__(kVarTx * kVarTy) k_var_smooth(PixelPlanes p, VarParams prm, const float* src,
-                                                                float* dst) {
+                                                                float* dst, int dst_pitch, bool last) {
     extern __shared__ float4 vsm[];
     const int r = prm.radius;
     const int tw = kVarTx + 2 * r, th = kVarTy + 2 * r, tn = tw * th;
@@ -198,11 +297,11 @@ __global__ void __launch_bounds__(kVarTx * kVarTy) k_var_smooth(PixelPlanes p, V
     __syncthreads();
     const int x = x0 + threadIdx.x, y = y0 + threadIdx.y;
     if (x >= prm.w || y >= prm.h) return;
-    const int64_t pidx = int64_t(y) * prm.pitch + x;
+    const int64_t pidx = int64_t(y) * dst_pitch + x;
     const int ei = (threadIdx.y + r) * tw + threadIdx.x + r;
     const float src_i = V[ei];
     if (!(src_i > 0.0f)) {
-        dst[pidx] = src_i;
+        dst[pidx] = last ? -src_i : src_i;
         return;
     }
     const float4 gi = G[ei];
@@ -261,14 +360,16 @@ cudaError_t launch_smooth_r(Job& j, const VarParams& prm, float*& curr, float*& 
     constexpr bool kMask = (2 * R + 1) * (2 * R + 1) - 1 <= 64;
     for (int it = 0; it < iters; ++it) {
         const CUtensorMap& vmap = curr == j.p.var_ping ? ping : pong;
+        const bool last = it + 1 == iters;
+        float* const dst = last ? j.p.variance_denoised : next;
+        const int dst_pitch = last ? prm.w : prm.pitch;
+        const dim3 block(kVarTx, kVarTy / kVarRows);
         if (!kMask || iters == 1)
-            k_var_smooth_r<R, 0><<<vgrid, dim3(kVarTx, kVarTy), 0, j.stream>>>(j.p, prm, next, timeouts, gmap, vmap);
+            k_var_smooth_r<R, 0><<<vgrid, block, 0, j.stream>>>(j.p, prm, dst, dst_pitch, last, timeouts, gmap, vmap);
         else if (it == 0)
-            k_var_smooth_r<R, kMask ? 1 : 0><<<vgrid, dim3(kVarTx, kVarTy), 0, j.stream>>>(j.p, prm, next, timeouts,
-                                                                                         gmap, vmap);
+            k_var_smooth_r<R, kMask ? 1 : 0><<<vgrid, block, 0, j.stream>>>(j.p, prm, dst, dst_pitch, last, timeouts, gmap, vmap);
         else
-            k_var_smooth_r<R, kMask ? 2 : 0><<<vgrid, dim3(kVarTx, kVarTy), 0, j.stream>>>(j.p, prm, next, timeouts,
-                                                                                         gmap, vmap);
+            k_var_smooth_r<R, kMask ? 2 : 0><<<vgrid, block, 0, j.stream>>>(j.p, prm, dst, dst_pitch, last, timeouts, gmap, vmap);
         float* t = curr;
         curr = next;
         next = t;
@@ -276,16 +377,17 @@ cudaError_t launch_smooth_r(Job& j, const VarParams& prm, float*& curr, float*& 
     return cudaGetLastError();
 }
 
-// max(iterated, clamped raw) (main.cpp:1252-1261); for a pixel without a hit the iterated plane
-// holds the negated clamped raw variance, so the max is the clamped raw variance.
-__global__ void k_var_final(PixelPlanes p, int w, int h, int pitch, float max_variance, const float* curr) {
-    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= int64_t(w) * h) return;
-    float raw = pixel_variance(p.square_diff[i], p.n[i]);
-    if (!isfinite(raw)) raw = 1e-8f;
-    raw = fclamps(raw, 1e-8f, max_variance);
-    const int64_t y = i / w, x = i - y * w;
-    p.variance_denoised[i] = fmaxs(curr[y * pitch + x], raw);
+// The ratio bounds of VarParams. With x the ratio of two variances, |1 - x| / sqrt(x) passes sigma at
+// ((sqrt(sigma^2 + 4) -+ sigma) / 2)^2, with a logarithmic slope of at least 1/2; the reference's float
+// quotient is off by less than 2^-22, so its decision can differ within 2^-21 of them; 2^-19 covers the bounds'
+// own roundings.
+void ratio_bounds(VarParams& prm) {
+    const double s = prm.compat_sigma, root = std::sqrt(s * s + 4.0), band = 1.0 / 524288.0;
+    const double hi = 0.25 * (root + s) * (root + s), lo = 1.0 / hi;
+    prm.lo_out = float(lo * (1.0 - band));
+    prm.lo_in = float(lo * (1.0 + band));
+    prm.hi_in = float(hi * (1.0 - band));
+    prm.hi_out = float(hi * (1.0 + band));
 }
 
 }  // namespace
@@ -300,10 +402,14 @@ cudaError_t launch_variance(Job& j) {
     k_var_init<<<grid_for(np, 256), 256, 0, j.stream>>>(j.p, j.g.w, j.g.h, pitch, max_variance, curr);
     VarParams prm{j.g.w, j.g.h, j.cfg.var_window_radius, pitch, j.cfg.var_normal_threshold, j.cfg.var_depth_threshold,
                   j.cfg.var_compat_sigma, j.cfg.var_shrinkage_k};
+    prm.depth_half_ulp = 0.5f * (std::nextafter(prm.depth_threshold, HUGE_VALF) - prm.depth_threshold);
+    ratio_bounds(prm);
     const int r = prm.radius;
     const dim3 vgrid((j.g.w + kVarTx - 1) / kVarTx, (j.g.h + kVarTy - 1) / kVarTy);
     cudaError_t e = cudaSuccess;
-    if (r >= 1 && r <= 4) {
+    // the bounds' reasoning wants products of variances in the normal range, the fused depth gate a
+    // threshold whose half ulp scales without underflow
+    if (r >= 1 && r <= 4 && max_variance <= 1e18f && prm.depth_threshold >= 1e-21f && prm.depth_threshold <= 1e18f) {
         e = r == 1 ? launch_smooth_r<1>(j, prm, curr, next, vgrid)
           : r == 2 ? launch_smooth_r<2>(j, prm, curr, next, vgrid)
           : r == 3 ? launch_smooth_r<3>(j, prm, curr, next, vgrid)
@@ -314,15 +420,16 @@ cudaError_t launch_variance(Job& j) {
         if (smem > size_t(200) * 1024) return cudaErrorInvalidValue;  // radius beyond the shared-memory tile
         e = cudaFuncSetAttribute(k_var_smooth, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
         for (int it = 0; it < j.cfg.var_iterations && e == cudaSuccess; ++it) {
-            k_var_smooth<<<vgrid, dim3(kVarTx, kVarTy), smem, j.stream>>>(j.p, prm, curr, next);
+            const bool last = it + 1 == j.cfg.var_iterations;
+            k_var_smooth<<<vgrid, dim3(kVarTx, kVarTy), smem, j.stream>>>(
+                j.p, prm, curr, last ? j.p.variance_denoised : next, last ? prm.w : pitch, last);
             float* t = curr;
             curr = next;
             next = t;
         }
     }
     if (e != cudaSuccess) return e;
-    k_var_final<<<grid_for(np, 256), 256, 0, j.stream>>>(j.p, j.g.w, j.g.h, pitch, max_variance, curr);
-    j.launches += 2 + j.cfg.var_iterations;
+    j.launches += 1 + j.cfg.var_iterations;
     return cudaGetLastError();
 }
 
