@@ -78,7 +78,6 @@ uint64_t plan(const Geometry& g, PixelPlanes& p, NodePlanes& n, float* (*cls)[5]
     L.add(p.var_total, np);
     L.add(p.var_eff, np);
     L.add(p.var_ratio, np);
-    for (int c = 0; c < 3; ++c) L.add(p.sqrt_var_mean[c], np);
     for (int c = 0; c < 3; ++c) L.add(p.sqrt_var_stable[c], np);
     L.add(p.win, 6 * np);
     L.add(p.variance_denoised, np);
@@ -132,7 +131,6 @@ void rebase_all(PixelPlanes& p, NodePlanes& n, char* base) {
         rebase(p.f_normal[c], base);
         rebase(p.f_albedo[c], base);
         rebase(p.denoised[c], base);
-        rebase(p.sqrt_var_mean[c], base);
         rebase(p.sqrt_var_stable[c], base);
         if (c == 0) rebase(p.win, base);
         rebase(n.n_normal[c], base);

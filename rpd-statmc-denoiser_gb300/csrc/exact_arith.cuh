@@ -80,30 +80,4 @@ __device__ __forceinline__ bool quotient_to_float(uint64_t am, int ae, uint64_t 
     return true;
 }
 
-
-// a + b for nonnegative normalised operands (b may be 0)
-__device__ __forceinline__ XD xd_add(XD a, XD b) {
-    if (b.m == 0ull) return a;
-    if (a.m == 0ull) return b;
-    if (a.e < b.e) {
-        const XD t = a;
-        a = b;
-        b = t;
-    }
-    const int d = a.e - b.e;
-    if (d >= 54) return a;  // b is below half an ulp of a
-    const uint64_t A = a.m << 10;
-    uint64_t B = b.m << 10;
-    if (d) B = (B >> d) | ((B & ((1ull << d) - 1ull)) ? 1ull : 0ull);  // bits shifted out: sticky
-    const uint64_t S = A + B;                                        // below 2^64
-    const int k = (S >> 63) ? 11 : 10;
-    return xd_round(S >> k, S & ((1ull << k) - 1ull), 1ull << (k - 1), a.e - 10 + k);
-}
-
-// the parts of a positive normal double
-__device__ __forceinline__ XD xd_of_double(double v) {
-    const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(v));
-    return XD{(b & ((1ull << 52) - 1ull)) | (1ull << 52), int((b >> 52) & 0x7ffull) - 1075};
-}
-
 }  // namespace rpd

@@ -1,8 +1,8 @@
 // statmc_denoise (main.cpp:957-1162): the per-channel square-root-domain Welch
 // compatibility window with the RPD relaxation.
 //
-//   k_sqrt_var_mean    sqrt-domain variance of the mean, floored at EPS_SMALL (972-980)
-//   k_sqrt_var_stable  max with its 3x3 inverse-distance average (981-990); the same pass packs
+//   k_sqrt_var_stable  sqrt-domain variance of the mean, floored at EPS_SMALL (972-980), and its
+//                      max with its 3x3 inverse-distance average (981-990); the same pass packs
 //                      every pixel's neighbour record into six float4 planes (p.win):
 //                        W_GATE (unit normal xyz, depth)      the normal / depth gates
 //                        W_ALB  (albedo xyz, 1/max(n-1, 1))   the albedo gate; 0 marks a pixel
@@ -54,7 +54,6 @@
 
 #include "rpd_internal.h"
 #include "device_math.cuh"
-#include "exact_arith.cuh"
 #include "tma.cuh"
 
 namespace rpd {
@@ -107,26 +106,65 @@ __device__ __forceinline__ float pixel_variance(float m2, int n) {  // core/stat
     return (n > 1) ? m2 / float(n - 1) : 0.0f;
 }
 
-__global__ void k_sqrt_var_mean(PixelPlanes p, int64_t np) {
-    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= np) return;
-    const int n = p.n[i];
-    for (int c = 0; c < 3; ++c) {
-        const float var = (n <= 1) ? 0.0f : p.sqrt_sq[c][i] / float(n - 1);
-        p.sqrt_var_mean[c][i] = fmaxs(var / float(imaxs(1, n)), 1e-8f);
-    }
+// The sqrt-domain variance of the mean of channel c, floored at EPS_SMALL (main.cpp:972-980).
+__device__ __forceinline__ float sqrt_var_of_mean(const PixelPlanes& p, int c, int64_t i, int n) {
+    const float var = (n <= 1) ? 0.0f : p.sqrt_sq[c][i] / float(n - 1);
+    return fmaxs(var / float(imaxs(1, n)), 1e-8f);
 }
 
-// sample_vec3_local_average (main.cpp:170-184) of the sqrt variance of the mean, then the
-// component max (981-990). The reference accumulates in double: v * weight with weights 1/3
-// (corners, 1.0 / 3.0 rounded), 1/2 and 1 (both exact), nine additions in (dy, dx) order, one
-// division by the summed weights. A 32 x 8 block stages, per pixel of its (clamped) 34 x 10 halo,
-// the three products each channel can need (v, v * 0.5, v * (1.0 / 3.0)) in double once. Of a
-// pixel's three channels, the first's nine additions run exactly in integer instructions
-// (exact_arith.cuh) and the others' as double additions, so the integer and double pipes share
-// the work; each quotient is rounded to float through a single-precision estimate and an exact
-// integer remainder (the double division only where that cannot decide). The values are
-// positive: sqrt_var_mean is floored at 1e-8.
+// a + b as the rounded sum and its exact error (Knuth's TwoSum)
+__device__ __forceinline__ float two_sum(float a, float b, float& err) {
+    const float s = a + b, t = s - a;
+    err = (a - (s - t)) + (b - t);
+    return s;
+}
+
+// The constants of the 3x3 average as pairs of floats: the corner weight 1.0 / 3.0 and the inverse of the
+// summed weights, each the double's value to 2^-48.
+struct AverageConsts {
+    double weight_sum;
+    float third_h, third_l, inv_h, inv_l;
+};
+
+// sample_vec3_local_average (main.cpp:170-184) of nine values around t, `tw` floats a row. The
+// reference accumulates in double: v * weight with weights 1/3 (corners, 1.0 / 3.0 rounded), 1/2 and 1,
+// nine additions in (dy, dx) order, one division by the summed weights, and a rounding to float. Its
+// double is within 2^-48 of the exact average of the nine floats, the sums of exact-error pairs below
+// within 2^-44: where they round to the same float with 2^-40 added or taken away, that float is the
+// reference's and `decided`. Elsewhere (infinities, NaN, and ties: the average is a sum of floats over 26, so
+// of values of like size one in 60 lies halfway between two floats) reference_average decides.
+__device__ __forceinline__ float local_average(const float* t, int tw, const AverageConsts& k, bool& decided) {
+    float e0, e1, e2, e3, e4, e5, e6, e7;
+    const float c0 = two_sum(t[-tw - 1], t[-tw + 1], e0), c1 = two_sum(t[tw - 1], t[tw + 1], e1);
+    const float ch = two_sum(c0, c1, e2), cl = (e0 + e1) + e2;
+    const float d0 = two_sum(t[-tw], t[tw], e3), d1 = two_sum(t[-1], t[1], e4);
+    const float dh = two_sum(d0, d1, e5), dl = (e3 + e4) + e5;
+    const float ph = ch * k.third_h;
+    const float pl = __fmaf_rn(ch, k.third_h, -ph) + __fmaf_rn(ch, k.third_l, cl * k.third_h);
+    const float s = two_sum(ph, 0.5f * dh, e6), sum = two_sum(s, t[0], e7);
+    const float suml = ((e6 + e7) + pl) + 0.5f * dl;
+    const float q = sum * k.inv_h;
+    const float ql = __fmaf_rn(sum, k.inv_h, -q) + __fmaf_rn(sum, k.inv_l, suml * k.inv_h);
+    const float up = q + __fmaf_rn(q, 9.094947e-13f, ql), down = q + __fmaf_rn(q, -9.094947e-13f, ql);  // 2^-40
+    decided = up == down && up < INFINITY;
+    return up;
+}
+
+// The same average by the reference's double operations.
+__device__ __forceinline__ float reference_average(const float* t, int tw, double weight_sum) {
+    const double third = 1.0 / (1.0 + 2.0);
+    double a = double(t[-tw - 1]) * third;
+    a += double(t[-tw]) * 0.5;
+    a += double(t[-tw + 1]) * third;
+    a += double(t[-1]) * 0.5;
+    a += double(t[0]);
+    a += double(t[1]) * 0.5;
+    a += double(t[tw - 1]) * third;
+    a += double(t[tw]) * 0.5;
+    a += double(t[tw + 1]) * third;
+    return float(a / weight_sum);
+}
+
 // 1 / max(n - 1, 1) of a pixel with one sample, one ulp above 1 to tell it from two samples: the
 // degrees of freedom n_i + n_j - 2 of a vanishing denominator need n (count_minus_one).
 constexpr float kSingleRp = 1.00000012f;
@@ -136,9 +174,10 @@ enum WinPlane { W_GATE = 0, W_ALB, W_SM, W_SV, W_RPD, W_CM, W_COUNT };
 // The neighbour record of pixel i (the planes of p.win) and the window's debug planes
 // (main.cpp:1010-1023). Records of pixels without a primary hit are zero but for W_CM, which
 // holds what the window writes for them (main.cpp:1001-1006): the colour mean and the
-// unclamped variance over n.
-__device__ __forceinline__ void pack_window_record(const PixelPlanes& p, int64_t np, int64_t i, const float sv[3],
-                                                   float var2_max) {
+// unclamped variance over n. W_SV waits for the stabilised variances: `rpd5` gets its fourth entry; false
+// for a pixel without a hit.
+__device__ __forceinline__ bool pack_window_record(const PixelPlanes& p, int64_t np, int64_t i, float var2_max,
+                                                   float& rpd5) {
     float4* win = p.win;
     const int n_raw = p.n[i];
     const float m2 = p.square_diff[i];
@@ -147,7 +186,7 @@ __device__ __forceinline__ void pack_window_record(const PixelPlanes& p, int64_t
         const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         for (int k = W_GATE; k < W_CM; ++k) win[k * np + i] = z;
         win[W_CM * np + i] = make_float4(cm.x, cm.y, cm.z, pixel_variance(m2, n_raw) / float(imaxs(1, n_raw)));
-        return;
+        return false;
     }
     float var = pixel_variance(m2, n_raw);
     if (!isfinite(var)) var = 1e-8f;
@@ -161,59 +200,69 @@ __device__ __forceinline__ void pack_window_record(const PixelPlanes& p, int64_t
     win[W_GATE * np + i] = make_float4(p.f_normal[0][i], p.f_normal[1][i], p.f_normal[2][i], p.f_depth[i]);
     win[W_ALB * np + i] = make_float4(p.f_albedo[0][i], p.f_albedo[1][i], p.f_albedo[2][i], rp);
     win[W_SM * np + i] = make_float4(p.sqrt_mean[0][i], p.sqrt_mean[1][i], p.sqrt_mean[2][i], p.rpd[4][i]);
-    win[W_SV * np + i] = make_float4(sv[0], sv[1], sv[2], p.rpd[5][i]);
+    rpd5 = p.rpd[5][i];
     win[W_RPD * np + i] = make_float4(p.rpd[0][i], p.rpd[1][i], p.rpd[2][i], p.rpd[3][i]);
     win[W_CM * np + i] = make_float4(cm.x, cm.y, cm.z, vm);
+    return true;
 }
 
+// max of the sqrt variance of the mean with its 3x3 average (main.cpp:981-990) and the window's
+// records. A block stages its pixels' values and a halo of one, clamped into the image.
+// Bound by memory latency: about 210 bytes per pixel read and written in three phases (65 us at the
+// copy rate for 1920x1080). 200 us with the values in a pass of their own and the double additions in integer
+// instructions; 179 us with the pairs of singles, 119 with the ties queued, 111 with the other records before
+// the averages.
 constexpr int kSvTx = 32, kSvTy = 8;
-__global__ void __launch_bounds__(kSvTx * kSvTy) k_sqrt_var_stable(PixelPlanes p, int w, int h, double weight_sum,
+__global__ void __launch_bounds__(kSvTx * kSvTy) k_sqrt_var_stable(PixelPlanes p, int w, int h, AverageConsts k,
                                                                   float var2_max) {
-    __shared__ double tile[3][3][(kSvTy + 2) * (kSvTx + 2)];  // [channel][v, v/2, v/3][pixel]
-    const int tw = kSvTx + 2, tn = (kSvTy + 2) * (kSvTx + 2);
+    constexpr int tw = kSvTx + 2, tn = (kSvTy + 2) * (kSvTx + 2);
+    __shared__ float tile[3][tn];
+    // the undecided averages (tile entry * 3 + channel), and their values by the threads in turn: done where
+    // they turn up, nearly every warp would wait for a lane's double operations
+    __shared__ int queue[kSvTx * kSvTy * 3], s_queued;
     const int x0 = blockIdx.x * kSvTx, y0 = blockIdx.y * kSvTy;
     const int tid = threadIdx.y * kSvTx + threadIdx.x;
-    const double third = 1.0 / (1.0 + 2.0);
+    if (tid == 0) s_queued = 0;
     for (int e = tid; e < tn; e += kSvTx * kSvTy) {
         const int gx = iclamps(x0 - 1 + e % tw, 0, w - 1), gy = iclamps(y0 - 1 + e / tw, 0, h - 1);
         const int64_t q = int64_t(gy) * w + gx;
-        for (int c = 0; c < 3; ++c) {
-            const double v = double(p.sqrt_var_mean[c][q]);
-            tile[c][0][e] = v;
-            tile[c][1][e] = v * 0.5;
-            tile[c][2][e] = v * third;
+        const int n = p.n[q];
+        for (int c = 0; c < 3; ++c) tile[c][e] = sqrt_var_of_mean(p, c, q, n);
+    }
+    const int x = x0 + threadIdx.x, y = y0 + threadIdx.y;
+    const bool mine = x < w && y < h;
+    const int64_t i = int64_t(y) * w + x;
+    // the records' other fields while the block's values arrive
+    float rpd5 = 0.0f;
+    const bool hit = mine && pack_window_record(p, int64_t(w) * h, i, var2_max, rpd5);
+    __syncthreads();
+    const int e = (threadIdx.y + 1) * tw + threadIdx.x + 1;
+    float sv[3];
+    int slot[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        bool decided;
+        const float avg = local_average(&tile[c][e], tw, k, decided);
+        sv[c] = fmaxs(tile[c][e], avg);
+        slot[c] = -1;
+        if (mine && !decided) {
+            slot[c] = atomicAdd(&s_queued, 1);
+            queue[slot[c]] = 3 * e + c;
         }
     }
     __syncthreads();
-    const int x = x0 + threadIdx.x, y = y0 + threadIdx.y;
-    if (x >= w || y >= h) return;
-    const int64_t i = int64_t(y) * w + x;
-    const int e = (threadIdx.y + 1) * tw + threadIdx.x + 1;
-    const XD wsum = xd_of_double(weight_sum);
-    float sv[3];
+    for (int q = tid; q < s_queued; q += kSvTx * kSvTy) {
+        const float* t = &tile[queue[q] % 3][queue[q] / 3];
+        queue[q] = __float_as_int(fmaxs(*t, reference_average(t, tw, k.weight_sum)));
+    }
+    __syncthreads();
+    if (!mine) return;
+#pragma unroll
     for (int c = 0; c < 3; ++c) {
-        const double* t1 = tile[c][0];
-        const double* th = tile[c][1];
-        const double* tt = tile[c][2];
-        // the reference's nine double additions in its order, each rounded as the double-precision
-        // add rounds it, in integer arithmetic (GB300's double-precision pipe is the scarce one)
-        XD x = xd_of_double(tt[e - tw - 1]);
-        x = xd_add(x, xd_of_double(th[e - tw]));
-        x = xd_add(x, xd_of_double(tt[e - tw + 1]));
-        x = xd_add(x, xd_of_double(th[e - 1]));
-        x = xd_add(x, xd_of_double(t1[e]));
-        x = xd_add(x, xd_of_double(th[e + 1]));
-        x = xd_add(x, xd_of_double(tt[e + tw - 1]));
-        x = xd_add(x, xd_of_double(th[e + tw]));
-        x = xd_add(x, xd_of_double(tt[e + tw + 1]));
-        const double a = xd_to_double(x);
-        const XD ax = xd_of_double(a);
-        float q;
-        if (!quotient_to_float(ax.m, ax.e, wsum.m, wsum.e, q)) q = float(a / weight_sum);
-        sv[c] = fmaxs(p.sqrt_var_mean[c][i], q);
+        if (slot[c] >= 0) sv[c] = __int_as_float(queue[slot[c]]);
         p.sqrt_var_stable[c][i] = sv[c];
     }
-    pack_window_record(p, int64_t(w) * h, i, sv, var2_max);
+    if (hit) p.win[W_SV * (int64_t(w) * h) + i] = make_float4(sv[0], sv[1], sv[2], rpd5);
 }
 
 struct StatmcParams {
@@ -955,13 +1004,17 @@ cudaError_t launch_statmc(Job& j) {
     const float var2_max = j.cfg.color_sigma_max * j.cfg.color_sigma_max;
     {
         KernelScope ks(j, RPD_KERNEL_SQRT_VARIANCE);
-        k_sqrt_var_mean<<<grid_for(np, 256), 256, 0, j.stream>>>(j.p, np);
         // the summed weights of the 3x3 average, accumulated as the reference accumulates them
-        double weight_sum = 0.0;
+        AverageConsts k{};
         for (int dy = -1; dy <= 1; ++dy)
-            for (int dx = -1; dx <= 1; ++dx) weight_sum += 1.0 / (1.0 + double(dx * dx + dy * dy));
+            for (int dx = -1; dx <= 1; ++dx) k.weight_sum += 1.0 / (1.0 + double(dx * dx + dy * dy));
+        const double third = 1.0 / (1.0 + 2.0), inv = 1.0 / k.weight_sum;
+        k.third_h = float(third);
+        k.third_l = float(third - double(k.third_h));
+        k.inv_h = float(inv);
+        k.inv_l = float(inv - double(k.inv_h));
         const dim3 sgrid((j.g.w + kSvTx - 1) / kSvTx, (j.g.h + kSvTy - 1) / kSvTy);
-        k_sqrt_var_stable<<<sgrid, dim3(kSvTx, kSvTy), 0, j.stream>>>(j.p, j.g.w, j.g.h, weight_sum, var2_max);
+        k_sqrt_var_stable<<<sgrid, dim3(kSvTx, kSvTy), 0, j.stream>>>(j.p, j.g.w, j.g.h, k, var2_max);
     }
     KernelScope ks(j, RPD_KERNEL_STATMC_WINDOW);
     StatmcParams prm{};
@@ -1036,7 +1089,7 @@ cudaError_t launch_statmc(Job& j) {
             j.launches += 1;
         }
     }
-    j.launches += 3;
+    j.launches += 2;
     return e;
 }
 

@@ -73,7 +73,6 @@ struct PixelPlanes {
     float* var_eff;
     float* var_ratio;
     // statmc scratch: stabilised sqrt variance of the mean (main.cpp:972-990)
-    float* sqrt_var_mean[3];
     float* sqrt_var_stable[3];
     // statmc_denoise's packed neighbour records: six float4 planes of W*H, one after the other
     // (record k of pixel i at win[k * W*H + i]), written with the stabilised sqrt variance and
