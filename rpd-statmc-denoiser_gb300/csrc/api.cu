@@ -778,7 +778,7 @@ static int push_host_banded(Job* j, const std::vector<HostPlane>& planes, const 
         const Band& b = bands[bi];
         RPD_CUDA(cudaStreamWaitEvent(j->stream, j->band_copied[bi], 0));
         if (counts) RPD_CUDA(launch_offsets_scan(*j, dcounts[bi], b.p1 - b.p0));
-        else RPD_CUDA(launch_offsets_uniform(*j, b.p1 - b.p0, spp));
+        else if (spp == 0) RPD_CUDA(launch_offsets_uniform(*j, b.p1 - b.p0, spp));
         const int st = push_tail(j, dev[bi], first + b.p0, b.p1 - b.p0, spp, counts ? counts + b.p0 : nullptr,
                                  RPD_MEM_HOST, b.k1 - b.k0);
         if (st != RPD_OK) return st;
@@ -877,7 +877,7 @@ int rpd_job_push_samples(rpd_job* job, const rpd_sample_soa* s, int64_t first, i
         d.flags = s->flags;
         d.category = s->category;
         if (counts) RPD_CUDA(launch_offsets_scan(*j, counts, count));
-        else RPD_CUDA(launch_offsets_uniform(*j, count, spp));
+        else if (spp == 0) RPD_CUDA(launch_offsets_uniform(*j, count, spp));
     }
     if (!d.normal[0] || !d.normal[1] || !d.normal[2] || !d.depth ||
         (!d.albedo[0] && !d.pixel_albedo[0]))
@@ -885,8 +885,8 @@ int rpd_job_push_samples(rpd_job* job, const rpd_sample_soa* s, int64_t first, i
     return push_tail(j, d, first, count, spp, counts, where, total);
 }
 
-// The part of a push shared by both sample formats: the offsets are computed, d points at
-// device planes. Runs the statistics pass and the grid pass.
+// The part of a push shared by both sample formats: the offsets of per-pixel counts are computed (a uniform
+// push's are multiples of spp, see sample_offset), d points at device planes. Runs the statistics pass and the grid pass.
 int rpd_job_push_samples16(rpd_job* job, const rpd_sample_soa16* s, int64_t first, int64_t count, int32_t spp,
                            const int32_t* counts, rpd_memory where) {
     Job* j = reinterpret_cast<Job*>(job);
@@ -970,7 +970,7 @@ int rpd_job_push_samples16(rpd_job* job, const rpd_sample_soa16* s, int64_t firs
         d.flags = s->flags;
         d.category = s->category;
         if (counts) RPD_CUDA(launch_offsets_scan(*j, counts, count));
-        else RPD_CUDA(launch_offsets_uniform(*j, count, spp));
+        else if (spp == 0) RPD_CUDA(launch_offsets_uniform(*j, count, spp));
     }
     return push_tail(j, d, first, count, spp, counts, where, total);
 }
@@ -1063,7 +1063,7 @@ static int push_tail(Job* j, DeviceSamples& d, int64_t first, int64_t count, int
         const int64_t* d_max = (counts && max_count == INT32_MAX) ? offsets_count_max(*j, count) : nullptr;
         RPD_CUDA(launch_grid_fast(*j, d, first, count, gp, counts ? 0 : spp, max_count, nsamp, d_max));
     }
-    else if (rpd) RPD_CUDA(launch_accumulate_grid(*j, d, first, count));
+    else if (rpd) RPD_CUDA(launch_accumulate_grid(*j, d, first, count, counts ? 0 : spp));
     j->pass_open = true;
     j->have_samples = true;
     j->features_valid = false;
@@ -1098,6 +1098,7 @@ int rpd_recompute_sensitivity(rpd_job* job) {
         int st = ensure_features(*j);
         if (st != RPD_OK) return st;
         RPD_CUDA(launch_sensitivity(*j));
+        j->cache_valid = true;
     }
     return ensure_cache(*j);
 }
@@ -1111,11 +1112,6 @@ int rpd_statmc_denoise(rpd_job* job) {
     if (st != RPD_OK) return st;
     st = ensure_cache(*j);
     if (st != RPD_OK) return st;
-    // the window's recheck counters and its slow-pixel list describe the last call
-    RPD_CUDA(cudaMemsetAsync(j->p.counters + RPD_COUNTER_WINDOW_PAIR_RECHECKS, 0, 2 * sizeof(unsigned long long),
-                             j->stream));
-    RPD_CUDA(cudaMemsetAsync(j->p.counters + RPD_COUNTER_WINDOW_SLOW_PIXELS, 0, sizeof(unsigned long long),
-                             j->stream));
     RPD_CUDA(launch_statmc(*j));
     return RPD_OK;
 }
@@ -1844,7 +1840,7 @@ int push_device_async(Job& j, const DeviceSamples& d, int64_t first, int64_t cou
     StageTimer timer(j, RPD_STAGE_ACCUMULATE);
     if (!offsets_ready) {
         if (counts) RPD_CUDA(launch_offsets_scan(j, counts, count));
-        else RPD_CUDA(launch_offsets_uniform(j, count, spp));
+        else if (spp == 0) RPD_CUDA(launch_offsets_uniform(j, count, spp));
     }
     DeviceSamples dd = d;
     return push_tail(&j, dd, first, count, spp, counts, RPD_MEM_DEVICE,

@@ -57,6 +57,11 @@ __device__ __forceinline__ float relative_depth_delta(float a, float b) {
     return fabsf(a - b) / m;
 }
 
+// The first sample of a push's pixel i: spp > 0 for a uniform push, else the scanned counts.
+__device__ __forceinline__ int64_t sample_offset(const int64_t* offsets, int spp, int64_t i) {
+    return spp > 0 ? i * spp : offsets[i];
+}
+
 __device__ __forceinline__ bool finite3(float a, float b, float c) {
     return isfinite(a) && isfinite(b) && isfinite(c);
 }

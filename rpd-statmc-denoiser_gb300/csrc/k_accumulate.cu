@@ -602,11 +602,11 @@ __device__ __forceinline__ void store_prep(const GridPrep& gp, int64_t k, const 
 // planes are rpd_sample_soa16's (s.c16), decoded to float here; WIDE reads them 8 samples (16
 // bytes) per load. PART: what the thread keeps of its pixel.
 template <bool VEC4, bool COMPACT, bool WIDE, Part PART>
-__device__ __forceinline__ void accumulate_pixel(const PixelPlanes& p, const DeviceSamples& s, const int64_t* offsets,
+__device__ __forceinline__ void accumulate_pixel(const PixelPlanes& p, const DeviceSamples& s, const int64_t* offsets, int spp,
                                                  int64_t local, int64_t first, const GridPrep& gp, int fresh) {
     constexpr bool colour = PART != kLuminance, lumi = PART != kColour;
     const int64_t idx = first + local;
-    const int64_t k0 = offsets[local], k1 = offsets[local + 1];
+    const int64_t k0 = sample_offset(offsets, spp, local), k1 = sample_offset(offsets, spp, local + 1);
     const bool prep = gp.lum != nullptr;
     const bool has_pu = COMPACT ? s.c16.pixel_u[0] != nullptr : s.pixel_u[0] != nullptr;
     const bool has_lu = COMPACT ? s.c16.lens_u[0] != nullptr : s.lens_u[0] != nullptr;
@@ -777,16 +777,16 @@ __device__ __forceinline__ void accumulate_pixel(const PixelPlanes& p, const Dev
 // per load do not: 24 split warps read more lines at a time than L1 holds (1920x1080x16 0.64 -> 0.72 ms).
 template <bool VEC4, bool COMPACT, bool WIDE, int MINB, bool SPLIT>
 __global__ void __launch_bounds__(128, MINB) k_accumulate_pixels(PixelPlanes p, DeviceSamples s, const int64_t* offsets,
-                                                                 int64_t first, int64_t count, GridPrep gp, int fresh) {
+                                                                 int spp, int64_t first, int64_t count, GridPrep gp, int fresh) {
     if constexpr (SPLIT) {
         const int64_t local = int64_t(blockIdx.x) * 64 + (threadIdx.x & 63);
         if (local >= count) return;
-        if (threadIdx.x < 64) accumulate_pixel<VEC4, COMPACT, WIDE, kLuminance>(p, s, offsets, local, first, gp, fresh);
-        else accumulate_pixel<VEC4, COMPACT, WIDE, kColour>(p, s, offsets, local, first, gp, fresh);
+        if (threadIdx.x < 64) accumulate_pixel<VEC4, COMPACT, WIDE, kLuminance>(p, s, offsets, spp, local, first, gp, fresh);
+        else accumulate_pixel<VEC4, COMPACT, WIDE, kColour>(p, s, offsets, spp, local, first, gp, fresh);
     } else {
         const int64_t local = int64_t(blockIdx.x) * 128 + threadIdx.x;
         if (local >= count) return;
-        accumulate_pixel<VEC4, COMPACT, WIDE, kWhole>(p, s, offsets, local, first, gp, fresh);
+        accumulate_pixel<VEC4, COMPACT, WIDE, kWhole>(p, s, offsets, spp, local, first, gp, fresh);
     }
 }
 
@@ -1228,8 +1228,8 @@ __global__ void __launch_bounds__(128) k_grid_ordered(Geometry g, double* pass_g
             for (int e = 0; e < ne; ++e) any |= we[e] > 1e-8f;
             if (!any) continue;
             const int64_t local = idx - first;
-            const int64_t k0 = offsets ? offsets[local] : local * spp;
-            const int64_t k1 = offsets ? offsets[local + 1] : (local + 1) * spp;
+            const int64_t k0 = sample_offset(offsets, spp, local);
+            const int64_t k1 = sample_offset(offsets, spp, local + 1);
             const float support_left = float(nx * g.step) - half_support;
             const float support_top = float(ny * g.step) - half_support;
             for (int64_t k = k0; k < k1; ++k) {
@@ -1437,12 +1437,14 @@ const int64_t* offsets_count_max(const Job& j, int64_t count) {
 // which keeps more of the sample sectors a thread reads again a step later (3 % more throughput
 // on the served stream, where other requests' kernels share the SMs).
 template <bool VEC4, bool COMPACT, bool WIDE, int MINB, bool SPLIT>
-cudaError_t run_accumulate(Job& j, const DeviceSamples& s, int64_t first, int64_t count, const GridPrep& gp, int fresh) {
-    const cudaError_t e = cudaFuncSetAttribute(k_accumulate_pixels<VEC4, COMPACT, WIDE, MINB, SPLIT>,
-                                               cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxL1);
+cudaError_t run_accumulate(Job& j, const DeviceSamples& s, int32_t spp, int64_t first, int64_t count, const GridPrep& gp, int fresh) {
+    static FuncAttribute carveout;
+    const cudaError_t e = carveout.at_least(reinterpret_cast<const void*>(&k_accumulate_pixels<VEC4, COMPACT, WIDE, MINB, SPLIT>),
+                                            cudaFuncAttributePreferredSharedMemoryCarveout, j.ctx->device,
+                                            cudaSharedmemCarveoutMaxL1);
     if (e != cudaSuccess) return e;
     k_accumulate_pixels<VEC4, COMPACT, WIDE, MINB, SPLIT><<<grid_for(count, SPLIT ? 64 : 128), 128, 0, j.stream>>>(
-        j.p, s, j.offsets, first, count, gp, fresh);
+        j.p, s, j.offsets, spp, first, count, gp, fresh);
     return cudaSuccess;
 }
 
@@ -1464,8 +1466,9 @@ cudaError_t run_rows(Job& j, const DeviceSamples& s, int64_t first, int64_t coun
     for (int* off : {&ra.albedo, &ra.pu, &ra.lu, &ra.bu, &ra.li, &ra.eu})
         if (*off >= 0) *off *= kRowPixels * RB;
     const int smem = 1024 + 2 * ((ra.planes * kRowPixels * RB + 1023) & ~1023);
-    const cudaError_t e =
-        cudaFuncSetAttribute(k_accumulate_rows<COMPACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    static FuncAttribute limit;
+    const cudaError_t e = limit.at_least(reinterpret_cast<const void*>(&k_accumulate_rows<COMPACT>),
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, j.ctx->device, smem);
     if (e != cudaSuccess) return e;
     k_accumulate_rows<COMPACT><<<grid_for(count, kRowPixels), kRowRoles * 32, smem, j.stream>>>(j.p, s, spp, first, count, gp, fresh, ra);
     return cudaGetLastError();
@@ -1579,30 +1582,30 @@ cudaError_t launch_accumulate_pixels(Job& j, const DeviceSamples& s, int64_t fir
                    (!h.brdf_u[0] || aligned(h.brdf_u[c], 16)) && (!h.light_u[0] || aligned(h.light_u[c], 16)) &&
                    (!h.env_u[0] || aligned(h.env_u[c], 16));
         if (wide)
-            e = run_accumulate<true, true, true, 1, false>(j, s, first, count, gp, fresh);
+            e = run_accumulate<true, true, true, 1, false>(j, s, spp, first, count, gp, fresh);
         else if (vec4 && many)
-            e = run_accumulate<true, true, false, 1, false>(j, s, first, count, gp, fresh);
+            e = run_accumulate<true, true, false, 1, false>(j, s, spp, first, count, gp, fresh);
         else if (vec4)
-            e = run_accumulate<true, true, false, 4, false>(j, s, first, count, gp, fresh);
+            e = run_accumulate<true, true, false, 4, false>(j, s, spp, first, count, gp, fresh);
         else
-            e = run_accumulate<false, true, false, 8, true>(j, s, first, count, gp, fresh);
+            e = run_accumulate<false, true, false, 8, true>(j, s, spp, first, count, gp, fresh);
     } else {
         if (vec4 && many)
-            e = run_accumulate<true, false, false, 1, false>(j, s, first, count, gp, fresh);
+            e = run_accumulate<true, false, false, 1, false>(j, s, spp, first, count, gp, fresh);
         else if (vec4)
-            e = run_accumulate<true, false, false, 3, false>(j, s, first, count, gp, fresh);
+            e = run_accumulate<true, false, false, 3, false>(j, s, spp, first, count, gp, fresh);
         else
-            e = run_accumulate<false, false, false, 8, true>(j, s, first, count, gp, fresh);
+            e = run_accumulate<false, false, false, 8, true>(j, s, spp, first, count, gp, fresh);
     }
     if (e != cudaSuccess) return e;
     j.launches += 1;
     return cudaGetLastError();
 }
 
-cudaError_t launch_accumulate_grid(Job& j, const DeviceSamples& s, int64_t first, int64_t count) {
+cudaError_t launch_accumulate_grid(Job& j, const DeviceSamples& s, int64_t first, int64_t count, int32_t spp) {
     KernelScope ks(j, RPD_KERNEL_GRID);
     const int64_t threads = j.g.nn * kDeps;
-    k_grid_ordered<<<grid_for(threads, 128), 128, 0, j.stream>>>(j.g, j.n.pass_grid, s, j.offsets, 0, first, count);
+    k_grid_ordered<<<grid_for(threads, 128), 128, 0, j.stream>>>(j.g, j.n.pass_grid, s, j.offsets, spp, first, count);
     j.pass_indirect = true;
     j.launches += 1;
     return cudaGetLastError();

@@ -354,8 +354,8 @@ __global__ void __launch_bounds__(kGroups * 32) k_grid_fast(GridParams gpar, flo
             const float fx = float(__shfl_sync(0xffffffffu, x, src));
             const float fy = float(__shfl_sync(0xffffffffu, y, src));
             const int64_t local = pidx - gpar.first;
-            const int64_t kend = offsets[local + 1];
-            for (int64_t k = offsets[local] + lane; k < kend; k += 32) {
+            const int64_t kend = sample_offset(offsets, gpar.spp, local + 1);
+            for (int64_t k = sample_offset(offsets, gpar.spp, local) + lane; k < kend; k += 32) {
                 const uint32_t key = gp.key[k];
                 if (key & absent) continue;
                 const float yv = gp.lum[k];
@@ -434,8 +434,8 @@ __global__ void __launch_bounds__(32) k_grid_screen(GridParams gpar, float2* pas
                            bool pmixed, Totals& ts) {
         const float fx = float(px), fy = float(py);
         const int64_t local = pidx - gpar.first;
-        const int64_t kend = offsets[local + 1];
-        for (int64_t k = offsets[local] + lane; k < kend; k += 32) {
+        const int64_t kend = sample_offset(offsets, gpar.spp, local + 1);
+        for (int64_t k = sample_offset(offsets, gpar.spp, local) + lane; k < kend; k += 32) {
             const uint32_t key = gp.key[k];
             if (key & absent) continue;
             const float yv = gp.lum[k];
@@ -1044,8 +1044,8 @@ __device__ void odd_node(const GridParams& gpar, float2* grid, const DeviceSampl
         pixel(i, x, y, idx);
         if (is_deviant(idx)) continue;
         const int b0 = nominal_bin(x, y);
-        const int64_t local = idx - gpar.first, kend = offsets[local + 1];
-        for (int64_t k = offsets[local] + lane; k < kend; k += 32) {
+        const int64_t local = idx - gpar.first, kend = sample_offset(offsets, gpar.spp, local + 1);
+        for (int64_t k = sample_offset(offsets, gpar.spp, local) + lane; k < kend; k += 32) {
             const uint32_t key = gp.key[k];
             if (!(key & key_absent_bit(0)) && exact_bin(x, y, k) != b0) set.add(pattern_of(key));
         }
@@ -1062,8 +1062,8 @@ __device__ void odd_node(const GridParams& gpar, float2* grid, const DeviceSampl
             if (is_deviant(idx)) continue;
             const int b0 = nominal_bin(x, y);
             const float w = weight(x, y);
-            const int64_t local = idx - gpar.first, kend = offsets[local + 1];
-            for (int64_t k = offsets[local] + lane; k < kend; k += 32) {
+            const int64_t local = idx - gpar.first, kend = sample_offset(offsets, gpar.spp, local + 1);
+            for (int64_t k = sample_offset(offsets, gpar.spp, local) + lane; k < kend; k += 32) {
                 const uint32_t key = gp.key[k];
                 if ((key & key_absent_bit(0)) || pattern_of(key) != P) continue;
                 const int b = exact_bin(x, y, k);
@@ -1103,8 +1103,8 @@ __device__ void odd_node(const GridParams& gpar, float2* grid, const DeviceSampl
                 add_class(tx, w, cs[0], cs[1], cs[2], cs[3], cs[4]);
                 if (!mixed) add_class(ts, w, cs[0], cs[1], cs[2], cs[3], cs[4]);
             }
-            const int64_t local = idx - gpar.first, kend = offsets[local + 1];
-            for (int64_t k = offsets[local] + lane; k < kend; k += 32) {
+            const int64_t local = idx - gpar.first, kend = sample_offset(offsets, gpar.spp, local + 1);
+            for (int64_t k = sample_offset(offsets, gpar.spp, local) + lane; k < kend; k += 32) {
                 const uint32_t key = gp.key[k];
                 if (key & absent) continue;
                 const float yv = gp.lum[k];
@@ -1528,8 +1528,8 @@ __global__ void __launch_bounds__(RW * DS * 32) k_grid_random(RandParams rp, flo
             p0 = p0 < gpar.first ? gpar.first : p0;
             p1 = p1 > gpar.first + gpar.count ? gpar.first + gpar.count : p1;
             if (ay > 0.0f && p0 < p1) {
-                const int64_t k0 = offsets[p0 - gpar.first];
-                const int len = int(offsets[p1 - gpar.first] - k0);
+                const int64_t k0 = sample_offset(offsets, gpar.spp, p0 - gpar.first);
+                const int len = int(sample_offset(offsets, gpar.spp, p1 - gpar.first) - k0);
                 n = MODE == kWalkColumnQuads ? (len > 0 ? int(((k0 + len - 1) >> 2) - (k0 >> 2) + 1) : 0) : len;
                 rt->k0[lane] = k0;
                 rt->len[lane] = len;
@@ -1987,8 +1987,9 @@ cudaError_t launch_random_vec(Job& j, const RandParams& rp, const GridPrep& gp) 
     constexpr int NW = RW * DS;
     const size_t smem = size_t(NW) * RandLayout<WB, DS>::kWarpBytes + size_t(NW) * sizeof(RowTable) +
                         size_t(rp.cols) * sizeof(float);
-    cudaError_t e = cudaFuncSetAttribute(k_grid_random<WB, RW, DS, MODE, DIMS>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    static FuncAttribute limit;
+    const cudaError_t e = limit.at_least(reinterpret_cast<const void*>(&k_grid_random<WB, RW, DS, MODE, DIMS>),
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, j.ctx->device, int64_t(smem));
     if (e != cudaSuccess) return e;
     const unsigned nblocks = unsigned(rp.gp.count_nodes);
     k_grid_random<WB, RW, DS, MODE, DIMS><<<nblocks, NW * 32, smem, j.stream>>>(rp, rp.target, j.offsets, gp);
@@ -2029,8 +2030,9 @@ cudaError_t launch_random_shape(Job& j, const RandParams& rp, const GridPrep& gp
 template <int NC, int RG, int U, int DIMS>
 cudaError_t launch_strips_unit(Job& j, const StripParams& sp, unsigned blocks, float2* target, const GridPrep& gp) {
     constexpr int smem = NC * RG * StripLayout<DIMS>::kWarpBytes + StripLayout<DIMS>::edge_bytes(NC);
-    const cudaError_t e = cudaFuncSetAttribute(k_grid_strips<NC, RG, U, DIMS>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    static FuncAttribute limit;
+    const cudaError_t e = limit.at_least(reinterpret_cast<const void*>(&k_grid_strips<NC, RG, U, DIMS>),
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, j.ctx->device, smem);
     if (e != cudaSuccess) return e;
     k_grid_strips<NC, RG, U, DIMS><<<blocks, NC * RG * 64, smem, j.stream>>>(sp, target, gp);
     j.launches += 1;
@@ -2171,11 +2173,15 @@ cudaError_t launch_grid_fast(Job& j, const DeviceSamples& s, int64_t first, int6
             const size_t smem = size_t(int_w ? LaneBins<true>::kSlots : LaneBins<false>::kSlots) * 32 * sizeof(float) +
                                 list_bytes;
             if (int_w) {
-                e = cudaFuncSetAttribute(k_grid_screen<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+                static FuncAttribute limit;
+                e = limit.at_least(reinterpret_cast<const void*>(&k_grid_screen<true>),
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize, j.ctx->device, int64_t(smem));
                 if (e != cudaSuccess) return e;
                 k_grid_screen<true><<<nblocks, 32, smem, j.stream>>>(gpar, target, s, j.offsets, gp);
             } else {
-                e = cudaFuncSetAttribute(k_grid_screen<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+                static FuncAttribute limit;
+                e = limit.at_least(reinterpret_cast<const void*>(&k_grid_screen<false>),
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize, j.ctx->device, int64_t(smem));
                 if (e != cudaSuccess) return e;
                 k_grid_screen<false><<<nblocks, 32, smem, j.stream>>>(gpar, target, s, j.offsets, gp);
             }

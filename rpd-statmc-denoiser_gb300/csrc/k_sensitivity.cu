@@ -418,6 +418,34 @@ __device__ __forceinline__ float tiles_lookup(const Geometry& g, const float* ti
     return lerp_std(top, bottom, ty);
 }
 
+__global__ void k_sens_zero(PixelPlanes p, int64_t np) {
+    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i >= np) return;
+    p.sens_confidence[i] = 0.0f;
+    p.sens_gradient[i] = 0.0f;
+}
+
+__constant__ int c_rpd_field[6] = {N_BRDF, N_LENS, N_LIGHT_UV, N_LIGHT_SELECT, N_ENV, N_RR};
+
+__device__ __forceinline__ void rpd_components(const Geometry& g, const NodePlanes& n, const PixelPlanes& p, int64_t i, int x,
+                                               int y, float sens_gradient) {
+    const float attenuation = 1.0f - fclamps(sens_gradient, 0.0f, 1.0f);
+    for (int c = 0; c < 6; ++c) {
+        const float v = fclamps(tiles_lookup(g, n.field[c_rpd_field[c]], x, y), 0.0f, 1.0f);
+        p.rpd[c][i] = fclamps(v * attenuation, 0.0f, 1.0f);
+    }
+}
+
+// The RPD components alone (a sensitivity of zeros, or one read back).
+__global__ void k_rpd_cache(Geometry g, NodePlanes n, PixelPlanes p) {
+    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i >= g.np) return;
+    const int y = int(i / g.w), x = int(i % g.w);
+    rpd_components(g, n, p, i, x, y, p.sens_gradient[i]);
+}
+
+// The pixels' sensitivity and, from the gradient in hand, their RPD components. Bound by instruction issue: at
+// 1920x1080 46 us and 45 us in two passes, 82 us in one.
 __global__ void k_sens_pixels(Geometry g, NodePlanes n, PixelPlanes p) {
     const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= g.np) return;
@@ -428,28 +456,9 @@ __global__ void k_sens_pixels(Geometry g, NodePlanes n, PixelPlanes p) {
     const float up = tiles_lookup(g, n.field[N_ALL], x, imaxs(0, y - 1));
     const float down = tiles_lookup(g, n.field[N_ALL], x, imins(g.h - 1, y + 1));
     const float grad = sqrtf((right - left) * (right - left) + (down - up) * (down - up));
-    p.sens_gradient[i] = fclamps(0.5f * grad, 0.0f, 1.0f);
-}
-
-__global__ void k_sens_zero(PixelPlanes p, int64_t np) {
-    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= np) return;
-    p.sens_confidence[i] = 0.0f;
-    p.sens_gradient[i] = 0.0f;
-}
-
-__constant__ int c_rpd_field[6] = {N_BRDF, N_LENS, N_LIGHT_UV, N_LIGHT_SELECT, N_ENV, N_RR};
-
-__global__ void k_rpd_cache(Geometry g, NodePlanes n, PixelPlanes p) {
-    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= g.np) return;
-    const int y = int(i / g.w), x = int(i % g.w);
-    const float gradient = fclamps(p.sens_gradient[i], 0.0f, 1.0f);
-    const float attenuation = 1.0f - gradient;
-    for (int c = 0; c < 6; ++c) {
-        const float v = fclamps(tiles_lookup(g, n.field[c_rpd_field[c]], x, y), 0.0f, 1.0f);
-        p.rpd[c][i] = fclamps(v * attenuation, 0.0f, 1.0f);
-    }
+    const float gradient = fclamps(0.5f * grad, 0.0f, 1.0f);
+    p.sens_gradient[i] = gradient;
+    rpd_components(g, n, p, i, x, y, gradient);
 }
 
 __global__ void k_expand(Geometry g, const float* tiles, float* out) {

@@ -223,6 +223,10 @@ __global__ void __launch_bounds__(kSvTx * kSvTy) k_sqrt_var_stable(PixelPlanes p
     const int x0 = blockIdx.x * kSvTx, y0 = blockIdx.y * kSvTy;
     const int tid = threadIdx.y * kSvTx + threadIdx.x;
     if (tid == 0) s_queued = 0;
+    // the window's recheck counters and its slow-pixel list describe the last call
+    if (tid == 0 && blockIdx.x == 0 && blockIdx.y == 0)
+        p.counters[RPD_COUNTER_WINDOW_PAIR_RECHECKS] = p.counters[RPD_COUNTER_WINDOW_PIXEL_RECHECKS] =
+            p.counters[RPD_COUNTER_WINDOW_SLOW_PIXELS] = 0ull;
     for (int e = tid; e < tn; e += kSvTx * kSvTy) {
         const int gx = iclamps(x0 - 1 + e % tw, 0, w - 1), gy = iclamps(y0 - 1 + e / tw, 0, h - 1);
         const int64_t q = int64_t(gy) * w + gx;
@@ -974,19 +978,11 @@ cudaError_t window_map(Job& j, int r, int by) {
 template <int RC>
 cudaError_t launch_tma(Job& j, const StatmcParams& prm, const LineTable& lt, int by) {
     const size_t smem = tile_bytes(prm.r, by);
-    // the dynamic shared memory size this instantiation allows, per device
-    static std::mutex mu;
-    static std::unordered_map<int, size_t> configured;
-    {
-        std::lock_guard<std::mutex> lock(mu);
-        size_t& allowed = configured[j.ctx->device];
-        if (smem > allowed) {
-            const cudaError_t e = cudaFuncSetAttribute(k_statmc_tma<RC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                       int(smem));
-            if (e != cudaSuccess) return e;
-            allowed = smem;
-        }
-    }
+    static FuncAttribute limit;
+    if (const cudaError_t e = limit.at_least(reinterpret_cast<const void*>(&k_statmc_tma<RC>),
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, j.ctx->device, int64_t(smem));
+        e != cudaSuccess)
+        return e;
     const cudaError_t e = window_map(j, prm.r, by);
     if (e != cudaSuccess) return e;
     CUtensorMap map;

@@ -321,7 +321,7 @@ cudaError_t launch_offsets_scan(Job& j, const int32_t* d_counts, int64_t count);
 const int64_t* offsets_count_max(const Job& j, int64_t count);
 cudaError_t launch_accumulate_pixels(Job& j, const DeviceSamples& s, int64_t first, int64_t count,
                                      const GridPrep& gp, int32_t spp);
-cudaError_t launch_accumulate_grid(Job& j, const DeviceSamples& s, int64_t first, int64_t count);
+cudaError_t launch_accumulate_grid(Job& j, const DeviceSamples& s, int64_t first, int64_t count, int32_t spp);
 // max_count bounds the samples of one pixel; total_samples bounds the samples of the push. Either
 // bound can make the bin weights exact integers (no bin of a node can then pass 2^32 units).
 // d_max_count: the push's largest per-pixel count in device memory when the host does not know it
@@ -400,6 +400,22 @@ int job_create(Ctx* c, const rpd_config* cfg, cudaMemPool_t pool, Job** out);
 // offsets_ready: j.offsets already holds the push's offsets (a scan of the same counts).
 int push_device_async(Job& j, const DeviceSamples& d, int64_t first, int64_t count, int32_t spp, const int32_t* counts,
                       int64_t total_bound, bool offsets_ready = false);
+
+// A kernel's attribute (its dynamic shared memory limit, its carve-out), set on each device the first time a
+// launch asks for that much or more: a 64x48 frame, bound by the host's calls, takes 82 us with three of them set
+// anew and four launches and clears that have since been folded into others, 77 us now.
+struct FuncAttribute {
+    std::mutex mu;
+    std::unordered_map<int, int64_t> value;  // per device
+    cudaError_t at_least(const void* kernel, cudaFuncAttribute attr, int device, int64_t v) {
+        std::lock_guard<std::mutex> lock(mu);
+        const auto it = value.find(device);
+        if (it != value.end() && it->second >= v) return cudaSuccess;
+        const cudaError_t e = cudaFuncSetAttribute(kernel, attr, int(v));
+        if (e == cudaSuccess) value[device] = v;
+        return e;
+    }
+};
 
 inline unsigned grid_for(int64_t n, int block) {
     return static_cast<unsigned>((n + block - 1) / block);
