@@ -1,8 +1,8 @@
 // compute_adaptive_sample_counts (main.cpp:1273-1446).
 //
 //   k_importance        variance source and importance = sqrt (1303-1327)
-//   k_smooth_importance edge-aware smoothing (1331-1368), its double-precision products carried
-//                       out exactly in integer instructions
+//   k_smooth_importance edge-aware smoothing (1331-1368), in pairs of singles where they decide the
+//                       float, else its double-precision products exactly in integer instructions
 //   k_allocate_coop     the budget-preserving allocation (1329-1438) in parallel, with the
 //                       reference's integers bit for bit (k_allocate.cu)
 //   k_allocate_serial   the same allocation as one device thread in the reference's order. It
@@ -21,7 +21,7 @@ namespace {
 
 __device__ __forceinline__ float pixel_variance(float m2, int n) { return (n > 1) ? m2 / float(n - 1) : 0.0f; }
 
-__global__ void k_importance(PixelPlanes p, int64_t np, float sigma_max) {
+__global__ void k_importance(PixelPlanes p, int64_t np, float sigma_max, float* importance) {
     const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= np) return;
     float raw = pixel_variance(p.square_diff[i], p.n[i]);
@@ -30,7 +30,7 @@ __global__ void k_importance(PixelPlanes p, int64_t np, float sigma_max) {
     float dsv = p.variance_denoised[i];
     if (!isfinite(dsv) || dsv <= 0.0f) dsv = raw;
     const float vs = fclamps(fmaxs(raw, dsv), 1e-8f, sigma_max * sigma_max);
-    p.importance[i] = sqrtf(vs);
+    importance[i] = sqrtf(vs);
 }
 
 // The edge-aware smoothing of one pixel (main.cpp:1339-1366) in the reference's double-precision
@@ -131,6 +131,59 @@ __device__ bool smooth_pixel_int(const PixelPlanes& p, int w, int h, int radius,
     return true;
 }
 
+// (h, l) + (a, b), kept as a pair: h + a with its exact error (Knuth's TwoSum)
+__device__ __forceinline__ void pair_add(float& h, float& l, float a, float b) {
+    const float s = h + a, t = s - h;
+    l += ((h - (s - t)) + (a - t)) + b;
+    h = s;
+}
+
+// The same pixel in pairs of singles: a weight is the product of three floats, exact to 2^-46, and the sums
+// keep their additions' errors. The low parts of sums of n terms are off by at most n^2 2^-50 of the sum, the
+// reference's doubles by less, so where the quotient rounds to the same float with `margin` = 2^-36 (n <= 49, radius
+// 3) added or taken away, that float is the reference's. Returns false elsewhere: exact ties, sums too small
+// for their low parts, zeros, infinities and NaN.
+template <int R>
+__device__ __forceinline__ bool smooth_pixel_pairs(const PixelPlanes& p, int w, int h, int radius, const float* in, int x,
+                                                   int y, int64_t idx, float& out) {
+    const int rad = R > 0 ? R : radius;
+    const float ni0 = p.f_normal[0][idx], ni1 = p.f_normal[1][idx], ni2 = p.f_normal[2][idx];
+    const float di = p.f_depth[idx];
+    float ah = 0.0f, al = 0.0f, wh = 0.0f, wl = 0.0f;
+#pragma unroll
+    for (int dy = -rad; dy <= rad; ++dy) {
+        const int yy = y + dy;
+        if (yy < 0 || yy >= h) continue;
+        const int64_t row = idx + int64_t(dy) * w;
+#pragma unroll
+        for (int dx = -rad; dx <= rad; ++dx) {
+            const int xx = x + dx;
+            if (xx < 0 || xx >= w) continue;
+            const int64_t nidx = row + dx;
+            if (p.hit_count[nidx] == 0) continue;
+            const float spatial_w = 1.0f / (1.0f + float(dx * dx + dy * dy));
+            const float normal_w = fclamps(
+                (dot3(ni0, ni1, ni2, p.f_normal[0][nidx], p.f_normal[1][nidx], p.f_normal[2][nidx]) + 1.0f) * 0.5f,
+                0.0f, 1.0f);
+            const float depth_w = expf(-4.0f * relative_depth_delta(di, p.f_depth[nidx]));
+            const float imp = in[nidx];
+            const float nd = normal_w * depth_w, nde = __fmaf_rn(normal_w, depth_w, -nd);
+            const float wn = nd * spatial_w, wne = __fmaf_rn(nd, spatial_w, -wn) + nde * spatial_w;
+            const float a = wn * imp, ae = __fmaf_rn(wn, imp, -a) + wne * imp;
+            pair_add(wh, wl, wn, wne);
+            pair_add(ah, al, a, ae);
+        }
+    }
+    const float q = ah / wh;
+    const float ql = (__fmaf_rn(-q, wh, ah) + __fmaf_rn(-q, wl, al)) / wh;
+    const float up = q + __fmaf_rn(q, 1.4551915e-11f, ql), down = q + __fmaf_rn(q, -1.4551915e-11f, ql);  // 2^-36
+    out = up;
+    return up == down && up < INFINITY && wh > 1e-6f && ah > 1e-20f;
+}
+
+// Bound by instruction issue: 40 us at 1280x720, radius 1. A frame there with one adaptive step took 2.825 ms with the
+// integer form for every pixel and the result copied back, 2.792 with pairs first and the planes' roles exchanged;
+// a burst of 8 served requests of 3 steps 16.99 and 16.52 ms.
 __global__ void k_smooth_importance(PixelPlanes p, int w, int h, int radius, const float* in, float* out,
                                     int fp64) {
     const int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -142,7 +195,10 @@ __global__ void k_smooth_importance(PixelPlanes p, int w, int h, int radius, con
     const int y = int(idx / w), x = int(idx % w);
     float v = 0.0f;
     bool done = false;
-    if (!fp64) {
+    if (!fp64 && radius <= 3)
+        done = radius == 1 ? smooth_pixel_pairs<1>(p, w, h, radius, in, x, y, idx, v)
+                           : smooth_pixel_pairs<0>(p, w, h, radius, in, x, y, idx, v);
+    if (!fp64 && !done) {
         done = radius == 1 ? smooth_pixel_int<1>(p, w, h, radius, in, x, y, idx, v)
                            : smooth_pixel_int<0>(p, w, h, radius, in, x, y, idx, v);
     }
@@ -245,11 +301,6 @@ __global__ void k_fill_counts(int32_t* counts, int64_t np, int value) {
     if (i < np) counts[i] = value;
 }
 
-__global__ void k_copy(const float* src, float* dst, int64_t n) {
-    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i < n) dst[i] = src[i];
-}
-
 }  // namespace
 
 namespace {
@@ -283,14 +334,14 @@ cudaError_t launch_adaptive(Job& j) {
     k_fill_counts<<<grid_for(np, 256), 256, 0, j.stream>>>(j.p.counts, np, floor_per_pixel);
     j.launches += 1;
     if (extra_sample_total <= 0) return cudaGetLastError();
-    k_importance<<<grid_for(np, 256), 256, 0, j.stream>>>(j.p, np, j.cfg.adaptive_sigma_max);
-    j.launches += 1;
     const int radius = j.cfg.adaptive_importance_smoothing_radius;
+    k_importance<<<grid_for(np, 256), 256, 0, j.stream>>>(j.p, np, j.cfg.adaptive_sigma_max,
+                                                          radius > 0 ? j.p.importance_tmp : j.p.importance);
+    j.launches += 1;
     if (radius > 0) {
-        k_smooth_importance<<<grid_for(np, 128), 128, 0, j.stream>>>(j.p, w, h, radius, j.p.importance,
-                                                                     j.p.importance_tmp, j.smooth_fp64 ? 1 : 0);
-        k_copy<<<grid_for(np, 256), 256, 0, j.stream>>>(j.p.importance_tmp, j.p.importance, np);
-        j.launches += 2;
+        k_smooth_importance<<<grid_for(np, 128), 128, 0, j.stream>>>(j.p, w, h, radius, j.p.importance_tmp,
+                                                                     j.p.importance, j.smooth_fp64 ? 1 : 0);
+        j.launches += 1;
     }
     return launch_allocation(j, extra_sample_total, floor_per_pixel);
 }
