@@ -2153,10 +2153,13 @@ cudaError_t launch_grid_fast(Job& j, const DeviceSamples& s, int64_t first, int6
             TotalsParams tp{j.g, first, count, ny0, ny1, 1, 1, sh, fresh ? 1 : 0, odd_count, odd_nodes};
             const int cells = 32 / step, image_cells = (j.g.w + step - 1) / step;
             tp.col_warps = std::max(1, (image_cells - 1 + cells - 2) / (cells - 1));
-            // node rows per warp: one more strip than node rows is walked, so as many as leave
-            // 16 warps per SM
-            const int64_t warps16 = int64_t(kStripSms) * 16;
-            tp.len = int(std::min<int64_t>(16, std::max<int64_t>(1, int64_t(tp.col_warps) * (ny1 - ny0) / warps16)));
+            // node rows per warp: one more strip than node rows is walked, so as many as fit in the 20
+            // warps an SM holds at 90 registers, in one wave (1280x720 with an adaptive pass, grid 333 us
+            // with the 16-warp quotient rounded down, two waves of single rows, and 292 us; half as many
+            // warps 445)
+            const int64_t resident = int64_t(kStripSms) * 20;
+            const int64_t rows = (int64_t(tp.col_warps) * (ny1 - ny0) + resident - 1) / resident;
+            tp.len = int(std::min<int64_t>(16, std::max<int64_t>(1, rows)));
             const int64_t warps = int64_t(tp.col_warps) * ((ny1 - ny0 + tp.len - 1) / tp.len);
             k_grid_totals<<<unsigned((warps + 3) / 4), 128, 0, j.stream>>>(tp, target, gp);
             if ((e = cudaGetLastError()) != cudaSuccess) return e;
