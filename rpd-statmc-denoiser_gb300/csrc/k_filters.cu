@@ -63,12 +63,20 @@ __device__ __forceinline__ float exp2_approx(float x) {
     return r;
 }
 
+// to 2^-23
+__device__ __forceinline__ float sqrt_approx(float x) {
+    float r;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 // acos(clamp(d, -1, 1))^2 of N values. With t = 1 - cos a, a^2 = 4 asin^2(sqrt(t / 2)) is a power
 // series in t (2t + t^2 / 3 + ...) that converges up to t = 2: for angles up to 90 degrees a polynomial
 // a^2 = t p(t) of degree 7 in t, fitted to minimise the relative error over t in [0, 1] by
 // iteratively reweighted least squares on Chebyshev nodes (1.7e-7 with the rounding of its
-// single-precision evaluation; the square of an angle to 2 ulp is off by up to 4.8e-7). Larger angles,
-// rare between pixels that weigh anything, through pi - acos(|d|), behind one branch for all N. A NaN
+// single-precision evaluation; the square of an angle to 2 ulp is off by up to 4.8e-7). Larger angles
+// through pi - acos(|d|), behind one branch for all N (normals in every direction take it at nearly every tap:
+// a joint bilateral of such an image 0.87 ms with the IEEE square root, 0.63 with the approximate one). A NaN
 // falls out of the saturation: the callers add 0 * d to the exponent.
 template <int N>
 __device__ __forceinline__ void angles_squared(const float (&d)[N], float (&a2)[N]) {
@@ -91,7 +99,7 @@ __device__ __forceinline__ void angles_squared(const float (&d)[N], float (&a2)[
     if (least < 0.0f) {
 #pragma unroll
         for (int k = 0; k < N; ++k) {
-            const float a = 3.14159265f - sqrtf(a2[k]);
+            const float a = 3.14159265f - sqrt_approx(a2[k]);
             if (d[k] < 0.0f) a2[k] = a * a;
         }
     }
@@ -155,10 +163,11 @@ __device__ __forceinline__ void atrous_row(const AtrousTap& tap, float lx, float
 
 // One a-trous pass over records (rgb, luminance), unit normals and albedo. rgb: the interleaved
 // output of the last pass, else nullptr.
-// Bound by instruction issue with the records' latency close behind (64% of the issue slots at 16
+// Bound by instruction issue with the records' latency close behind (68% of the issue slots at 16
 // warps per SM). One pass at 1920x1080: about 150 us with one pixel per thread, the arc cosine and the
 // colour read as three components; 113-127 us with four pixels and the polynomial, 89-101 us with
-// one branch per row for the angles above 90 degrees, 85-94 us with the reads a row ahead.
+// one branch per row for the angles above 90 degrees, 85-94 us with the reads a row ahead, 79-87 us
+// with the approximate square root there (the IEEE one has a path of its own, which splits the code).
 // Limits for three or four blocks per SM spill or lose the reads ahead: 5-7% slower.
 __global__ void __launch_bounds__(256, 2) k_atrous_pass(const float4* __restrict__ in, float4* __restrict__ out,
                                                      float* __restrict__ rgb, const float4* __restrict__ nrm,
@@ -395,7 +404,7 @@ __device__ __forceinline__ void bilateral_taps(const float4* __restrict__ S, int
 // Bound by instruction issue (85% of the slots). At 1920x1080, r = 6: 0.94 ms with one pixel per thread,
 // clamped coordinates at every tap, three separate gaussian sums and the arc cosine; 0.64 ms with two
 // pixels, the row sums and the polynomial, 0.56 ms with one branch per tap for both angles and four taps
-// per turn at two blocks per SM (three blocks 0.58, eight taps 0.58).
+// per turn at two blocks per SM (three blocks 0.58, eight taps 0.58), 0.53 ms with the approximate square root.
 template <bool kTiled>
 __global__ void __launch_bounds__(kBx * kBy, 2)
     k_joint_bilateral(const float4* __restrict__ rec, BilateralParams prm, float* __restrict__ gaussian,
