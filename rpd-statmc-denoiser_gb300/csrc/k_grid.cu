@@ -673,8 +673,8 @@ __global__ void __launch_bounds__(32) k_grid_screen(GridParams gpar, float2* pas
 // A validity pattern at a time: its sums enter every class it holds. Samples outside their pixel's
 // nominal bin, and pixels with more patterns than the statistics pass keeps (deviant), are
 // k_grid_odd's. The bound is load latency (18 warps per SM, one pass over 24 bytes a pixel): with
-// k_grid_odd 0.119 ms at 1920x1080 against 0.213 ms for the pattern form; where a pixel's samples
-// hold three patterns, 0.30 against 0.82 ms.
+// k_grid_odd 0.098 ms at 1920x1080 against 0.213 ms for the pattern form; where a pixel's samples
+// hold three patterns, 0.28 against 0.82 ms.
 struct TotalsParams {
     Geometry g;
     int64_t first, count;
@@ -996,25 +996,37 @@ __device__ void odd_node(const GridParams& gpar, float2* grid, const DeviceSampl
     // one row of 2 step - 1 pixels (or two, for steps up to 8) at a time
     const int lw = step <= 8 ? 16 : 32, rows = 32 / lw;
     const int lx = lane & (lw - 1), lr = lane / lw;
-    for (int y0 = ylo; y0 <= yhi; y0 += rows) {
-        const int x = xlo + lx, y = y0 + lr;
-        const int64_t idx = int64_t(y) * g.w + x;
-        bool odd = false;
-        if (x <= xhi && y <= yhi && idx >= gpar.first && idx < gpar.first + gpar.count) {
-            const uint32_t bits = __float_as_uint(gp.pat2[idx].y);
-            odd = odd_pixel(bits);
-            deviants = deviants || ((bits >> 8) & kPixDeviant);
+    // in batches, their loads before any is used: the scan was most of a node's time, a chain of one load
+    // latency per row (the grid's totals and screen bins of 1920x1080x16, where a block takes two nodes in turn:
+    // 117 -> 108 us; 98 us with the odd pixels' samples spread over the lanes below)
+    constexpr int kBatch = 8;
+    constexpr int kDeviantEntry = 0x8000;
+    const int x = xlo + lx;
+    for (int yb = ylo; yb <= yhi; yb += rows * kBatch) {
+        uint32_t bits[kBatch];
+#pragma unroll
+        for (int b = 0; b < kBatch; ++b) {
+            const int y = yb + b * rows + lr;
+            const int64_t idx = int64_t(y) * g.w + x;
+            const bool in = x <= xhi && y <= yhi && idx >= gpar.first && idx < gpar.first + gpar.count;
+            bits[b] = in ? __float_as_uint(gp.pat2[idx].y) : uint32_t(kPixUniform) << 8;  // not odd
         }
-        const unsigned m = __ballot_sync(0xffffffffu, odd);
-        if (odd) list[nodd + __popc(m & ((1u << lane) - 1))] = uint16_t((y - ylo) * 64 + x - xlo);
-        nodd += __popc(m);
+#pragma unroll
+        for (int b = 0; b < kBatch; ++b) {
+            const bool odd = odd_pixel(bits[b]);
+            const bool dev = ((bits[b] >> 8) & kPixDeviant) != 0;
+            deviants = deviants || dev;
+            const unsigned m = __ballot_sync(0xffffffffu, odd);
+            if (odd) list[nodd + __popc(m & ((1u << lane) - 1))] = uint16_t((dev ? kDeviantEntry : 0) | ((yb + b * rows + lr - ylo) * 64 + x - xlo));
+            nodd += __popc(m);
+        }
     }
     if (nodd == 0) return;
     __syncwarp();
     deviants = __any_sync(0xffffffffu, deviants);
     auto pixel = [&](int i, int& x, int& y, int64_t& idx) {
         x = xlo + (list[i] & 63);
-        y = ylo + (list[i] >> 6);
+        y = ylo + ((list[i] & (kDeviantEntry - 1)) >> 6);
         idx = int64_t(y) * g.w + x;
     };
     auto weight = [&](int x, int y) {
@@ -1028,7 +1040,30 @@ __device__ void odd_node(const GridParams& gpar, float2* grid, const DeviceSampl
     auto nominal_bin = [&](int x, int y) {
         return ((y - (ny - 1) * step) >> (sh - 1)) * 4 + ((x - (nx - 1) * step) >> (sh - 1));
     };
-    auto is_deviant = [&](int64_t idx) { return ((__float_as_uint(gp.pat2[idx].y) >> 8) & kPixDeviant) != 0; };
+    auto is_deviant = [&](int i) { return (list[i] & kDeviantEntry) != 0; };
+    // f(x, y, k) for every sample k of the odd pixels that are not deviant: a uniform push's pixels and samples
+    // are one range over the lanes
+    const bool has_pu = s.compact ? s.c16.pixel_u[0] && s.c16.pixel_u[1] : s.pixel_u[0] && s.pixel_u[1];
+    auto for_samples = [&](auto f) {
+        if (!has_pu) return;  // no sample has a screen position
+        int x, y;
+        int64_t idx;
+        if (gpar.spp > 0) {
+            for (int t = lane; t < nodd * gpar.spp; t += 32) {
+                const int i = t / gpar.spp;
+                if (is_deviant(i)) continue;
+                pixel(i, x, y, idx);
+                f(x, y, (idx - gpar.first) * gpar.spp + (t - i * gpar.spp));
+            }
+            return;
+        }
+        for (int i = 0; i < nodd; ++i) {
+            if (is_deviant(i)) continue;
+            pixel(i, x, y, idx);
+            const int64_t kend = offsets[idx - gpar.first + 1];
+            for (int64_t k = offsets[idx - gpar.first] + lane; k < kend; k += 32) f(x, y, k);
+        }
+    };
     auto pattern_of = [](uint32_t key) {
         uint32_t p = 0u;
 #pragma unroll
@@ -1038,43 +1073,26 @@ __device__ void odd_node(const GridParams& gpar, float2* grid, const DeviceSampl
     };
     // the patterns of the samples to move
     PatternSet set;
-    for (int i = 0; i < nodd; ++i) {
-        int x, y;
-        int64_t idx;
-        pixel(i, x, y, idx);
-        if (is_deviant(idx)) continue;
-        const int b0 = nominal_bin(x, y);
-        const int64_t local = idx - gpar.first, kend = sample_offset(offsets, gpar.spp, local + 1);
-        for (int64_t k = sample_offset(offsets, gpar.spp, local) + lane; k < kend; k += 32) {
-            const uint32_t key = gp.key[k];
-            if (!(key & key_absent_bit(0)) && exact_bin(x, y, k) != b0) set.add(pattern_of(key));
-        }
-    }
+    for_samples([&](int x, int y, int64_t k) {
+        const uint32_t key = gp.key[k];
+        const int b = exact_bin(x, y, k);
+        if (!(key & key_absent_bit(0)) && b != nominal_bin(x, y)) set.add(pattern_of(key));
+    });
     set.unite_warp();
-    Totals unused;
     for (uint32_t P = set.pop(); P != 0u; P = set.pop()) {
         bins.clear();
         __syncwarp();
-        for (int i = 0; i < nodd; ++i) {
-            int x, y;
-            int64_t idx;
-            pixel(i, x, y, idx);
-            if (is_deviant(idx)) continue;
-            const int b0 = nominal_bin(x, y);
+        for_samples([&](int x, int y, int64_t k) {
+            const uint32_t key = gp.key[k];
+            const float yv = gp.lum[k];
+            const int b = exact_bin(x, y, k), b0 = nominal_bin(x, y);
+            if ((key & key_absent_bit(0)) || b == b0 || pattern_of(key) != P) return;
             const float w = weight(x, y);
-            const int64_t local = idx - gpar.first, kend = sample_offset(offsets, gpar.spp, local + 1);
-            for (int64_t k = sample_offset(offsets, gpar.spp, local) + lane; k < kend; k += 32) {
-                const uint32_t key = gp.key[k];
-                if ((key & key_absent_bit(0)) || pattern_of(key) != P) continue;
-                const int b = exact_bin(x, y, k);
-                if (b == b0) continue;
-                const float yv = gp.lum[k];
-                bins.add_weight(b, w, 1.0f);
-                bins.add_sum(b, w, yv, 0.0f);
-                bins.add_weight(b0, -w, 1.0f);
-                bins.add_sum(b0, -w, yv, 0.0f);
-            }
-        }
+            bins.add_weight(b, w, 1.0f);
+            bins.add_sum(b, w, yv, 0.0f);
+            bins.add_weight(b0, -w, 1.0f);
+            bins.add_sum(b0, -w, yv, 0.0f);
+        });
         const float2 v = bins.reduce_value();
         if (v.x == 0.0f && v.y == 0.0f) continue;
 #pragma unroll
