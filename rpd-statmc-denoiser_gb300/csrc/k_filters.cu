@@ -161,7 +161,8 @@ __device__ __forceinline__ void atrous_row(const AtrousTap& tap, float lx, float
     }
 }
 
-// One a-trous pass over records (rgb, luminance), unit normals and albedo. rgb: the interleaved
+// One a-trous pass over records (rgb, luminance), unit normals and albedo. sx, sy: the step, at most the
+// image's width and height (atrous_step). rgb: the interleaved
 // output of the last pass, else nullptr.
 // Bound by instruction issue with the records' latency close behind (68% of the issue slots at 16
 // warps per SM). One pass at 1920x1080: about 150 us with one pixel per thread, the arc cosine and the
@@ -171,16 +172,16 @@ __device__ __forceinline__ void atrous_row(const AtrousTap& tap, float lx, float
 // Limits for three or four blocks per SM spill or lose the reads ahead: 5-7% slower.
 __global__ void __launch_bounds__(256, 2) k_atrous_pass(const float4* __restrict__ in, float4* __restrict__ out,
                                                      float* __restrict__ rgb, const float4* __restrict__ nrm,
-                                                     const float4* __restrict__ alb, int w, int h, int step, float kc,
+                                                     const float4* __restrict__ alb, int w, int h, int sx, int sy, float kc,
                                                      float kn, float ka) {
     const int x = blockIdx.x * 32 + threadIdx.x;
-    const int group = blockIdx.y * 8 + threadIdx.y;  // rows y0, y0 + step, ... of one group
-    const int y0 = group / step * (kAtrousRows * step) + group % step;
+    const int group = blockIdx.y * 8 + threadIdx.y;  // rows y0, y0 + sy, ... of one group
+    const int y0 = group / sy * (kAtrousRows * sy) + group % sy;
     if (x >= w || y0 >= h) return;
     AtrousPixels p;
 #pragma unroll
     for (int k = 0; k < kAtrousRows; ++k) {
-        const int64_t i = int64_t(imins(y0 + k * step, h - 1)) * w + x;
+        const int64_t i = int64_t(imins(y0 + k * sy, h - 1)) * w + x;
         p.ni[k] = nrm[i];
         p.ai[k] = alb[i];
         p.li[k] = in[i].w;
@@ -188,16 +189,16 @@ __global__ void __launch_bounds__(256, 2) k_atrous_pass(const float4* __restrict
     }
     int64_t rows[kAtrousRows + 4];
 #pragma unroll
-    for (int j = 0; j < kAtrousRows + 4; ++j) rows[j] = int64_t(iclamps(y0 + (j - 2) * step, 0, h - 1)) * w;
+    for (int j = 0; j < kAtrousRows + 4; ++j) rows[j] = int64_t(iclamps(y0 + (j - 2) * sy, 0, h - 1)) * w;
     auto load = [&](int j, int xx) {
         const int64_t q = rows[j] + xx;
         return AtrousTap{in[q], nrm[q], alb[q]};
     };
-    int xx = iclamps(x - 2 * step, 0, w - 1);
+    int xx = iclamps(x - 2 * sx, 0, w - 1);
     AtrousTap tap[2] = {load(0, xx), {}};  // each tap is read a row ahead of its use
 #pragma unroll 1
     for (int kx = 0; kx < 5; ++kx) {
-        const int xn = iclamps(x + (kx - 1) * step, 0, w - 1);
+        const int xn = iclamps(x + (kx - 1) * sx, 0, w - 1);
         const float lx = b3_log2(kx);
         tap[1] = load(1, xx);
         atrous_row<0>(tap[0], lx, kc, kn, ka, p);
@@ -219,7 +220,7 @@ __global__ void __launch_bounds__(256, 2) k_atrous_pass(const float4* __restrict
     }
 #pragma unroll
     for (int k = 0; k < kAtrousRows; ++k) {
-        const int y = y0 + k * step;
+        const int y = y0 + k * sy;
         if (y >= h) continue;
         const int64_t i = int64_t(y) * w + x;
         float4 v;
@@ -490,12 +491,9 @@ float neg_log2e_two_sq(float sigma, double scale = 1.0) {
     return float(-1.4426950408889634 * scale / (2.0 * double(sigma) * double(sigma)));
 }
 
-// 2^it, or the image's larger side where that is less: from there on every tap but the centre's row or
-// column is clamped to the edge.
-int atrous_step(int it, int w, int h) {
-    const int side = std::max(w, h);
-    return it < 30 ? std::min(1 << it, side) : side;
-}
+// 2^it, or the image's extent where that is less: from there on every tap but the centre's is clamped to the
+// edge. (Groups of rows a step apart beyond the height would exceed the grid.)
+int atrous_step(int it, int extent) { return it < 30 ? std::min(1 << it, extent) : extent; }
 
 }  // namespace
 
@@ -516,12 +514,12 @@ cudaError_t launch_atrous(const float* raw, const float* normal, const float* al
     k_atrous_records<<<grid_for(np, 256), 256, 0, stream>>>(raw, normal, albedo, np, a, nrm, alb);
     const float kc = neg_log2e_two_sq(sigma_c), kn = neg_log2e_two_sq(sigma_n), ka = neg_log2e_two_sq(sigma_a);
     for (int it = 0; it < iterations; ++it) {
-        const int step = atrous_step(it, w, h);
-        // groups of kAtrousRows rows `step` apart: `step` of them per kAtrousRows * step rows
-        const int64_t span = int64_t(kAtrousRows) * step;
-        const int64_t groups = (h + span - 1) / span * step;
+        const int sx = atrous_step(it, w), sy = atrous_step(it, h);
+        // groups of kAtrousRows rows sy apart: sy of them per kAtrousRows * sy rows
+        const int64_t span = int64_t(kAtrousRows) * sy;
+        const int64_t groups = (h + span - 1) / span * sy;
         const dim3 grid((w + 31) / 32, unsigned((groups + 7) / 8));
-        k_atrous_pass<<<grid, dim3(32, 8), 0, stream>>>(a, b, it + 1 == iterations ? out : nullptr, nrm, alb, w, h, step,
+        k_atrous_pass<<<grid, dim3(32, 8), 0, stream>>>(a, b, it + 1 == iterations ? out : nullptr, nrm, alb, w, h, sx, sy,
                                                         kc, kn, ka);
         std::swap(a, b);
     }
@@ -540,7 +538,7 @@ cudaError_t launch_atrous_plain(const float* raw, const float* normal, const flo
     float* other = buf_b;
     *result = const_cast<float*>(raw);
     for (int it = 0; it < iterations; ++it) {
-        k_atrous_pass_plain<<<grid, block, 0, stream>>>(in, out, normal, albedo, w, h, atrous_step(it, w, h), kc, kn, ka);
+        k_atrous_pass_plain<<<grid, block, 0, stream>>>(in, out, normal, albedo, w, h, atrous_step(it, std::max(w, h)), kc, kn, ka);
         *result = out;
         in = out;
         float* t = out;

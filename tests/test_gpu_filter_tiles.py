@@ -99,3 +99,19 @@ def test_angle_polynomial():
     want = 4 * np.arcsin(np.sqrt(t.astype(np.float64) / 2)) ** 2
     assert np.max(np.abs(p[keep] - want[keep]) / want[keep]) <= 4 * 2.0**-24 + 2.0**-23
     assert np.all(p[~keep] == 0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("w,h", [(600_000, 1), (2, 300_000)])
+def test_steps_beyond_a_thin_image(gpu_ctx, w, h):
+    """Steps that pass the height of a wide image and the width of a tall one, to the extent of the other side:
+    the records form against the form without records, which takes one pixel per thread (the same
+    arithmetic, at the no-allocation test's 1e-6)."""
+    torch = pytest.importorskip("torch")
+    from test_zz_no_alloc import _run_noalloc
+
+    raw, normal, albedo = images(w, h, True)
+    want = _run_noalloc(gpu_ctx, torch.cuda.Stream(), raw, normal, albedo, (0.3, 0.6, 0.1), 21)
+    got = gpu_ctx.atrous(raw, normal, albedo, 0.3, 0.6, 0.1, 21)
+    err = np.max(np.abs(got.astype(np.float64) - want) / np.maximum(np.abs(want), 1e-3))
+    assert err <= 1e-6
