@@ -417,7 +417,7 @@ int rpd_config_validate(const rpd_config* c, char* msg, size_t cap) {
 // 1920x1080 0.88 ms per a-trous call and 0.93 per joint bilateral, 0.50 and 0.61 with the pool).
 // 512 MiB holds the a-trous filter's 64 bytes per pixel at 3840x2160; beyond it, and when another
 // allocation would fail, the driver unmaps what is free. rpd_ctx_destroy gives it all back. Creating the pool
-// costs a context about 1 ms, once.
+// costs a context about 25 us, once.
 constexpr uint64_t kPoolKeep = uint64_t(512) << 20;
 
 int rpd_ctx_create(int device, uint64_t budget, rpd_ctx** out) {
