@@ -600,13 +600,17 @@ __device__ __forceinline__ void store_prep(const GridPrep& gp, int64_t k, const 
 // VEC4: every present plane is 16-byte aligned at the pixel's first sample and the pixel's
 // sample count is a multiple of 4, so each plane is read four samples per load. COMPACT: the
 // planes are rpd_sample_soa16's (s.c16), decoded to float here; WIDE reads them 8 samples (16
-// bytes) per load. PART: what the thread keeps of its pixel.
+// bytes) per load. PART: what the thread keeps of its pixel. The two parts of a split pixel both read
+// its count p.n, which the luminance part writes: their block meets between the last of these loads and the
+// first store. At the end of the walk that costs nothing, as a block's places are free when its slowest
+// warp is done. Every thread of a split block gets there (local >= count: no pixel), a warp's threads together.
 template <bool VEC4, bool COMPACT, bool WIDE, Part PART>
 __device__ __forceinline__ void accumulate_pixel(const PixelPlanes& p, const DeviceSamples& s, const int64_t* offsets, int spp,
-                                                 int64_t local, int64_t first, const GridPrep& gp, int fresh) {
-    constexpr bool colour = PART != kLuminance, lumi = PART != kColour;
+                                                 int64_t local, int64_t first, int64_t count, const GridPrep& gp, int fresh) {
+    constexpr bool colour = PART != kLuminance, lumi = PART != kColour, split = PART != kWhole;
+    const bool mine = !split || local < count;
     const int64_t idx = first + local;
-    const int64_t k0 = sample_offset(offsets, spp, local), k1 = sample_offset(offsets, spp, local + 1);
+    const int64_t k0 = mine ? sample_offset(offsets, spp, local) : 0, k1 = mine ? sample_offset(offsets, spp, local + 1) : 0;
     const bool prep = gp.lum != nullptr;
     const bool has_pu = COMPACT ? s.c16.pixel_u[0] != nullptr : s.pixel_u[0] != nullptr;
     const bool has_lu = COMPACT ? s.c16.lens_u[0] != nullptr : s.lens_u[0] != nullptr;
@@ -626,14 +630,15 @@ __device__ __forceinline__ void accumulate_pixel(const PixelPlanes& p, const Dev
     a.cs = cls_local + (uint32_t(gp.width) >> 31);  // the width is positive: offset 0
     acc_init(a);
     if (k0 == k1) {
-        if (prep && lumi) acc_store_empty(gp, idx);
-        return;
+        if (mine && prep && lumi) acc_store_empty(gp, idx);
+        if (!split) return;
     }
+    const bool some = !split || k0 != k1;
     // fresh: the frame's first push over every pixel, whose statistics the frame start zeroed
     if (fresh) acc_zero(a);
-    else acc_load<PART>(a, p, idx);
+    else if (some) acc_load<PART>(a, p, idx);
     px.per_sample_albedo = !COMPACT && s.albedo[0] != nullptr;
-    load_pixel_albedo<COMPACT>(px, s, local);
+    if (some) load_pixel_albedo<COMPACT>(px, s, local);
     const bool dims = prep && lumi;  // the random dimensions are only read for the grid pass
 
     if (COMPACT) {
@@ -766,6 +771,10 @@ __device__ __forceinline__ void accumulate_pixel(const PixelPlanes& p, const Dev
         }
     }
 
+    if (split) {
+        __syncthreads();
+        if (!some) return;
+    }
     acc_store<PART>(a, p, gp, idx, prep);
 }
 
@@ -780,13 +789,12 @@ __global__ void __launch_bounds__(128, MINB) k_accumulate_pixels(PixelPlanes p, 
                                                                  int spp, int64_t first, int64_t count, GridPrep gp, int fresh) {
     if constexpr (SPLIT) {
         const int64_t local = int64_t(blockIdx.x) * 64 + (threadIdx.x & 63);
-        if (local >= count) return;
-        if (threadIdx.x < 64) accumulate_pixel<VEC4, COMPACT, WIDE, kLuminance>(p, s, offsets, spp, local, first, gp, fresh);
-        else accumulate_pixel<VEC4, COMPACT, WIDE, kColour>(p, s, offsets, spp, local, first, gp, fresh);
+        if (threadIdx.x < 64) accumulate_pixel<VEC4, COMPACT, WIDE, kLuminance>(p, s, offsets, spp, local, first, count, gp, fresh);
+        else accumulate_pixel<VEC4, COMPACT, WIDE, kColour>(p, s, offsets, spp, local, first, count, gp, fresh);
     } else {
         const int64_t local = int64_t(blockIdx.x) * 128 + threadIdx.x;
         if (local >= count) return;
-        accumulate_pixel<VEC4, COMPACT, WIDE, kWhole>(p, s, offsets, spp, local, first, gp, fresh);
+        accumulate_pixel<VEC4, COMPACT, WIDE, kWhole>(p, s, offsets, spp, local, first, count, gp, fresh);
     }
 }
 
