@@ -26,7 +26,8 @@ __device__ __forceinline__ float pixel_variance(float m2, int n) { return (n > 1
 inline int var_pitch(int w) { return (w + 3) & ~3; }
 
 // The clamped variance (main.cpp:1182-1186), negated for a pixel without a primary hit; the
-// pixel's gate record.
+// pixel's gate record. A pixel with a hit holds at least EPS_SMALL: the clamp's upper bound is less for
+// an adaptive_sigma_max below 1e-4, but every iteration reads such a value through max(EPS_SMALL, .).
 __global__ void k_var_init(PixelPlanes p, int w, int h, int pitch, float max_variance, float* curr) {
     const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= int64_t(w) * h) return;
@@ -35,7 +36,7 @@ __global__ void k_var_init(PixelPlanes p, int w, int h, int pitch, float max_var
     v = fclamps(v, 1e-8f, max_variance);
     const bool hit = p.hit_count[i] > 0;
     const int64_t y = i / w, x = i - y * w;
-    curr[y * pitch + x] = hit ? v : -v;
+    curr[y * pitch + x] = hit ? fmaxs(1e-8f, v) : -v;
     p.var_gate[i] = make_float4(p.f_normal[0][i], p.f_normal[1][i], p.f_normal[2][i], p.f_depth[i]);
 }
 
@@ -137,12 +138,12 @@ __device__ __noinline__ float2 var_exact_sums(const float* V, int vw, float var_
 // That gate compares |var_i - var_j| / max(EPS_SMALL, sqrt(var_i var_j)) with sigma, which for a given
 // var_i is a test of var_j against two bounds. Within 2^-19 of a bound, where the quotient's rounding
 // decides, the pixel's sums are taken again with the quotient itself (var_exact_sums). Passed neighbours are at
-// least EPS_SMALL, as is every value of the planes for a pixel with a hit (the update only raises it), so
-// the reference's maxima with EPS_SMALL change nothing.
+// least EPS_SMALL, as is every value of the planes for a pixel with a hit (k_var_init's; the update only raises
+// it), so the reference's maxima with EPS_SMALL change nothing.
 //
-// LAST: the iteration's result is the denoised variance itself. The reference takes the maximum with the
-// clamped raw variance (main.cpp:1252-1261), where the iterations began and below which none falls;
-// a pixel without a hit holds its negative.
+// last: the iteration's result is the denoised variance itself. The reference takes the maximum with the
+// clamped raw variance (main.cpp:1252-1261), which the iterations began at or, raised to EPS_SMALL, above, and below
+// which none falls; a pixel without a hit holds its negative.
 //
 // Bound by instruction issue. At 1920x1080, radius 3: MODE 1 184 us and MODE 2 94 us with one pixel per
 // thread, an rsqrt and two guarded quotients per neighbour, 17 us for the
