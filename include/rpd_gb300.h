@@ -439,7 +439,8 @@ int rpd_probe_fp32_issue(int device, int32_t repeats, double* per_second, double
 
 /* atrous_wavelet filter() core (denoising/atrous_wavelet.cpp:151-197): `iterations`
  * passes of atrous_filter_pass with step 2^i. raw/normal/albedo/out are interleaved RGB
- * W*H*3 floats in `where` memory. */
+ * W*H*3 floats in `where` memory. Both filters refuse images of more than 524,280 rows, and
+ * rpd_joint_bilateral radii ceil(3 sigma_p) above 120, with RPD_ERR_CUDA. */
 int rpd_atrous_wavelet(rpd_ctx* ctx, const float* raw, const float* normal, const float* albedo,
                        int32_t width, int32_t height, float sigma_c, float sigma_n, float sigma_a,
                        int32_t iterations, float* out, rpd_memory where);

@@ -1575,6 +1575,7 @@ int rpd_atrous_wavelet(rpd_ctx* ctx, const float* raw, const float* normal, cons
     Ctx* c = reinterpret_cast<Ctx*>(ctx);
     if (!c || !raw || !normal || !albedo || !out || w <= 0 || h <= 0 || iterations < 0)
         return fail(RPD_ERR_INVALID_ARGUMENT, "bad a-trous arguments");
+    if (iterations > 0) RPD_CUDA(filter_limits(h, 0.0f));
     RPD_CUDA(cudaSetDevice(c->device));
     cudaStream_t st = c->util_stream;
     const uint64_t bytes = uint64_t(w) * h * 12;
@@ -1611,6 +1612,7 @@ int rpd_joint_bilateral(rpd_ctx* ctx, const float* raw, const float* normal, con
     Ctx* c = reinterpret_cast<Ctx*>(ctx);
     if (!c || !raw || !normal || !albedo || !gaussian || !bilateral || !joint || w <= 0 || h <= 0)
         return fail(RPD_ERR_INVALID_ARGUMENT, "bad joint-bilateral arguments");
+    RPD_CUDA(filter_limits(h, sigma_p));
     RPD_CUDA(cudaSetDevice(c->device));
     cudaStream_t st = c->util_stream;
     const uint64_t bytes = uint64_t(w) * h * 12;

@@ -486,6 +486,12 @@ __global__ void __launch_bounds__(kBx * kBy, 2)
     }
 }
 
+// The largest radius taken: (2 r + 1)^2 taps per pixel. (sigma_p up to 40; a call for minutes is an error,
+// not a request.)
+constexpr int kBMaxRadius = 120;
+// Blocks of 8 rows of one pixel per thread: the tallest image that the grid's second dimension holds.
+constexpr int kFilterRows = 65535 * 8;
+
 float inv_two_sq(float sigma) { return float(1.0 / (2.0 * double(sigma) * double(sigma))); }
 float neg_log2e_two_sq(float sigma, double scale = 1.0) {
     return float(-1.4426950408889634 * scale / (2.0 * double(sigma) * double(sigma)));
@@ -496,6 +502,11 @@ float neg_log2e_two_sq(float sigma, double scale = 1.0) {
 int atrous_step(int it, int extent) { return it < 30 ? std::min(1 << it, extent) : extent; }
 
 }  // namespace
+
+cudaError_t filter_limits(int h, float sigma_p) {
+    if (h > kFilterRows) return cudaErrorInvalidConfiguration;
+    return std::ceil(3.0f * sigma_p) > float(kBMaxRadius) ? cudaErrorInvalidValue : cudaSuccess;
+}
 
 uint64_t atrous_scratch_bytes(int w, int h) { return uint64_t(w) * h * 4 * sizeof(float4); }
 

@@ -352,6 +352,9 @@ cudaError_t allocator_stats(Job& j, int32_t* out);
 int allocator_timeline(Job& j, uint64_t* ns, int32_t max, int32_t* n);
 cudaError_t launch_finalize(Job& j);
 cudaError_t launch_expand(Job& j, const float* node_field, float* out);
+// What the post-filters refuse before they allocate: images of more than 524,280 rows, and joint bilateral radii
+// above 120 (a sigma_p of 0: no joint bilateral).
+cudaError_t filter_limits(int h, float sigma_p);
 // `iterations` a-trous passes over records in `scratch` (atrous_scratch_bytes), the last one writing
 // the interleaved RGB `out`, which may be one of the inputs.
 uint64_t atrous_scratch_bytes(int w, int h);
