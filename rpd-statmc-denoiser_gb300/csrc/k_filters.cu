@@ -311,6 +311,10 @@ struct BilateralParams {
 
 constexpr int kBx = 32, kBy = 8;  // threads of a block
 constexpr int kBRows = 2;         // pixels of a thread, one above the other
+constexpr int kBMaxTiled = 16;    // the largest radius whose halo tile is in shared memory
+constexpr size_t bilateral_tile_bytes(int r) {
+    return 128 + size_t(kBx + 2 * r) * (kBy * kBRows + 2 * r) * B_COUNT * sizeof(float4) + size_t(2 * r + 1) * sizeof(float2);
+}
 
 // A thread's pixels (x, y0 .. y0 + kBRows - 1): their records and the three filters' sums (rgb, weight).
 struct BilateralPixels {
@@ -583,19 +587,19 @@ cudaError_t launch_joint_bilateral(const float* raw, const float* normal, const 
     const dim3 block(kBx, kBy);
     const int rows = kBy * kBRows;
     const dim3 grid((w + kBx - 1) / kBx, (h + rows - 1) / rows);
-    const size_t tables = size_t(2) * (2 * size_t(prm.r) + 1) * sizeof(float);
-    const bool tiled = prm.r <= 16;
+    const bool tiled = prm.r <= kBMaxTiled;
     CUtensorMap map{};
-    size_t smem = 128 + tables;
+    size_t smem = 128 + size_t(2 * prm.r + 1) * sizeof(float2);  // below 48 KB up to kBMaxRadius
     if (tiled) {
-        smem += size_t(kBx + 2 * prm.r) * (rows + 2 * prm.r) * B_COUNT * sizeof(float4);
+        smem = bilateral_tile_bytes(prm.r);
         e = encode_record_map(&map, rec, w, h, B_COUNT, kBx + 2 * prm.r, rows + 2 * prm.r);
         if (e != cudaSuccess) return e;
     }
+    // the limit belongs to the kernel, not to the call: always the largest tile's, so that no thread lowers it
+    // between another one's setting and its launch
     if (smem > 48 * 1024) {
-        e = tiled ? cudaFuncSetAttribute(k_joint_bilateral<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem))
-                  : cudaFuncSetAttribute(k_joint_bilateral<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         int(smem));
+        e = cudaFuncSetAttribute(k_joint_bilateral<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 int(bilateral_tile_bytes(kBMaxTiled)));
         if (e != cudaSuccess) return e;
     }
     if (tiled)

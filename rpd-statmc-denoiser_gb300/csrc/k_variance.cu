@@ -418,8 +418,10 @@ cudaError_t launch_variance(Job& j) {
     } else {
         const size_t smem = size_t(kVarTx + 2 * r) * size_t(kVarTy + 2 * r) * (sizeof(float4) + sizeof(float)) +
                             size_t(2 * r + 1) * size_t(2 * r + 1) * sizeof(float);
-        if (smem > size_t(200) * 1024) return cudaErrorInvalidValue;  // radius beyond the shared-memory tile
-        e = cudaFuncSetAttribute(k_var_smooth, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+        constexpr size_t limit = size_t(200) * 1024;
+        if (smem > limit) return cudaErrorInvalidValue;  // radius beyond the shared-memory tile
+        // (the kernel's limit, the same for every call: jobs on several threads may have different radii)
+        e = cudaFuncSetAttribute(k_var_smooth, cudaFuncAttributeMaxDynamicSharedMemorySize, int(limit));
         for (int it = 0; it < j.cfg.var_iterations && e == cudaSuccess; ++it) {
             const bool last = it + 1 == j.cfg.var_iterations;
             k_var_smooth<<<vgrid, dim3(kVarTx, kVarTy), smem, j.stream>>>(
