@@ -670,11 +670,13 @@ __global__ void __launch_bounds__(32) k_grid_screen(GridParams gpar, float2* pas
 // totals add up over the strip's two halves and the node's two cells. Each pixel is visited once (and
 // once more for the cell that neighbouring warps share) instead of once per node it supports, in
 // registers instead of lane-private bins in shared memory; warps are independent of each other.
-// A validity pattern at a time: its sums enter every class it holds. Samples outside their pixel's
-// nominal bin, and pixels with more patterns than the statistics pass keeps (deviant), are
-// k_grid_odd's. The bound is load latency (18 warps per SM, one pass over 24 bytes a pixel): with
-// k_grid_odd 0.098 ms at 1920x1080 against 0.213 ms for the pattern form; where a pixel's samples
-// hold three patterns, 0.28 against 0.82 ms.
+// A validity pattern at a time: its sums enter every class it holds. Then, where some pixel holds more patterns than
+// the statistics pass keeps (deviant), a class at a time over the class sums of such pixels. Samples outside
+// their pixel's nominal bin, and deviant pixels some of whose samples lack the position, are
+// k_grid_odd's. The bound is load latency (20 warps per SM, one pass over 24 bytes a pixel): with
+// k_grid_odd 0.100 ms at 1920x1080x16 against 0.213 ms for the pattern form; where a pixel's samples
+// hold three patterns, 0.28 against 0.82 ms, eight patterns 0.54 against 1.01 ms (29 ms with every deviant
+// pixel left to k_grid_odd, class by class and sample by sample).
 struct TotalsParams {
     Geometry g;
     int64_t first, count;
@@ -691,10 +693,18 @@ struct TotalsParams {
 __host__ __device__ constexpr int dep_random(int c) { return c == 0 ? 0 : 2 * c - 1; }
 __host__ __device__ constexpr int dep_screen(int c) { return 2 * c; }
 
-// Does k_grid_odd look at a pixel with these bits (pat2.y)?
+// Of a pixel with these bits (pat2.y): is it deviant, and are its class sums the screen's too (every sample
+// with a random dimension has a position)? Then k_grid_totals takes it class by class, else
+// k_grid_odd sample by sample.
+constexpr uint32_t kDeviantBit = uint32_t(kPixDeviant) << 8, kMixedBit = uint32_t(kPixMixed) << 8;
+__device__ __forceinline__ bool deviant(uint32_t bits) { return bits & kDeviantBit; }
+__device__ __forceinline__ bool class_pixel(uint32_t bits) { return (bits & (kDeviantBit | kMixedBit)) == kDeviantBit; }
+__device__ __forceinline__ bool sample_pixel(uint32_t bits) {
+    return (bits & (kDeviantBit | kMixedBit)) == (kDeviantBit | kMixedBit);
+}
+// Does k_grid_odd look at the pixel? (Only a sample with a position makes a pixel not uniform.)
 __device__ __forceinline__ bool odd_pixel(uint32_t bits) {
-    const uint32_t pats = bits | (bits >> 16) | (bits >> 24);
-    return ((bits >> 8) & kPixDeviant) || (!((bits >> 8) & kPixUniform) && (pats & RPD_SAMPLE_PIXEL_VALID));
+    return !(bits & (uint32_t(kPixUniform) << 8)) || sample_pixel(bits);
 }
 
 // A set of patterns, one bit each (patterns are even: bit p / 2).
@@ -737,7 +747,7 @@ __device__ __forceinline__ DF df_scaled(float a, DF b) {  // a * b
     return r;
 }
 
-__global__ void __launch_bounds__(128) k_grid_totals(TotalsParams tp, float2* grid, GridPrep gp) {
+__global__ void __launch_bounds__(128, 5) k_grid_totals(TotalsParams tp, float2* grid, GridPrep gp) {
     const int lane = threadIdx.x & 31;
     const int64_t gw = int64_t(blockIdx.x) * 4 + (threadIdx.x >> 5);
     const Geometry& g = tp.g;
@@ -759,7 +769,7 @@ __global__ void __launch_bounds__(128) k_grid_totals(TotalsParams tp, float2* gr
     // the patterns of the warp's pixels, and the nodes (of its rows r0 .. r1 - 1) with odd pixels: the
     // lanes' strips first, then the cells'
     PatternSet set;
-    bool odd_prev = false;
+    bool odd_prev = false, classes = false;
     for (int s = s0; s < s1; ++s) {
         bool odd = false;
         for (int k0 = 0; k0 < step; k0 += 4) {
@@ -773,7 +783,8 @@ __global__ void __launch_bounds__(128) k_grid_totals(TotalsParams tp, float2* gr
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 odd = odd || odd_pixel(bits[i]);
-                if ((bits[i] >> 8) & kPixDeviant) continue;
+                classes = classes || class_pixel(bits[i]);
+                if (deviant(bits[i])) continue;
                 set.add(bits[i] & 0xffu);
                 set.add((bits[i] >> 16) & 0xffu);
                 set.add(bits[i] >> 24);
@@ -789,12 +800,15 @@ __global__ void __launch_bounds__(128) k_grid_totals(TotalsParams tp, float2* gr
         if (l || r) tp.odd_nodes[atomicAdd(tp.odd_count, 1u)] = int32_t(int64_t(s) * g.nodes_x + c0 + lane);
     }
     set.unite_warp();
+    classes = __any_sync(0xffffffffu, classes);
     // column factors (in units of 1 / step) of the cell's left and right node
     const uint32_t il = uint32_t(step - col), ir = uint32_t(col);
     const float fl = float(il) * inv_step, fr = float(ir) * inv_step;
     bool store_only = tp.fresh != 0;  // the grid is still zero: write instead of add
-    for (uint32_t P = set.pop(); P != 0u; P = set.pop()) {
-        const bool pix = (P & RPD_SAMPLE_PIXEL_VALID) != 0;
+    // one walk over the strips for pattern P, or for class cls of the deviant pixels (P: that class alone)
+    auto walk = [&](auto by_class, uint32_t P, int cls) {
+        constexpr bool kByClass = decltype(by_class)::value;
+        const bool pix = kByClass || (P & RPD_SAMPLE_PIXEL_VALID) != 0;
         // the column's part of the next node row's totals: weights, squared weights, y, y^2
         uint32_t nw = 0u;
         unsigned long long nw2 = 0ull;
@@ -814,24 +828,34 @@ __global__ void __launch_bounds__(128) k_grid_totals(TotalsParams tp, float2* gr
                 for (int k0 = hs * half; k0 < (hs + 1) * half; k0 += 4) {
                     float4 A[4];
                     float2 B[4];
+                    auto read = [&](auto load) {
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const int y = s * step + k0 + i;
-                        const int64_t p = int64_t(y) * g.w + x;
-                        A[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                        B[i] = make_float2(0.0f, 0.0f);
-                        if (k0 + i < (hs + 1) * half && xin && y < g.h && inside(p)) {
+                        for (int i = 0; i < 4; ++i) {
+                            const int y = s * step + k0 + i;
+                            const int64_t p = int64_t(y) * g.w + x;
+                            A[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                            B[i] = make_float2(0.0f, 0.0f);
+                            if (k0 + i < (hs + 1) * half && xin && y < g.h && inside(p)) load(i, p);
+                        }
+                    };
+                    if constexpr (!kByClass) {
+                        read([&](int i, int64_t p) {
                             A[i] = gp.pat4[p];
                             B[i] = gp.pat2[p];
-                        }
+                        });
+                    } else {
+                        read([&](int i, int64_t p) {
+                            A[i] = make_float4(gp.cls[cls][0][p], gp.cls[cls][1][p], gp.cls[cls][2][p], gp.cls[cls][3][p]);
+                            B[i] = make_float2(gp.cls[cls][4][p], gp.pat2[p].y);
+                        });
                     }
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         const uint32_t bits = __float_as_uint(B[i].y);
-                        if ((bits >> 8) & kPixDeviant) continue;
+                        if (kByClass ? !class_pixel(bits) : deviant(bits)) continue;
                         float4 a = A[i];
                         float s2l = B[i].x;
-                        if ((bits & 0xffu) != P) {
+                        if (!kByClass && (bits & 0xffu) != P) {
                             const int more = ((bits >> 16) & 0xffu) == P ? 0 : (bits >> 24) == P ? 1 : -1;
                             if (more < 0) continue;
                             const int64_t p = int64_t(s * step + k0 + i) * g.w + x;
@@ -966,13 +990,21 @@ __global__ void __launch_bounds__(128) k_grid_totals(TotalsParams tp, float2* gr
             __syncwarp();
         }
         store_only = false;
-    }
+    };
+    for (uint32_t P = set.pop(); P != 0u; P = set.pop()) walk(std::false_type{}, P, 0);
+    if (!classes) return;
+#pragma unroll 1
+    for (int c = 0; c < kClasses; ++c) walk(std::true_type{}, class_bit(c), c);
 }
 
 // What k_grid_totals leaves out, one warp per node. It takes every sample of a pixel in the pixel's
 // nominal screen bin: a pixel some of whose samples may not be (a position within 2^-12 of the
 // pixel's end, or outside it) is looked over sample by sample here, and a sample that the reference
-// bins elsewhere is moved (very few are). Deviant pixels are summed class by class.
+// bins elsewhere is moved (very few are). Deviant pixels with random dimensions that lack a position
+// (sample_pixel) are its own altogether. A pattern at a time over all the samples, which enter every
+// class it holds. Where a node has many odd pixels (positions all over the place) the first pattern looked for is
+// the first pixel's first, and the others turn up meanwhile; where it has a few (seven in a 1920x1080x16 frame),
+// hardly any of their samples is to be moved, and a first walk only looks for patterns.
 // Blocks of one warp take the listed nodes in turn; each node is one warp's, in a fixed order.
 __device__ void odd_node(const GridParams& gpar, float2* grid, const DeviceSamples& s, const int64_t* offsets,
                          const GridPrep& gp, int64_t node, float* sm) {
@@ -992,7 +1024,6 @@ __device__ void odd_node(const GridParams& gpar, float2* grid, const DeviceSampl
     const int xlo = imaxs(0, (nx - 1) * step + 1), xhi = imins(g.w - 1, (nx + 1) * step - 1);
     const int ylo = imaxs(0, (ny - 1) * step + 1), yhi = imins(g.h - 1, (ny + 1) * step - 1);
     int nodd = 0;
-    bool deviants = false;
     // one row of 2 step - 1 pixels (or two, for steps up to 8) at a time
     const int lw = step <= 8 ? 16 : 32, rows = 32 / lw;
     const int lx = lane & (lw - 1), lr = lane / lw;
@@ -1000,7 +1031,7 @@ __device__ void odd_node(const GridParams& gpar, float2* grid, const DeviceSampl
     // latency per row (the grid's totals and screen bins of 1920x1080x16, where a block takes two nodes in turn:
     // 117 -> 108 us; 98 us with the odd pixels' samples spread over the lanes below)
     constexpr int kBatch = 8;
-    constexpr int kDeviantEntry = 0x8000;
+    constexpr int kSampleEntry = 0x8000;  // a sample_pixel
     const int x = xlo + lx;
     for (int yb = ylo; yb <= yhi; yb += rows * kBatch) {
         uint32_t bits[kBatch];
@@ -1014,19 +1045,16 @@ __device__ void odd_node(const GridParams& gpar, float2* grid, const DeviceSampl
 #pragma unroll
         for (int b = 0; b < kBatch; ++b) {
             const bool odd = odd_pixel(bits[b]);
-            const bool dev = ((bits[b] >> 8) & kPixDeviant) != 0;
-            deviants = deviants || dev;
             const unsigned m = __ballot_sync(0xffffffffu, odd);
-            if (odd) list[nodd + __popc(m & ((1u << lane) - 1))] = uint16_t((dev ? kDeviantEntry : 0) | ((yb + b * rows + lr - ylo) * 64 + x - xlo));
+            if (odd) list[nodd + __popc(m & ((1u << lane) - 1))] = uint16_t((sample_pixel(bits[b]) ? kSampleEntry : 0) | ((yb + b * rows + lr - ylo) * 64 + x - xlo));
             nodd += __popc(m);
         }
     }
     if (nodd == 0) return;
     __syncwarp();
-    deviants = __any_sync(0xffffffffu, deviants);
     auto pixel = [&](int i, int& x, int& y, int64_t& idx) {
         x = xlo + (list[i] & 63);
-        y = ylo + ((list[i] & (kDeviantEntry - 1)) >> 6);
+        y = ylo + ((list[i] & (kSampleEntry - 1)) >> 6);
         idx = int64_t(y) * g.w + x;
     };
     auto weight = [&](int x, int y) {
@@ -1040,28 +1068,25 @@ __device__ void odd_node(const GridParams& gpar, float2* grid, const DeviceSampl
     auto nominal_bin = [&](int x, int y) {
         return ((y - (ny - 1) * step) >> (sh - 1)) * 4 + ((x - (nx - 1) * step) >> (sh - 1));
     };
-    auto is_deviant = [&](int i) { return (list[i] & kDeviantEntry) != 0; };
-    // f(x, y, k) for every sample k of the odd pixels that are not deviant: a uniform push's pixels and samples
-    // are one range over the lanes
     const bool has_pu = s.compact ? s.c16.pixel_u[0] && s.c16.pixel_u[1] : s.pixel_u[0] && s.pixel_u[1];
+    // f(x, y, k, own) for every sample k of the odd pixels (own: of a sample_pixel): a uniform push's pixels and
+    // samples are one range over the lanes
     auto for_samples = [&](auto f) {
-        if (!has_pu) return;  // no sample has a screen position
         int x, y;
         int64_t idx;
         if (gpar.spp > 0) {
             for (int t = lane; t < nodd * gpar.spp; t += 32) {
                 const int i = t / gpar.spp;
-                if (is_deviant(i)) continue;
                 pixel(i, x, y, idx);
-                f(x, y, (idx - gpar.first) * gpar.spp + (t - i * gpar.spp));
+                f(x, y, (idx - gpar.first) * gpar.spp + (t - i * gpar.spp), (list[i] & kSampleEntry) != 0);
             }
             return;
         }
         for (int i = 0; i < nodd; ++i) {
-            if (is_deviant(i)) continue;
             pixel(i, x, y, idx);
+            const bool own = (list[i] & kSampleEntry) != 0;
             const int64_t kend = offsets[idx - gpar.first + 1];
-            for (int64_t k = offsets[idx - gpar.first] + lane; k < kend; k += 32) f(x, y, k);
+            for (int64_t k = offsets[idx - gpar.first] + lane; k < kend; k += 32) f(x, y, k, own);
         }
     };
     auto pattern_of = [](uint32_t key) {
@@ -1071,71 +1096,72 @@ __device__ void odd_node(const GridParams& gpar, float2* grid, const DeviceSampl
             if (!(key & key_absent_bit(c))) p |= class_bit(c);
         return p;
     };
-    // the patterns of the samples to move
-    PatternSet set;
-    for_samples([&](int x, int y, int64_t k) {
-        const uint32_t key = gp.key[k];
-        const int b = exact_bin(x, y, k);
-        if (!(key & key_absent_bit(0)) && b != nominal_bin(x, y)) set.add(pattern_of(key));
-    });
-    set.unite_warp();
-    for (uint32_t P = set.pop(); P != 0u; P = set.pop()) {
+    // is the sample one for the sums below? b: its bin
+    auto counts = [&](uint32_t key, int x, int y, int b, bool own) {
+        return own ? key != kKeyNone : !(key & key_absent_bit(0)) && b != nominal_bin(x, y);
+    };
+    PatternSet others;
+    uint32_t P;
+    const bool many = 8 * nodd > (xhi - xlo + 1) * (yhi - ylo + 1);  // more than an eighth of its pixels
+    if (many) {
+        int px, py;
+        int64_t idx;
+        pixel(0, px, py, idx);
+        P = __float_as_uint(gp.pat2[idx].y) & 0xffu;
+    } else {
+        for_samples([&](int x, int y, int64_t k, bool own) {
+            const uint32_t key = gp.key[k];
+            const int b = has_pu ? exact_bin(x, y, k) : 0;
+            if (counts(key, x, y, b, own)) others.add(pattern_of(key));
+        });
+        others.unite_warp();
+        P = others.pop();
+    }
+    for (bool gather = many; P != 0u; gather = false) {
+        Totals own_totals;
         bins.clear();
         __syncwarp();
-        for_samples([&](int x, int y, int64_t k) {
+        for_samples([&](int x, int y, int64_t k, bool own) {
             const uint32_t key = gp.key[k];
             const float yv = gp.lum[k];
-            const int b = exact_bin(x, y, k), b0 = nominal_bin(x, y);
-            if ((key & key_absent_bit(0)) || b == b0 || pattern_of(key) != P) return;
-            const float w = weight(x, y);
-            bins.add_weight(b, w, 1.0f);
-            bins.add_sum(b, w, yv, 0.0f);
-            bins.add_weight(b0, -w, 1.0f);
-            bins.add_sum(b0, -w, yv, 0.0f);
-        });
-        const float2 v = bins.reduce_value();
-        if (v.x == 0.0f && v.y == 0.0f) continue;
-#pragma unroll
-        for (int c = 0; c < kClasses; ++c)
-            if (P & class_bit(c)) df_accum(base + dep_screen(c) * kDepStride + lane, v.x, v.y);
-    }
-    __syncwarp();
-    if (!deviants) return;
-    for (int c = 0; c < kClasses; ++c) {
-        const uint32_t absent = key_absent_bit(c) | key_absent_bit(0);
-        Totals tx, ts;
-        bins.clear();
-        __syncwarp();
-        for (int i = 0; i < nodd; ++i) {
-            int x, y;
-            int64_t idx;
-            pixel(i, x, y, idx);
-            const PixPattern pp = load_pattern(gp, idx);
-            if (!(pp.pf & kPixDeviant)) continue;
-            float cs[5];
-            class_sums(gp, c, idx, pp, cs);
-            if (cs[0] == 0.0f) continue;
-            const float w = weight(x, y);
-            const bool mixed = c > 0 && (pp.pf & kPixMixed);
-            if (lane == 0) {
-                add_class(tx, w, cs[0], cs[1], cs[2], cs[3], cs[4]);
-                if (!mixed) add_class(ts, w, cs[0], cs[1], cs[2], cs[3], cs[4]);
+            const int b = has_pu ? exact_bin(x, y, k) : 0;
+            if (!counts(key, x, y, b, own)) return;
+            const uint32_t pat = pattern_of(key);
+            if (pat != P) {
+                if (gather) others.add(pat);
+                return;
             }
-            const int64_t local = idx - gpar.first, kend = sample_offset(offsets, gpar.spp, local + 1);
-            for (int64_t k = sample_offset(offsets, gpar.spp, local) + lane; k < kend; k += 32) {
-                const uint32_t key = gp.key[k];
-                if (key & absent) continue;
-                const float yv = gp.lum[k];
-                const int b = exact_bin(x, y, k);
+            const float w = weight(x, y);
+            if (!(key & key_absent_bit(0))) {
                 bins.add_weight(b, w, 1.0f);
                 bins.add_sum(b, w, yv, 0.0f);
-                if (mixed) add_sample(ts, w, yv);
+            }
+            if (own) {
+                add_sample(own_totals, w, yv);
+            } else {
+                const int b0 = nominal_bin(x, y);
+                bins.add_weight(b0, -w, 1.0f);
+                bins.add_sum(b0, -w, yv, 0.0f);
+            }
+        });
+        const bool pix = (P & RPD_SAMPLE_PIXEL_VALID) != 0;
+        const float2 v = bins.reduce_value();
+        float2 t[4];
+        reduce_totals(own_totals, t);
+#pragma unroll
+        for (int c = 0; c < kClasses; ++c) {
+            if (!(P & class_bit(c))) continue;
+            if (pix && (v.x != 0.0f || v.y != 0.0f)) df_accum(base + dep_screen(c) * kDepStride + lane, v.x, v.y);
+            if (lane != 0) continue;
+            for (int q = 0; q < 4; ++q) {
+                if (t[q].x == 0.0f && t[q].y == 0.0f) continue;
+                if (pix) df_accum(base + dep_screen(c) * kDepStride + 32 + q, t[q].x, t[q].y);
+                if (c > 0) df_accum(base + dep_random(c) * kDepStride + 32 + q, t[q].x, t[q].y);
             }
         }
-        const float2 v = bins.reduce_value();
-        if (v.x != 0.0f || v.y != 0.0f) df_accum(base + dep_screen(c) * kDepStride + lane, v.x, v.y);
-        reduce_totals_into(ts, base + dep_screen(c) * kDepStride);
-        if (c > 0) reduce_totals_into(tx, base + dep_random(c) * kDepStride);
+        __syncwarp();
+        if (gather) others.unite_warp();
+        P = others.pop();
     }
 }
 
