@@ -436,9 +436,13 @@ template <typename Acc>
 __device__ __forceinline__ void store_classes(const Acc& a, const GridPrep& gp, int64_t idx, uint8_t pflags) {
     const PatternSums& p0 = a.pt[0];
     gp.pat4[idx] = make_float4(p0.c, p0.s1h, p0.s1l, p0.s2h);
-    uint32_t bits = p0.pat | (uint32_t(pflags | (a.dev ? kPixDeviant : 0)) << 8);
+    uint32_t bits = p0.pat | (uint32_t(pflags) << 8);
     if (!a.dev) {
         for (int k = 1; k < kPatterns; ++k) bits |= a.pt[k].pat << (8 * (k + 1));
+    } else {
+        const uint32_t pats = p0.pat | a.pt[1].pat | a.pt[2].pat;
+        const bool placed = (pats & class_bit(0)) || a.cs[0] > 0.0f;
+        bits |= uint32_t(kPixDeviant | (placed ? kPixPlaced : 0)) << 8;
     }
     gp.pat2[idx] = make_float2(p0.s2l, __uint_as_float(bits));
     if (!a.dev) {

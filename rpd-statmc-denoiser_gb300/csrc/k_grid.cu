@@ -672,8 +672,8 @@ __global__ void __launch_bounds__(32) k_grid_screen(GridParams gpar, float2* pas
 // registers instead of lane-private bins in shared memory; warps are independent of each other.
 // A validity pattern at a time: its sums enter every class it holds. Then, where some pixel holds more patterns than
 // the statistics pass keeps (deviant), a class at a time over the class sums of such pixels. Samples outside
-// their pixel's nominal bin, and deviant pixels some of whose samples lack the position, are
-// k_grid_odd's. The bound is load latency (20 warps per SM, one pass over 24 bytes a pixel): with
+// their pixel's nominal bin, and those of deviant pixels that lack the position, are put right by
+// k_grid_odd. The bound is load latency (20 warps per SM, one pass over 24 bytes a pixel): with
 // k_grid_odd 0.100 ms at 1920x1080x16 against 0.213 ms for the pattern form; where a pixel's samples
 // hold three patterns, 0.28 against 0.82 ms, eight patterns 0.54 against 1.01 ms (29 ms with every deviant
 // pixel left to k_grid_odd, class by class and sample by sample).
@@ -693,18 +693,21 @@ struct TotalsParams {
 __host__ __device__ constexpr int dep_random(int c) { return c == 0 ? 0 : 2 * c - 1; }
 __host__ __device__ constexpr int dep_screen(int c) { return 2 * c; }
 
-// Of a pixel with these bits (pat2.y): is it deviant, and are its class sums the screen's too (every sample
-// with a random dimension has a position)? Then k_grid_totals takes it class by class, else
-// k_grid_odd sample by sample.
-constexpr uint32_t kDeviantBit = uint32_t(kPixDeviant) << 8, kMixedBit = uint32_t(kPixMixed) << 8;
+// Of a pixel with these bits (pat2.y). Deviant: its class sums stand for the screen's too, but for samples with
+// a random dimension and no position (mixed). k_grid_odd takes those out again, unless the pixel has no
+// others (unplaced): then its class sums are for the random dimensions alone.
+constexpr uint32_t kDeviantBit = uint32_t(kPixDeviant) << 8, kMixedBit = uint32_t(kPixMixed) << 8,
+                   kPlacedBit = uint32_t(kPixPlaced) << 8;
 __device__ __forceinline__ bool deviant(uint32_t bits) { return bits & kDeviantBit; }
-__device__ __forceinline__ bool class_pixel(uint32_t bits) { return (bits & (kDeviantBit | kMixedBit)) == kDeviantBit; }
-__device__ __forceinline__ bool sample_pixel(uint32_t bits) {
-    return (bits & (kDeviantBit | kMixedBit)) == (kDeviantBit | kMixedBit);
+__device__ __forceinline__ bool unplaced_pixel(uint32_t bits) {
+    return (bits & (kDeviantBit | kMixedBit | kPlacedBit)) == (kDeviantBit | kMixedBit);
+}
+__device__ __forceinline__ bool mixed_deviant(uint32_t bits) {
+    return (bits & (kDeviantBit | kMixedBit | kPlacedBit)) == (kDeviantBit | kMixedBit | kPlacedBit);
 }
 // Does k_grid_odd look at the pixel? (Only a sample with a position makes a pixel not uniform.)
 __device__ __forceinline__ bool odd_pixel(uint32_t bits) {
-    return !(bits & (uint32_t(kPixUniform) << 8)) || sample_pixel(bits);
+    return !(bits & (uint32_t(kPixUniform) << 8)) || mixed_deviant(bits);
 }
 
 // A set of patterns, one bit each (patterns are even: bit p / 2).
@@ -769,7 +772,7 @@ __global__ void __launch_bounds__(128, 5) k_grid_totals(TotalsParams tp, float2*
     // the patterns of the warp's pixels, and the nodes (of its rows r0 .. r1 - 1) with odd pixels: the
     // lanes' strips first, then the cells'
     PatternSet set;
-    bool odd_prev = false, classes = false;
+    bool odd_prev = false, classes = false, unplaced = false;
     for (int s = s0; s < s1; ++s) {
         bool odd = false;
         for (int k0 = 0; k0 < step; k0 += 4) {
@@ -783,7 +786,8 @@ __global__ void __launch_bounds__(128, 5) k_grid_totals(TotalsParams tp, float2*
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 odd = odd || odd_pixel(bits[i]);
-                classes = classes || class_pixel(bits[i]);
+                unplaced = unplaced || unplaced_pixel(bits[i]);
+                classes = classes || (deviant(bits[i]) && !unplaced_pixel(bits[i]));
                 if (deviant(bits[i])) continue;
                 set.add(bits[i] & 0xffu);
                 set.add((bits[i] >> 16) & 0xffu);
@@ -801,14 +805,15 @@ __global__ void __launch_bounds__(128, 5) k_grid_totals(TotalsParams tp, float2*
     }
     set.unite_warp();
     classes = __any_sync(0xffffffffu, classes);
+    unplaced = __any_sync(0xffffffffu, unplaced);
     // column factors (in units of 1 / step) of the cell's left and right node
     const uint32_t il = uint32_t(step - col), ir = uint32_t(col);
     const float fl = float(il) * inv_step, fr = float(ir) * inv_step;
     bool store_only = tp.fresh != 0;  // the grid is still zero: write instead of add
-    // one walk over the strips for pattern P, or for class cls of the deviant pixels (P: that class alone)
-    auto walk = [&](auto by_class, uint32_t P, int cls) {
+    // one walk over the strips for pattern P, or for class cls (P: that class alone) of the deviant pixels, unplaced
+    // ones or the others; pix: with the screen's sums
+    auto walk = [&](auto by_class, uint32_t P, int cls, bool pix) {
         constexpr bool kByClass = decltype(by_class)::value;
-        const bool pix = kByClass || (P & RPD_SAMPLE_PIXEL_VALID) != 0;
         // the column's part of the next node row's totals: weights, squared weights, y, y^2
         uint32_t nw = 0u;
         unsigned long long nw2 = 0ull;
@@ -852,7 +857,7 @@ __global__ void __launch_bounds__(128, 5) k_grid_totals(TotalsParams tp, float2*
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         const uint32_t bits = __float_as_uint(B[i].y);
-                        if (kByClass ? !class_pixel(bits) : deviant(bits)) continue;
+                        if (kByClass ? !deviant(bits) || unplaced_pixel(bits) == pix : deviant(bits)) continue;
                         float4 a = A[i];
                         float s2l = B[i].x;
                         if (!kByClass && (bits & 0xffu) != P) {
@@ -991,21 +996,29 @@ __global__ void __launch_bounds__(128, 5) k_grid_totals(TotalsParams tp, float2*
         }
         store_only = false;
     };
-    for (uint32_t P = set.pop(); P != 0u; P = set.pop()) walk(std::false_type{}, P, 0);
-    if (!classes) return;
+    for (uint32_t P = set.pop(); P != 0u; P = set.pop()) walk(std::false_type{}, P, 0, (P & RPD_SAMPLE_PIXEL_VALID) != 0);
+    if (!classes && !unplaced) return;
 #pragma unroll 1
-    for (int c = 0; c < kClasses; ++c) walk(std::true_type{}, class_bit(c), c);
+    for (int c = classes ? 0 : kClasses; c < 2 * kClasses; ++c) {
+        if (c == kClasses && !unplaced) return;
+        if (c != kClasses) walk(std::true_type{}, class_bit(c % kClasses), c % kClasses, c < kClasses);  // (class 0 is the screen)
+    }
 }
 
 // What k_grid_totals leaves out, one warp per node. It takes every sample of a pixel in the pixel's
 // nominal screen bin: a pixel some of whose samples may not be (a position within 2^-12 of the
 // pixel's end, or outside it) is looked over sample by sample here, and a sample that the reference
-// bins elsewhere is moved (very few are). Deviant pixels with random dimensions that lack a position
-// (sample_pixel) are its own altogether. A pattern at a time over all the samples, which enter every
-// class it holds. Where a node has many odd pixels (positions all over the place) the first pattern looked for is
-// the first pixel's first, and the others turn up meanwhile; where it has a few (seven in a 1920x1080x16 frame),
-// hardly any of their samples is to be moved, and a first walk only looks for patterns.
+// bins elsewhere is moved (very few are). A deviant pixel's samples that lack the position are taken out
+// of the screen's sums. A pattern at a time, whose samples enter every class it holds. Where a node has many odd
+// pixels (positions all over the place) the first pattern looked for is the first pixel's first, and the
+// others turn up meanwhile; where it has a few (seven in a 1920x1080x16 frame), hardly any of their samples count, and
+// a first walk notes the patterns and, up to kOddPicks of them, the samples.
 // Blocks of one warp take the listed nodes in turn; each node is one warp's, in a fixed order.
+constexpr int kOddPicks = 256;
+struct OddPicks {
+    int64_t sample[kOddPicks];
+    uint16_t pixel[kOddPicks];
+};
 __device__ void odd_node(const GridParams& gpar, float2* grid, const DeviceSamples& s, const int64_t* offsets,
                          const GridPrep& gp, int64_t node, float* sm) {
     const int lane = threadIdx.x;
@@ -1014,7 +1027,8 @@ __device__ void odd_node(const GridParams& gpar, float2* grid, const DeviceSampl
     const int step = g.step, sh = __ffs(step) - 1;
     const float wscale = float(step) * float(step), inv_wscale = 1.0f / wscale;
     LaneBins<false> bins{sm, lane, wscale};
-    uint16_t* list = reinterpret_cast<uint16_t*>(sm + LaneBins<false>::kSlots * 32);
+    OddPicks& picks = *reinterpret_cast<OddPicks*>(sm + LaneBins<false>::kSlots * 32);
+    uint16_t* list = reinterpret_cast<uint16_t*>(&picks + 1);
     float2* base = grid + node * kDeps * kDepStride;
     const float support = float(g.support);
     const float half_support = 0.5f * support;
@@ -1031,7 +1045,7 @@ __device__ void odd_node(const GridParams& gpar, float2* grid, const DeviceSampl
     // latency per row (the grid's totals and screen bins of 1920x1080x16, where a block takes two nodes in turn:
     // 117 -> 108 us; 98 us with the odd pixels' samples spread over the lanes below)
     constexpr int kBatch = 8;
-    constexpr int kSampleEntry = 0x8000;  // a sample_pixel
+    constexpr int kMixedEntry = 0x8000;  // a mixed_deviant
     const int x = xlo + lx;
     for (int yb = ylo; yb <= yhi; yb += rows * kBatch) {
         uint32_t bits[kBatch];
@@ -1046,7 +1060,7 @@ __device__ void odd_node(const GridParams& gpar, float2* grid, const DeviceSampl
         for (int b = 0; b < kBatch; ++b) {
             const bool odd = odd_pixel(bits[b]);
             const unsigned m = __ballot_sync(0xffffffffu, odd);
-            if (odd) list[nodd + __popc(m & ((1u << lane) - 1))] = uint16_t((sample_pixel(bits[b]) ? kSampleEntry : 0) | ((yb + b * rows + lr - ylo) * 64 + x - xlo));
+            if (odd) list[nodd + __popc(m & ((1u << lane) - 1))] = uint16_t((mixed_deviant(bits[b]) ? kMixedEntry : 0) | ((yb + b * rows + lr - ylo) * 64 + x - xlo));
             nodd += __popc(m);
         }
     }
@@ -1054,7 +1068,7 @@ __device__ void odd_node(const GridParams& gpar, float2* grid, const DeviceSampl
     __syncwarp();
     auto pixel = [&](int i, int& x, int& y, int64_t& idx) {
         x = xlo + (list[i] & 63);
-        y = ylo + ((list[i] & (kSampleEntry - 1)) >> 6);
+        y = ylo + ((list[i] & (kMixedEntry - 1)) >> 6);
         idx = int64_t(y) * g.w + x;
     };
     auto weight = [&](int x, int y) {
@@ -1069,24 +1083,27 @@ __device__ void odd_node(const GridParams& gpar, float2* grid, const DeviceSampl
         return ((y - (ny - 1) * step) >> (sh - 1)) * 4 + ((x - (nx - 1) * step) >> (sh - 1));
     };
     const bool has_pu = s.compact ? s.c16.pixel_u[0] && s.c16.pixel_u[1] : s.pixel_u[0] && s.pixel_u[1];
-    // f(x, y, k, own) for every sample k of the odd pixels (own: of a sample_pixel): a uniform push's pixels and
-    // samples are one range over the lanes
+    // f(ok, i, x, y, k) for every sample k of the odd pixels (i: the pixel's list entry), the lanes in step (ok: the
+    // lane has one; else k is some sample): a uniform push's pixels and samples are one range over the lanes,
+    // with per-pixel counts eight lanes take a pixel
     auto for_samples = [&](auto f) {
         int x, y;
         int64_t idx;
         if (gpar.spp > 0) {
-            for (int t = lane; t < nodd * gpar.spp; t += 32) {
-                const int i = t / gpar.spp;
+            const int total = nodd * gpar.spp;
+            for (int t0 = 0; t0 < total; t0 += 32) {
+                const int t = imins(t0 + lane, total - 1), i = t / gpar.spp;
                 pixel(i, x, y, idx);
-                f(x, y, (idx - gpar.first) * gpar.spp + (t - i * gpar.spp), (list[i] & kSampleEntry) != 0);
+                f(t0 + lane < total, i, x, y, (idx - gpar.first) * gpar.spp + (t - i * gpar.spp));
             }
             return;
         }
-        for (int i = 0; i < nodd; ++i) {
+        for (int i0 = 0; i0 < nodd; i0 += 4) {
+            const int i = imins(i0 + (lane >> 3), nodd - 1);
             pixel(i, x, y, idx);
-            const bool own = (list[i] & kSampleEntry) != 0;
-            const int64_t kend = offsets[idx - gpar.first + 1];
-            for (int64_t k = offsets[idx - gpar.first] + lane; k < kend; k += 32) f(x, y, k, own);
+            const int64_t kend = i0 + (lane >> 3) < nodd ? offsets[idx - gpar.first + 1] : 0;
+            for (int64_t k = offsets[idx - gpar.first] + (lane & 7); __any_sync(0xffffffffu, k < kend); k += 8)
+                f(k < kend, i, x, y, k < kend ? k : 0);
         }
     };
     auto pattern_of = [](uint32_t key) {
@@ -1096,12 +1113,13 @@ __device__ void odd_node(const GridParams& gpar, float2* grid, const DeviceSampl
             if (!(key & key_absent_bit(c))) p |= class_bit(c);
         return p;
     };
-    // is the sample one for the sums below? b: its bin
-    auto counts = [&](uint32_t key, int x, int y, int b, bool own) {
-        return own ? key != kKeyNone : !(key & key_absent_bit(0)) && b != nominal_bin(x, y);
+    // is pixel i's sample one for the sums below? (b: its bin; without a pixel_u plane no key says that there is one)
+    auto counts = [&](uint32_t key, int i, int x, int y, int b) {
+        return key & key_absent_bit(0) ? key != kKeyNone && (list[i] & kMixedEntry) : b != nominal_bin(x, y);
     };
     PatternSet others;
     uint32_t P;
+    int found = 0;
     const bool many = 8 * nodd > (xhi - xlo + 1) * (yhi - ylo + 1);  // more than an eighth of its pixels
     if (many) {
         int px, py;
@@ -1109,55 +1127,73 @@ __device__ void odd_node(const GridParams& gpar, float2* grid, const DeviceSampl
         pixel(0, px, py, idx);
         P = __float_as_uint(gp.pat2[idx].y) & 0xffu;
     } else {
-        for_samples([&](int x, int y, int64_t k, bool own) {
+        for_samples([&](bool ok, int i, int x, int y, int64_t k) {
             const uint32_t key = gp.key[k];
             const int b = has_pu ? exact_bin(x, y, k) : 0;
-            if (counts(key, x, y, b, own)) others.add(pattern_of(key));
+            const bool pick = ok && counts(key, i, x, y, b);
+            const unsigned m = __ballot_sync(0xffffffffu, pick);
+            if (m == 0u) return;
+            if (pick) {
+                others.add(pattern_of(key));
+                const int at = found + __popc(m & ((1u << lane) - 1));
+                if (at < kOddPicks) {
+                    picks.sample[at] = k;
+                    picks.pixel[at] = uint16_t(i);
+                }
+            }
+            found += __popc(m);
         });
         others.unite_warp();
         P = others.pop();
+        __syncwarp();
     }
     for (bool gather = many; P != 0u; gather = false) {
-        Totals own_totals;
+        Totals lost;
         bins.clear();
         __syncwarp();
-        for_samples([&](int x, int y, int64_t k, bool own) {
+        auto add = [&](bool ok, int i, int x, int y, int64_t k) {
             const uint32_t key = gp.key[k];
             const float yv = gp.lum[k];
             const int b = has_pu ? exact_bin(x, y, k) : 0;
-            if (!counts(key, x, y, b, own)) return;
+            if (!ok || !counts(key, i, x, y, b)) return;
             const uint32_t pat = pattern_of(key);
             if (pat != P) {
                 if (gather) others.add(pat);
                 return;
             }
             const float w = weight(x, y);
-            if (!(key & key_absent_bit(0))) {
+            const int b0 = nominal_bin(x, y);
+            bins.add_weight(b0, -w, 1.0f);
+            bins.add_sum(b0, -w, yv, 0.0f);
+            if (key & key_absent_bit(0)) {
+                add_sample(lost, w, yv);
+            } else {
                 bins.add_weight(b, w, 1.0f);
                 bins.add_sum(b, w, yv, 0.0f);
             }
-            if (own) {
-                add_sample(own_totals, w, yv);
-            } else {
-                const int b0 = nominal_bin(x, y);
-                bins.add_weight(b0, -w, 1.0f);
-                bins.add_sum(b0, -w, yv, 0.0f);
+        };
+        if (many || found > kOddPicks) {
+            for_samples(add);
+        } else {
+            for (int e = lane; e < found; e += 32) {
+                int x, y;
+                int64_t idx;
+                const int i = picks.pixel[e];
+                pixel(i, x, y, idx);
+                add(true, i, x, y, picks.sample[e]);
             }
-        });
-        const bool pix = (P & RPD_SAMPLE_PIXEL_VALID) != 0;
+        }
         const float2 v = bins.reduce_value();
         float2 t[4];
-        reduce_totals(own_totals, t);
+        reduce_totals(lost, t);  // zeros for a pattern with the position
 #pragma unroll
         for (int c = 0; c < kClasses; ++c) {
             if (!(P & class_bit(c))) continue;
-            if (pix && (v.x != 0.0f || v.y != 0.0f)) df_accum(base + dep_screen(c) * kDepStride + lane, v.x, v.y);
+            float2* e = base + dep_screen(c) * kDepStride;
+            if (v.x != 0.0f || v.y != 0.0f) df_accum(e + lane, v.x, v.y);
             if (lane != 0) continue;
-            for (int q = 0; q < 4; ++q) {
-                if (t[q].x == 0.0f && t[q].y == 0.0f) continue;
-                if (pix) df_accum(base + dep_screen(c) * kDepStride + 32 + q, t[q].x, t[q].y);
-                if (c > 0) df_accum(base + dep_random(c) * kDepStride + 32 + q, t[q].x, t[q].y);
-            }
+            for (int q = 0; q < 4; ++q)
+                if (t[q].x != 0.0f || t[q].y != 0.0f) df_accum(e + 32 + q, -t[q].x, -t[q].y);
         }
         __syncwarp();
         if (gather) others.unite_warp();
@@ -2207,7 +2243,7 @@ cudaError_t launch_grid_fast(Job& j, const DeviceSamples& s, int64_t first, int6
             const int64_t warps = int64_t(tp.col_warps) * ((ny1 - ny0 + tp.len - 1) / tp.len);
             k_grid_totals<<<unsigned((warps + 3) / 4), 128, 0, j.stream>>>(tp, target, gp);
             if ((e = cudaGetLastError()) != cudaSuccess) return e;
-            const size_t smem = size_t(LaneBins<false>::kSlots) * 32 * sizeof(float) + size_t(4) * step * step * sizeof(uint16_t);
+            const size_t smem = size_t(LaneBins<false>::kSlots) * 32 * sizeof(float) + sizeof(OddPicks) + size_t(4) * step * step * sizeof(uint16_t);
             const unsigned odd_blocks = std::min<unsigned>(nblocks, unsigned(kStripSms) * 16);
             k_grid_odd<<<odd_blocks, 32, smem, j.stream>>>(gpar, target, s, j.offsets, gp, odd_count, odd_nodes);
             j.launches += 2;

@@ -274,6 +274,7 @@ struct DeviceSamples {           // rpd_sample_soa with pointers in HBM
 constexpr uint8_t kPixUniform = 0x1;  // every sample lies in its pixel's screen bin, at every node
 constexpr uint8_t kPixMixed = 0x2;    // some sample has a random dimension but no screen position
 constexpr uint8_t kPixDeviant = 0x4;  // the pixel's samples have more than kPatterns validity patterns
+constexpr uint8_t kPixPlaced = 0x8;   // (set where kPixDeviant is) some sample has the screen position
 constexpr float kUniformMax = 1.0f - 1.0f / 4096.0f;  // largest in-pixel offset of a uniform pixel
 __host__ __device__ constexpr uint8_t class_bit(int c) {
     return c == 0 ? RPD_SAMPLE_PIXEL_VALID : c == 1 ? RPD_SAMPLE_BRDF_VALID : c == 2 ? RPD_SAMPLE_LENS_VALID
