@@ -666,11 +666,12 @@ __global__ void __launch_bounds__(32) k_grid_screen(GridParams gpar, float2* pas
 // once more for the cell that neighbouring warps share) instead of once per node it supports, in
 // registers instead of lane-private bins in shared memory; warps are independent of each other.
 // A validity pattern at a time: its sums enter every class it holds. Then, where some pixel holds more patterns than
-// the statistics pass keeps (deviant), a class at a time over the class sums of such pixels. Samples outside
+// the statistics pass keeps (deviant), a class at a time over the class sums of such pixels; where there are
+// many patterns, a class at a time over all pixels. Samples outside
 // their pixel's nominal bin, and those of deviant pixels that lack the position, are put right by
 // k_grid_odd. The bound is load latency (20 warps per SM, one pass over 24 bytes a pixel): with
 // k_grid_odd 0.100 ms at 1920x1080x16 against 0.213 ms for the pattern form; where a pixel's samples
-// hold three patterns, 0.28 against 0.82 ms, eight patterns 0.54 against 1.01 ms (29 ms with every deviant
+// hold three patterns, 0.28 against 0.82 ms, eight patterns 0.50 against 1.01 ms (29 ms with every deviant
 // pixel left to k_grid_odd, class by class and sample by sample).
 struct TotalsParams {
     Geometry g;
@@ -680,6 +681,8 @@ struct TotalsParams {
     int col_warps;   // warps per `len` node rows
     int sh;          // log2 of the node step
     int fresh;       // the grid holds zeros (the frame's first push)
+    int parts;       // warps that share a strip's classes
+    int many;        // walks from which on the classes are walked instead of the patterns
     // the nodes with work for k_grid_odd: how many, and their indices
     unsigned* odd_count;
     int32_t* odd_nodes;
@@ -747,7 +750,8 @@ __device__ __forceinline__ DF df_scaled(float a, DF b) {  // a * b
 
 __global__ void __launch_bounds__(128, 5) k_grid_totals(TotalsParams tp, float2* grid, GridPrep gp) {
     const int lane = threadIdx.x & 31;
-    const int64_t gw = int64_t(blockIdx.x) * 4 + (threadIdx.x >> 5);
+    const int64_t warp = int64_t(blockIdx.x) * 4 + (threadIdx.x >> 5), gw = warp / tp.parts;
+    const int part = int(warp - gw * tp.parts);
     const Geometry& g = tp.g;
     const int sh = tp.sh, step = g.step, half = step >> 1;
     const int r0 = tp.ny0 + int(gw / tp.col_warps) * tp.len;
@@ -767,7 +771,7 @@ __global__ void __launch_bounds__(128, 5) k_grid_totals(TotalsParams tp, float2*
     // the patterns of the warp's pixels, and the nodes (of its rows r0 .. r1 - 1) with odd pixels: the
     // lanes' strips first, then the cells'
     PatternSet set;
-    bool odd_prev = false, classes = false, unplaced = false;
+    bool odd_prev = false, classes = false, unplaced = false, mixed = false;
     for (int s = s0; s < s1; ++s) {
         bool odd = false;
         for (int k0 = 0; k0 < step; k0 += 4) {
@@ -781,6 +785,7 @@ __global__ void __launch_bounds__(128, 5) k_grid_totals(TotalsParams tp, float2*
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 odd = odd || odd_pixel(bits[i]);
+                mixed = mixed || (bits[i] & kMixedBit);
                 unplaced = unplaced || unplaced_pixel(bits[i]);
                 classes = classes || (deviant(bits[i]) && !unplaced_pixel(bits[i]));
                 if (deviant(bits[i])) continue;
@@ -791,7 +796,7 @@ __global__ void __launch_bounds__(128, 5) k_grid_totals(TotalsParams tp, float2*
         }
         const unsigned m = __ballot_sync(0xffffffffu, odd || odd_prev);  // strips s - 1 and s: node row s
         odd_prev = odd;
-        if (s < r0 || m == 0u || lane > cells || !owned(lane)) continue;
+        if (part > 0 || s < r0 || m == 0u || lane > cells || !owned(lane)) continue;
         // node `lane`: the cells on its left and right
         const unsigned cell_lanes = cells == 1 ? 0xffffffffu : (1u << step) - 1u;
         const bool l = lane > 0 && ((m >> ((lane - 1) << sh)) & cell_lanes);
@@ -801,14 +806,17 @@ __global__ void __launch_bounds__(128, 5) k_grid_totals(TotalsParams tp, float2*
     set.unite_warp();
     classes = __any_sync(0xffffffffu, classes);
     unplaced = __any_sync(0xffffffffu, unplaced);
+    mixed = __any_sync(0xffffffffu, mixed);
     // column factors (in units of 1 / step) of the cell's left and right node
     const uint32_t il = uint32_t(step - col), ir = uint32_t(col);
     const float fl = float(il) * inv_step, fr = float(ir) * inv_step;
     bool store_only = tp.fresh != 0;  // the grid is still zero: write instead of add
-    // one walk over the strips for pattern P, or for class cls (P: that class alone) of the deviant pixels, unplaced
-    // ones or the others; pix: with the screen's sums
-    auto walk = [&](auto by_class, uint32_t P, int cls, bool pix) {
-        constexpr bool kByClass = decltype(by_class)::value;
+    // one walk over the strips for pattern P (kPattern), or for class cls (P: that class alone) of all pixels
+    // (kAll) or of the deviant ones (kDeviants: unplaced ones or the others); pix: with the screen's sums
+    constexpr int kPattern = 0, kDeviants = 1, kAll = 2;
+    auto walk = [&](auto mode, uint32_t P, int cls, bool pix) {
+        constexpr int kMode = decltype(mode)::value;
+        constexpr int kRows = kMode == kAll ? 2 : 4;
         // the column's part of the next node row's totals: weights, squared weights, y, y^2
         uint32_t nw = 0u;
         unsigned long long nw2 = 0ull;
@@ -824,13 +832,13 @@ __global__ void __launch_bounds__(128, 5) k_grid_totals(TotalsParams tp, float2*
             for (int hs = 0; hs < 2; ++hs) {
                 uint32_t bw[2] = {0u, 0u};  // [0] the node row above, [1] below
                 DF by[2];
-                // rows in fours, their records loaded before any is used
-                for (int k0 = hs * half; k0 < (hs + 1) * half; k0 += 4) {
-                    float4 A[4];
-                    float2 B[4];
+                // rows in fours (twos), their records loaded before any is used
+                for (int k0 = hs * half; k0 < (hs + 1) * half; k0 += kRows) {
+                    float4 A[kRows];
+                    float2 B[kRows];
                     auto read = [&](auto load) {
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) {
+                        for (int i = 0; i < kRows; ++i) {
                             const int y = s * step + k0 + i;
                             const int64_t p = int64_t(y) * g.w + x;
                             A[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -838,24 +846,40 @@ __global__ void __launch_bounds__(128, 5) k_grid_totals(TotalsParams tp, float2*
                             if (k0 + i < (hs + 1) * half && xin && y < g.h && inside(p)) load(i, p);
                         }
                     };
-                    if constexpr (!kByClass) {
-                        read([&](int i, int64_t p) {
-                            A[i] = gp.pat4[p];
-                            B[i] = gp.pat2[p];
-                        });
-                    } else {
+                    if constexpr (kMode == kDeviants) {
                         read([&](int i, int64_t p) {
                             A[i] = make_float4(gp.cls[cls][0][p], gp.cls[cls][1][p], gp.cls[cls][2][p], gp.cls[cls][3][p]);
                             B[i] = make_float2(gp.cls[cls][4][p], gp.pat2[p].y);
                         });
+                    } else {
+                        read([&](int i, int64_t p) {
+                            A[i] = gp.pat4[p];
+                            B[i] = gp.pat2[p];
+                        });
+                    }
+                    if constexpr (kMode == kAll) {
+                        float sums[kRows][5];
+#pragma unroll
+                        for (int i = 0; i < kRows; ++i) {
+                            const uint32_t bits = __float_as_uint(B[i].y);
+                            const PixPattern pp{A[i].x, A[i].y, A[i].z, A[i].w, B[i].x, uint8_t(bits), uint8_t(bits >> 8),
+                                                {uint8_t(bits >> 16), uint8_t(bits >> 24)}};
+                            class_sums(gp, cls, int64_t(s * step + k0 + i) * g.w + x, pp, sums[i]);
+                        }
+#pragma unroll
+                        for (int i = 0; i < kRows; ++i) {
+                            A[i] = make_float4(sums[i][0], sums[i][1], sums[i][2], sums[i][3]);
+                            B[i].x = sums[i][4];
+                        }
                     }
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
+                    for (int i = 0; i < kRows; ++i) {
                         const uint32_t bits = __float_as_uint(B[i].y);
-                        if (kByClass ? !deviant(bits) || unplaced_pixel(bits) == pix : deviant(bits)) continue;
+                        if (kMode == kPattern && deviant(bits)) continue;
+                        if (kMode == kDeviants && (!deviant(bits) || unplaced_pixel(bits) == pix)) continue;
                         float4 a = A[i];
                         float s2l = B[i].x;
-                        if (!kByClass && (bits & 0xffu) != P) {
+                        if (kMode == kPattern && (bits & 0xffu) != P) {
                             const int more = ((bits >> 16) & 0xffu) == P ? 0 : (bits >> 24) == P ? 1 : -1;
                             if (more < 0) continue;
                             const int64_t p = int64_t(s * step + k0 + i) * g.w + x;
@@ -991,12 +1015,27 @@ __global__ void __launch_bounds__(128, 5) k_grid_totals(TotalsParams tp, float2*
         }
         store_only = false;
     };
-    for (uint32_t P = set.pop(); P != 0u; P = set.pop()) walk(std::false_type{}, P, 0, (P & RPD_SAMPLE_PIXEL_VALID) != 0);
+    int patterns = 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) patterns += __popc(set.w[q]);
+    if (!mixed && patterns + (classes ? kClasses : 0) > tp.many) {
+        // (each class's entries are its own: the parts need no order; zero entries stay to be written)
+#pragma unroll 1
+        for (int c = part; c < kClasses; c += tp.parts) {
+            store_only = tp.fresh != 0;
+            walk(std::integral_constant<int, kAll>{}, class_bit(c), c, true);
+        }
+        return;
+    }
+    if (part > 0) return;
+    for (uint32_t P = set.pop(); P != 0u; P = set.pop())
+        walk(std::integral_constant<int, kPattern>{}, P, 0, (P & RPD_SAMPLE_PIXEL_VALID) != 0);
     if (!classes && !unplaced) return;
 #pragma unroll 1
     for (int c = classes ? 0 : kClasses; c < 2 * kClasses; ++c) {
         if (c == kClasses && !unplaced) return;
-        if (c != kClasses) walk(std::true_type{}, class_bit(c % kClasses), c % kClasses, c < kClasses);  // (class 0 is the screen)
+        if (c != kClasses)  // (class 0 is the screen)
+            walk(std::integral_constant<int, kDeviants>{}, class_bit(c % kClasses), c % kClasses, c < kClasses);
     }
 }
 
@@ -1009,7 +1048,7 @@ __global__ void __launch_bounds__(128, 5) k_grid_totals(TotalsParams tp, float2*
 // others turn up meanwhile; where it has a few (seven in a 1920x1080x16 frame), hardly any of their samples count, and
 // a first walk notes the patterns and, up to kOddPicks of them, the samples.
 // Blocks of one warp take the listed nodes in turn; each node is one warp's, in a fixed order.
-constexpr int kOddPicks = 256;
+constexpr int kOddPicks = 64;
 struct OddPicks {
     int64_t sample[kOddPicks];
     uint16_t pixel[kOddPicks];
@@ -2218,14 +2257,16 @@ cudaError_t launch_grid_fast(Job& j, const DeviceSamples& s, int64_t first, int6
         int sh = 0;
         while ((1 << sh) < step) ++sh;
         // (images of a few nodes fill the GPU with neither form, and the one launch of the pattern form
-        // is shorter than the two: 64x48, 63 nodes, 21 against 29 us; 256x256, 1089 nodes, 76 against 72)
+        // is shorter than the two: 64x48, 63 nodes, 21 against 29 us. 256x256, 1089 nodes: one pattern 21 against 35,
+        // three 75 against 45, eight 86 against 45; 640x360, 3726 nodes: 30 / 34, 134 / 79, 158 / 140; 1280x720:
+        // 88 / 56, 468 / 141, 544 / 269)
         if (gpar.uniform_ok && int_w && step >= 2 && step <= 16 && gpar.count_nodes > 512) {
             const int ny0 = int(gpar.node0 / j.g.nodes_x), ny1 = ny0 + int(gpar.count_nodes / j.g.nodes_x);
             // (scratch: a node plane that recompute_sensitivity writes before it reads)
             unsigned* odd_count = reinterpret_cast<unsigned*>(j.p.counters + RPD_COUNTER_COUNT_);
             int32_t* odd_nodes = reinterpret_cast<int32_t*>(j.n.prior[0]);
             if ((e = cudaMemsetAsync(odd_count, 0, sizeof(unsigned), j.stream)) != cudaSuccess) return e;
-            TotalsParams tp{j.g, first, count, ny0, ny1, 1, 1, sh, fresh ? 1 : 0, odd_count, odd_nodes};
+            TotalsParams tp{j.g, first, count, ny0, ny1, 1, 1, sh, fresh ? 1 : 0, 1, 0, odd_count, odd_nodes};
             const int cells = 32 / step, image_cells = (j.g.w + step - 1) / step;
             tp.col_warps = std::max(1, (image_cells - 1 + cells - 2) / (cells - 1));
             // node rows per warp: one more strip than node rows is walked, so as many as fit in the 20
@@ -2236,7 +2277,14 @@ cudaError_t launch_grid_fast(Job& j, const DeviceSamples& s, int64_t first, int6
             const int64_t rows = (int64_t(tp.col_warps) * (ny1 - ny0) + resident - 1) / resident;
             tp.len = int(std::min<int64_t>(16, std::max<int64_t>(1, rows)));
             const int64_t warps = int64_t(tp.col_warps) * ((ny1 - ny0 + tp.len - 1) / tp.len);
-            k_grid_totals<<<unsigned((warps + 3) / 4), 128, 0, j.stream>>>(tp, target, gp);
+            // Seven class walks stand for any number of pattern walks; each costs about 1.5 of them (up to three
+            // sums per pixel), so from eleven on (totals and screen bins of up to eight patterns, 1280x720x8: 428 -> 269
+            // us). Where seven times the warps fit on the GPU at once, seven share the classes, from two walks on
+            // (256x256x8 of eight patterns 188 -> 45 us, of three 70 -> 45, of one 33 -> 35); with fewer parts on
+            // larger images the repeated look for patterns costs other frames on the GPU more than it gives.
+            tp.parts = warps * kClasses <= resident ? kClasses : 1;
+            tp.many = tp.parts > 1 ? 1 : 10;
+            k_grid_totals<<<unsigned((warps * tp.parts + 3) / 4), 128, 0, j.stream>>>(tp, target, gp);
             if ((e = cudaGetLastError()) != cudaSuccess) return e;
             const size_t smem = size_t(LaneBins<false>::kSlots) * 32 * sizeof(float) + sizeof(OddPicks) + size_t(4) * step * step * sizeof(uint16_t);
             const unsigned odd_blocks = std::min<unsigned>(nblocks, unsigned(kStripSms) * 16);
