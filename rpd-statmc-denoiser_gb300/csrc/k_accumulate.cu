@@ -1461,12 +1461,14 @@ cudaError_t run_accumulate(Job& j, const DeviceSamples& s, int32_t spp, int64_t 
 }
 
 // The staged form of the statistics pass, if the push allows it: uniform samples per pixel, 16-byte
-// aligned planes, a pixel's row of each plane a multiple of 32 bytes. *taken: it ran. From 32 samples
-// per pixel: up to 16 the general form reads each line in few enough steps and executes a third
-// fewer instructions (1920x1080, general / staged: FP32 8 spp 0.33 / 0.45 ms, 16 spp 0.64 / 0.90, 32
-// spp 3.03 / 1.43, 64 spp 7.1 / 2.25; compact 16 spp 0.43 / 0.78, 32 spp 1.40 / 1.30, 64 spp 3.75 /
-// 2.26). Below a million samples its tensor maps' encoding on the host would show.
-constexpr int kRowMinSpp = 32;
+// aligned planes, a pixel's row of each plane a multiple of 32 bytes, and enough samples per pixel: up to
+// 16 the general form reads each line in few enough steps and executes a third fewer instructions. General / staged
+// at 1920x1080: FP32 8 spp 0.33 / 0.45 ms, 16 spp 0.64 / 0.90, 32 spp 3.03 / 1.43, 64 spp 7.1 / 2.25;
+// compact 16 spp 0.43 / 0.78, 32 spp 1.36 / 1.39 (1280x720 0.44 / 0.62), 48 spp 4.13 / 1.87. Compact planes without
+// the random dimensions (RPD off) are half the bytes again and never take it: 32 spp 0.50 / 0.86, 64 spp 1.10 /
+// 1.64, 640x360x256 0.52 / 0.78; FP32 ones are equal (64 spp 1.61 / 1.61). Below a million samples its tensor
+// maps' encoding on the host would show.
+constexpr int kRowMinSpp = 32, kRowMinSpp16 = 33;
 template <bool COMPACT>
 cudaError_t run_rows(Job& j, const DeviceSamples& s, int64_t first, int64_t count, const GridPrep& gp, int32_t spp,
                      int fresh, const void* const* planes, RowsArgs& ra) {
@@ -1490,7 +1492,8 @@ cudaError_t launch_accumulate_rows(Job& j, const DeviceSamples& s, int64_t first
                                    int32_t spp, int fresh, bool* taken) {
     *taken = false;
     const int es = s.compact ? 2 : 4;
-    if (spp < kRowMinSpp || (int64_t(spp) * es) % kRowBytes || count * int64_t(spp) < (int64_t(1) << 20) ||
+    if (s.compact && !gp.lum) return cudaSuccess;
+    if (spp < (s.compact ? kRowMinSpp16 : kRowMinSpp) || (int64_t(spp) * es) % kRowBytes || count * int64_t(spp) < (int64_t(1) << 20) ||
         count > INT32_MAX)
         return cudaSuccess;
     const void* planes[20];
