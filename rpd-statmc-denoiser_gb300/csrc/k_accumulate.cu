@@ -1464,8 +1464,8 @@ cudaError_t run_accumulate(Job& j, const DeviceSamples& s, int32_t spp, int64_t 
 // aligned planes, a pixel's row of each plane a multiple of 32 bytes, and enough samples per pixel: up to
 // 16 the general form reads each line in few enough steps and executes a third fewer instructions. General / staged
 // at 1920x1080: FP32 8 spp 0.33 / 0.45 ms, 16 spp 0.64 / 0.90, 32 spp 3.03 / 1.43, 64 spp 7.1 / 2.25;
-// compact 16 spp 0.43 / 0.78, 32 spp 1.36 / 1.39 (1280x720 0.44 / 0.62), 48 spp 4.13 / 1.87. Compact planes without
-// the random dimensions (RPD off) are half the bytes again and never take it: 32 spp 0.50 / 0.86, 64 spp 1.10 /
+// compact 16 spp 0.43 / 0.78, 32 spp 1.08 / 1.39 (1280x720 0.44 / 0.62), 48 spp 4.13 / 1.87. Compact planes without
+// the random dimensions (RPD off) are half the bytes again and never take it: 32 spp 0.58 / 0.86, 64 spp 1.08 /
 // 1.64, 640x360x256 0.52 / 0.78; FP32 ones are equal (64 spp 1.61 / 1.61). Below a million samples its tensor
 // maps' encoding on the host would show.
 constexpr int kRowMinSpp = 32, kRowMinSpp16 = 33;
