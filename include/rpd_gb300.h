@@ -239,7 +239,9 @@ int rpd_config_validate(const rpd_config* cfg, char* msg, size_t msg_capacity);
 /* ---- context and jobs ------------------------------------------------------------- */
 
 /* Opens the CUDA device and sets the HBM budget that jobs are admitted against
- * (0 = all free memory at creation). */
+ * (0 = all free memory at creation). Between calls of the post-filters and metrics the context
+ * keeps up to 512 MiB of their scratch, no more than the budget leaves beside its jobs and
+ * buffers (rpd_ctx_bytes_in_use does not count it); rpd_ctx_destroy gives it back. */
 int rpd_ctx_create(int device, uint64_t hbm_budget_bytes, rpd_ctx** out);
 void rpd_ctx_destroy(rpd_ctx* ctx);
 /* Bytes of HBM a job with this config would hold. */

@@ -232,6 +232,25 @@ void job_free(Job& j, void* p) {
     }
 }
 
+// What a context's pool keeps of the scratch it has freed, at most. The default pool keeps nothing: each of a
+// filter's calls mapped its scratch anew and unmapped it at the closing synchronisation (at
+// 1920x1080 0.88 ms per a-trous call and 0.93 per joint bilateral, 0.50 and 0.61 with the pool).
+// 512 MiB holds the a-trous filter's 64 bytes per pixel at 3840x2160; beyond it, and when another
+// allocation would fail, the driver unmaps what is free. rpd_ctx_destroy gives it all back. Creating the pool
+// costs a context about 25 us, once.
+constexpr uint64_t kPoolKeep = uint64_t(512) << 20;
+
+// Jobs, buffers and what the pool keeps stay within the context's budget together: called wherever in_use has changed.
+void bound_pool(Ctx& c) {
+    std::lock_guard<std::mutex> lock(c.pool_mu);
+    const uint64_t used = c.in_use.load();
+    uint64_t keep = std::min(kPoolKeep, c.budget - std::min(c.budget, used));
+    if (keep == c.pool_keep) return;
+    cudaMemPoolSetAttribute(c.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (keep < c.pool_keep) cudaMemPoolTrimTo(c.pool, keep);
+    c.pool_keep = keep;
+}
+
 // stream_only: the buffer is used on the job's stream alone, so a pool job may replace it in
 // stream order; a buffer that other streams use (the host-push staging) is always replaced
 // after the job's work has finished.
@@ -258,6 +277,7 @@ int grow_device(Job& j, void** buf, uint64_t* cap, uint64_t need, bool stream_on
         return fail(RPD_ERR_OUT_OF_MEMORY, std::string("cudaMalloc staging: ") + cudaGetErrorString(e));
     }
     j.ctx->in_use += want;
+    bound_pool(*j.ctx);
     *cap = want;
     return RPD_OK;
 }
@@ -279,6 +299,7 @@ int ensure_offsets(Job& j, int64_t count) {
         return fail(RPD_ERR_OUT_OF_MEMORY, std::string("cudaMalloc offsets: ") + cudaGetErrorString(e));
     }
     j.ctx->in_use += uint64_t(want) * 8;
+    bound_pool(*j.ctx);
     j.offsets_cap = want;
     return RPD_OK;
 }
@@ -412,14 +433,6 @@ int rpd_config_validate(const rpd_config* c, char* msg, size_t cap) {
     return RPD_OK;
 }
 
-// What a context's pool keeps of the scratch it has freed. The default pool keeps nothing: each of a
-// filter's calls mapped its scratch anew and unmapped it at the closing synchronisation (at
-// 1920x1080 0.88 ms per a-trous call and 0.93 per joint bilateral, 0.50 and 0.61 with the pool).
-// 512 MiB holds the a-trous filter's 64 bytes per pixel at 3840x2160; beyond it, and when another
-// allocation would fail, the driver unmaps what is free. rpd_ctx_destroy gives it all back. Creating the pool
-// costs a context about 25 us, once.
-constexpr uint64_t kPoolKeep = uint64_t(512) << 20;
-
 int rpd_ctx_create(int device, uint64_t budget, rpd_ctx** out) {
     if (!out) return fail(RPD_ERR_INVALID_ARGUMENT, "null output pointer");
     *out = nullptr;
@@ -438,8 +451,7 @@ int rpd_ctx_create(int device, uint64_t budget, rpd_ctx** out) {
     props.location.type = cudaMemLocationTypeDevice;
     props.location.id = device;
     if (e == cudaSuccess) e = cudaMemPoolCreate(&c->pool, &props);
-    uint64_t keep = kPoolKeep;
-    if (e == cudaSuccess) e = cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (e == cudaSuccess) bound_pool(*c);
     if (e != cudaSuccess) {
         if (c->pool) cudaMemPoolDestroy(c->pool);
         if (c->util_stream) cudaStreamDestroy(c->util_stream);
@@ -522,6 +534,7 @@ int job_create(Ctx* c, const rpd_config* cfg, cudaMemPool_t pool, Job** out) {
             return fail(RPD_ERR_OUT_OF_MEMORY, std::string("job arena: ") + cudaGetErrorString(e));
         }
         c->in_use += j->arena_bytes;
+        bound_pool(*c);
     }
     rebase_all(j->p, j->n, static_cast<char*>(j->arena));
     for (int c = 0; c < kClasses; ++c)
@@ -573,6 +586,7 @@ void rpd_job_destroy(rpd_job* job) {
         job_free(*j, j->lum);
         j->ctx->in_use -= j->lum_cap;
     }
+    bound_pool(*j->ctx);
     if (j->scalars) cudaFreeHost(j->scalars);
     for (int s = 0; s < RPD_STAGE_COUNT_; ++s) {
         if (j->ev_start[s]) cudaEventDestroy(j->ev_start[s]);
@@ -1437,6 +1451,7 @@ int rpd_device_alloc(rpd_ctx* ctx, uint64_t bytes, void** out) {
         return fail(RPD_ERR_OUT_OF_MEMORY, std::string("cudaMalloc: ") + cudaGetErrorString(e));
     }
     c->in_use += bytes;
+    bound_pool(*c);
     std::lock_guard<std::mutex> lock(c->mu);
     c->user_allocs[*out] = bytes;
     return RPD_OK;
@@ -1457,6 +1472,7 @@ int rpd_device_free(rpd_ctx* ctx, void* ptr) {
     RPD_CUDA(cudaSetDevice(c->device));
     RPD_CUDA(cudaFree(ptr));
     c->in_use -= bytes;
+    bound_pool(*c);
     return RPD_OK;
 }
 

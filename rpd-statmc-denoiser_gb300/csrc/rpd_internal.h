@@ -125,6 +125,8 @@ struct Ctx {
     std::mutex mu;
     cudaStream_t util_stream = nullptr;
     cudaMemPool_t pool = nullptr;  // scratch of the post-filters and metrics, see kPoolKeep
+    std::mutex pool_mu;
+    uint64_t pool_keep = 0;        // its release threshold (bound_pool)
     std::unordered_map<void*, uint64_t> user_allocs;  // rpd_device_alloc bookkeeping
 };
 
