@@ -1,6 +1,6 @@
 """Uniform compact pushes of many samples per pixel: without RPD their planes are 16 bytes per sample, and the
-statistics pass must take less time than over the FP32 planes of the same samples (about 0.7 of it; as
-long in the staged form, which is for pushes with the random dimensions). With and without RPD around the sample count
+statistics pass must take less time than over the FP32 planes of the same samples (about 0.6 of it; 0.82
+in the staged form, which is for pushes with the random dimensions). With and without RPD around the sample count
 where the staged form begins, compact and decoded pushes give the same bits.
 """
 from __future__ import annotations
@@ -60,4 +60,4 @@ def test_compact_costs_less_without_rpd(gpu_ctx):
     job.close()
     dev.free()
     c16.free()
-    assert ms[1] <= 0.85 * ms[0], ms
+    assert ms[1] <= 0.72 * ms[0], ms
