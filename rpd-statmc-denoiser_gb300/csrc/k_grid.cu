@@ -2199,8 +2199,9 @@ cudaError_t launch_strips_dims(Job& j, const StripParams& sp, float2* target, co
     const int64_t cw = strip_plan<NC>(wide), ct = strip_plan<2>(tall);
     const bool tall_fits = NC == 4 && sp.g.step >= 2 && ct != INT64_MAX;
     // (where a few blocks are the whole grid and a pixel's walk is long, half the rows per warp count for more than
-    // the strips: 256x256x32 at tile 16 85 -> 74 us, at tile 8 77 -> 62; at 4 samples 18 -> 21, so from 32)
-    const bool long_walk = tall_fits && sp.spp >= 32 && ct < 2 * cw &&
+    // the strips, up to half as many again: 256x256x32 at tile 16 85 -> 74 us, at tile 8 77 -> 62; at 4 samples
+    // 18 -> 21, so from 32; 2048x1152x64, with 38 strips against 20, 1.89 -> 2.5 ms)
+    const bool long_walk = tall_fits && sp.spp >= 32 && 2 * ct <= 3 * cw &&
                            int64_t(tall.col_blocks) * ((tall.ny1 - tall.ny0 + tall.len - 1) / tall.len) <= kStripSms;
     if (tall_fits && (ct <= cw || long_walk))
         return launch_strips_shape<2, NC == 4 ? 2 : 1, DIMS>(j, tall, target, gp);
