@@ -605,9 +605,10 @@ __device__ __forceinline__ void store_prep(const GridPrep& gp, int64_t k, const 
 // sample count is a multiple of 4, so each plane is read four samples per load. COMPACT: the
 // planes are rpd_sample_soa16's (s.c16), decoded to float here; WIDE reads them 8 samples (16
 // bytes) per load. PART: what the thread keeps of its pixel. The two parts of a split pixel both read
-// its count p.n, which the luminance part writes: their block meets between the last of these loads and the
-// first store. At the end of the walk that costs nothing, as a block's places are free when its slowest
-// warp is done. Every thread of a split block gets there (local >= count: no pixel), a warp's threads together.
+// its count p.n, which the luminance part writes: the block's 64 colour threads arrive at a barrier with the count in
+// hand, and its 64 luminance threads wait there before they store, each thread once (local >= count: no
+// pixel). The colour part, which never waits, has arrived long before. Per-pixel counts of 4 over 1280x720: 245 us; 255
+// with the whole block meeting at the walk's end, 234 without any order.
 template <bool VEC4, bool COMPACT, bool WIDE, Part PART>
 __device__ __forceinline__ void accumulate_pixel(const PixelPlanes& p, const DeviceSamples& s, const int64_t* offsets, int spp,
                                                  int64_t local, int64_t first, int64_t count, const GridPrep& gp, int fresh) {
@@ -641,6 +642,8 @@ __device__ __forceinline__ void accumulate_pixel(const PixelPlanes& p, const Dev
     // fresh: the frame's first push over every pixel, whose statistics the frame start zeroed
     if (fresh) acc_zero(a);
     else if (some) acc_load<PART>(a, p, idx);
+    // (the count is an operand: it has arrived)
+    if constexpr (PART == kColour) asm volatile("barrier.cta.arrive 1, 128;" : "+r"(a.n));
     px.per_sample_albedo = !COMPACT && s.albedo[0] != nullptr;
     if (some) load_pixel_albedo<COMPACT>(px, s, local);
     const bool dims = prep && lumi;  // the random dimensions are only read for the grid pass
@@ -775,10 +778,8 @@ __device__ __forceinline__ void accumulate_pixel(const PixelPlanes& p, const Dev
         }
     }
 
-    if (split) {
-        __syncthreads();
-        if (!some) return;
-    }
+    if constexpr (PART == kLuminance) asm volatile("barrier.cta.sync 1, 128;" ::: "memory");
+    if (split && !some) return;
     acc_store<PART>(a, p, gp, idx, prep);
 }
 
