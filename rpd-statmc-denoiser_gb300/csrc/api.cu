@@ -900,8 +900,6 @@ int rpd_job_push_samples(rpd_job* job, const rpd_sample_soa* s, int64_t first, i
     return push_tail(j, d, first, count, spp, counts, where, total);
 }
 
-// The part of a push shared by both sample formats: the offsets of per-pixel counts are computed (a uniform
-// push's are multiples of spp, see sample_offset), d points at device planes. Runs the statistics pass and the grid pass.
 int rpd_job_push_samples16(rpd_job* job, const rpd_sample_soa16* s, int64_t first, int64_t count, int32_t spp,
                            const int32_t* counts, rpd_memory where) {
     Job* j = reinterpret_cast<Job*>(job);
@@ -1032,6 +1030,8 @@ int rpd_encode_samples16(rpd_ctx* ctx, const rpd_sample_soa* in, int64_t n_sampl
     return RPD_OK;
 }
 
+// The part of a push shared by both sample formats: the offsets of per-pixel counts are computed (a uniform
+// push's are multiples of spp, see sample_offset), d points at device planes. Runs the statistics pass and the grid pass.
 static int push_tail(Job* j, DeviceSamples& d, int64_t first, int64_t count, int32_t spp, const int32_t* counts,
                      rpd_memory where, int64_t total) {
     int st = RPD_OK;
@@ -1040,6 +1040,7 @@ static int push_tail(Job* j, DeviceSamples& d, int64_t first, int64_t count, int
     GridPrep gp{};
     gp.width = j->g.w;
     const int sup = j->g.support;
+    // (above supports of 2^11, where in_own_bin's rounding bounds end, the grid pass does not use the flag)
     gp.bin_pixels = sup >= 4 && (sup & (sup - 1)) == 0 ? sup / 4 : 1;
     const bool fast_grid = rpd && !j->exact_grid;
     int64_t nsamp = total;

@@ -1047,8 +1047,8 @@ cudaError_t launch_statmc(Job& j) {
     prm.rp_above = 1.0f / 31.0f;
     cudaError_t e = cudaSuccess;
     const int r = prm.r;
-    // the fast window decides the depth gate through threshold * m, which for m >= 1e-8 stays a
-    // normal float away from 0 only when the threshold is at least about 1e-21
+    // the fast window decides the depth gate by a fused difference against m times half an ulp of the threshold,
+    // which for m >= 1e-8 is a normal float, an exact scaling, from thresholds of about 1e-21 on (depth_far)
     if (j.exact_window || r > 16 || !(prm.depth_threshold >= 1e-21f)) {
         k_statmc_window<<<grid_for(np, 128), 128, 0, j.stream>>>(j.p, prm);
         e = cudaGetLastError();

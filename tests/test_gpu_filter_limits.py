@@ -8,6 +8,7 @@ import pytest
 
 from conftest import B, R
 from test_gpu_filter_tiles import images, ptrs
+from test_gpu_parity import FLOOR, TOL, max_rel_err
 
 pytestmark = pytest.mark.gpu
 
@@ -44,3 +45,12 @@ def test_tall_images(gpu_ctx):
         assert e.value.status == ERR_CUDA
         got = call(*(x[:h] for x in a))
         assert np.allclose(got, a[0][:h], rtol=1e-5)  # a constant image stays what it is
+
+
+def test_passes_beyond_the_image(gpu_ctx):
+    w, h = 20, 13  # from the sixth pass on every tap but the centre's is at the border
+    a = images(w, h, True)
+    got = gpu_ctx.atrous(*a, 0.3, 0.6, 0.1, 28)
+    want = np.empty_like(a[0])
+    B.port().orc_atrous_wavelet(*ptrs(*a), w, h, 0.3, 0.6, 0.1, 28, want.ctypes.data, 1)
+    assert max_rel_err(got, want, FLOOR) <= TOL  # the plain form's bar
