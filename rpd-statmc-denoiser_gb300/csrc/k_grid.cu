@@ -812,9 +812,10 @@ __global__ void __launch_bounds__(128, 5) k_grid_totals(TotalsParams tp, float2*
     const float fl = float(il) * inv_step, fr = float(ir) * inv_step;
     bool store_only = tp.fresh != 0;  // the grid is still zero: write instead of add
     // one walk over the strips for pattern P (kPattern), or for class cls (P: that class alone) of all pixels
-    // (kAll) or of the deviant ones (kDeviants: unplaced ones or the others); pix: with the screen's sums
+    // (kAll) or of the deviant ones (kDeviants: unplaced ones or the others); pix: into the screen's sums, of the
+    // samples that have the position; rnd: into the random dimension's
     constexpr int kPattern = 0, kDeviants = 1, kAll = 2;
-    auto walk = [&](auto mode, uint32_t P, int cls, bool pix) {
+    auto walk = [&](auto mode, uint32_t P, int cls, bool pix, bool rnd) {
         constexpr int kMode = decltype(mode)::value;
         constexpr int kRows = kMode == kAll ? 2 : 4;
         // the column's part of the next node row's totals: weights, squared weights, y, y^2
@@ -861,7 +862,13 @@ __global__ void __launch_bounds__(128, 5) k_grid_totals(TotalsParams tp, float2*
                         float sums[kRows][5];
 #pragma unroll
                         for (int i = 0; i < kRows; ++i) {
-                            const uint32_t bits = __float_as_uint(B[i].y);
+                            uint32_t bits = __float_as_uint(B[i].y);
+                            if (pix && (bits & kMixedBit)) {  // the patterns with the position
+                                if (unplaced_pixel(bits)) bits = 0u;
+#pragma unroll
+                                for (int q = 0; q < 32; q += q ? 8 : 16)
+                                    if (!((bits >> q) & RPD_SAMPLE_PIXEL_VALID)) bits &= ~(0xffu << q);
+                            }
                             const PixPattern pp{A[i].x, A[i].y, A[i].z, A[i].w, B[i].x, uint8_t(bits), uint8_t(bits >> 8),
                                                 {uint8_t(bits >> 16), uint8_t(bits >> 24)}};
                             class_sums(gp, cls, int64_t(s * step + k0 + i) * g.w + x, pp, sums[i]);
@@ -998,7 +1005,7 @@ __global__ void __launch_bounds__(128, 5) k_grid_totals(TotalsParams tp, float2*
                 float2* e = grid + (int64_t(s) * g.nodes_x + c0 + node) * kDeps * kDepStride + 32;
                 for (int d = col; d < kDeps; d += step) {  // the cell's lanes take a dependency each
                     const int c = (d + 1) >> 1;  // its class: dep_random(c) and dep_screen(c) in order
-                    if (!(P & class_bit(c)) || ((d & 1) == 0 && !pix)) continue;
+                    if (!(P & class_bit(c)) || !((d & 1) ? rnd : pix)) continue;
                     float2* ed = e + d * kDepStride;
                     float2 o[4];
 #pragma unroll
@@ -1018,24 +1025,26 @@ __global__ void __launch_bounds__(128, 5) k_grid_totals(TotalsParams tp, float2*
     int patterns = 0;
 #pragma unroll
     for (int q = 0; q < 4; ++q) patterns += __popc(set.w[q]);
-    if (!mixed && patterns + (classes ? kClasses : 0) > tp.many) {
-        // (each class's entries are its own: the parts need no order; zero entries stay to be written)
+    // (where some samples lack the position, the screen's sums and the random dimensions' are a walk each)
+    if (patterns + (classes ? kClasses : 0) + (unplaced ? kClasses - 1 : 0) > (mixed ? 2 * tp.many : tp.many)) {
+        // (each walk's entries are its own: the parts need no order; zero entries stay to be written)
 #pragma unroll 1
-        for (int c = part; c < kClasses; c += tp.parts) {
+        for (int q = part; q < (mixed ? 2 * kClasses - 1 : kClasses); q += tp.parts) {
+            const int c = q < kClasses ? q : q - kClasses + 1;
             store_only = tp.fresh != 0;
-            walk(std::integral_constant<int, kAll>{}, class_bit(c), c, true);
+            walk(std::integral_constant<int, kAll>{}, class_bit(c), c, q < kClasses, !mixed || q >= kClasses);
         }
         return;
     }
     if (part > 0) return;
     for (uint32_t P = set.pop(); P != 0u; P = set.pop())
-        walk(std::integral_constant<int, kPattern>{}, P, 0, (P & RPD_SAMPLE_PIXEL_VALID) != 0);
+        walk(std::integral_constant<int, kPattern>{}, P, 0, (P & RPD_SAMPLE_PIXEL_VALID) != 0, true);
     if (!classes && !unplaced) return;
 #pragma unroll 1
     for (int c = classes ? 0 : kClasses; c < 2 * kClasses; ++c) {
         if (c == kClasses && !unplaced) return;
         if (c != kClasses)  // (class 0 is the screen)
-            walk(std::integral_constant<int, kDeviants>{}, class_bit(c % kClasses), c % kClasses, c < kClasses);
+            walk(std::integral_constant<int, kDeviants>{}, class_bit(c % kClasses), c % kClasses, c < kClasses, true);
     }
 }
 
@@ -2264,8 +2273,8 @@ cudaError_t launch_grid_fast(Job& j, const DeviceSamples& s, int64_t first, int6
         while ((1 << sh) < step) ++sh;
         // (images of a few nodes fill the GPU with neither form, and the one launch of the pattern form
         // is shorter than the two: 64x48, 63 nodes, 21 against 29 us. 256x256, 1089 nodes: one pattern 21 against 35,
-        // three 75 against 45, eight 86 against 45; 640x360, 3726 nodes: 30 / 34, 134 / 79, 158 / 140; 1280x720:
-        // 88 / 56, 468 / 141, 544 / 269)
+        // three 75 against 48, eight 86 against 50; 640x360, 3726 nodes: 30 / 34, 134 / 79, 158 / 140; 1280x720:
+        // 88 / 56, 468 / 141, 544 / 308)
         if (gpar.uniform_ok && int_w && step >= 2 && step <= 16 && gpar.count_nodes > 512) {
             const int ny0 = int(gpar.node0 / j.g.nodes_x), ny1 = ny0 + int(gpar.count_nodes / j.g.nodes_x);
             // (scratch: a node plane that recompute_sensitivity writes before it reads)
@@ -2284,9 +2293,10 @@ cudaError_t launch_grid_fast(Job& j, const DeviceSamples& s, int64_t first, int6
             tp.len = int(std::min<int64_t>(16, std::max<int64_t>(1, rows)));
             const int64_t warps = int64_t(tp.col_warps) * ((ny1 - ny0 + tp.len - 1) / tp.len);
             // Seven class walks stand for any number of pattern walks; each costs about 1.5 of them (up to three
-            // sums per pixel), so from eleven on (totals and screen bins of up to eight patterns, 1280x720x8: 428 -> 269
+            // sums per pixel), so from eleven on (totals and screen bins of up to eight patterns, 1280x720x8: 428 -> 308
             // us). Where seven times the warps fit on the GPU at once, seven share the classes, from two walks on
-            // (256x256x8 of eight patterns 188 -> 45 us, of three 70 -> 45, of one 33 -> 35); with fewer parts on
+            // (256x256x8 of eight patterns 188 -> 50 us, of three 70 -> 48, of one 33 -> 35; 256x256x4 where some samples
+            // lack the position, twice the walks, 301 -> 98); with fewer parts on
             // larger images the repeated look for patterns costs other frames on the GPU more than it gives.
             tp.parts = warps * kClasses <= resident ? kClasses : 1;
             tp.many = tp.parts > 1 ? 1 : 10;
